@@ -23,8 +23,8 @@
 // particles were after the previous step (particles drift away from their
 // brick between reorders); it is stored per brick relative to the brick's
 // centre, unwrapped across the periodic boundary, and this kernel writes the
-// box for the next step.  A box too large for shared memory falls back to the
-// brick itself plus one cell; particles outside the box gather and deposit
+// box for the next step.  A box too large for shared memory is cut to what
+// fits around the brick (tile_setup); particles outside the box gather and deposit
 // through global memory with the same arithmetic.
 //
 // The current of the brick is summed in a shared-memory box as 32-bit fixed
@@ -270,7 +270,9 @@ struct PackedBounds {
 // second zigzag segment is then left to the caller (Bq, at box address qa),
 // which deposits those of a warp together.  The cell range is checked where
 // it guards a global access; a cell decoded inside the box is in range.
-template <int DIMS, bool TILED, bool XC = false, bool XS = false>
+// PRE: a particle outside the box reads its nodes from tb.gA / tb.gB, 8 (2D:
+// 4) pairs of loads instead of 20 (2D: 9) field reads per node.
+template <int DIMS, bool TILED, bool XC = false, bool XS = false, bool PRE = false>
 __device__ __forceinline__ bool push_one(const GridP &g, const PartF32 &p, uint32_t n, const PState &s,
                                          const float *__restrict__ Ex, const float *__restrict__ Ey,
                                          const float *__restrict__ Ez, const float *__restrict__ Bx,
@@ -307,6 +309,14 @@ __device__ __forceinline__ bool push_one(const GridP &g, const PartF32 &p, uint3
     float pE[3] = {0.f, 0.f, 0.f}, pB[3] = {0.f, 0.f, 0.f};
     if (inside) {
         gather_box<DIMS>(tb, nb, wt, pE, pB);
+    } else if (PRE) {
+        const int wx = i == g.mx - 3 ? 1 - g.nx : 1, wy = (j == g.my - 3 ? 1 - g.ny : 1) * sy,
+                  wz = DIMS == 3 ? (k == g.mz - 3 ? 1 - g.nz : 1) * sz : 0;
+#pragma unroll
+        for (int c8 = 0; c8 < (DIMS == 3 ? 8 : 4); c8++) {
+            const int nd = cell + (c8 & 1) * wx + ((c8 >> 1) & 1) * wy + ((c8 >> 2) & 1) * wz;
+            accum(wt[c8], ldro(tb.gA + nd), ldro(tb.gB + nd), pE, pB);
+        }
     } else {
 #pragma unroll
         for (int c8 = 0; c8 < (DIMS == 3 ? 8 : 4); c8++) {
@@ -470,7 +480,7 @@ __device__ __forceinline__ void drain_queue(float (*q)[32], int k, const JOff &j
 // queue and deposited 32 at a time instead of in a branch that nearly every
 // warp would take for a few of its lanes.  The next particle loads while
 // this one moves.
-template <int DIMS, bool XC = false, bool XS = false>
+template <int DIMS, bool XC = false, bool XS = false, bool PRE = false>
 __device__ __forceinline__ void push_range_tiled(const GridP &g, const PartF32 &p, uint32_t p0, uint32_t p1,
                                                  const float *__restrict__ Ex, const float *__restrict__ Ey,
                                                  const float *__restrict__ Ez, const float *__restrict__ Bx,
@@ -486,7 +496,7 @@ __device__ __forceinline__ void push_range_tiled(const GridP &g, const PartF32 &
     auto move = [&](const PState &st, uint32_t b) {
         Part Bq;
         uint32_t qa = 0;
-        const bool cross = push_one<DIMS, true, XC, XS>(g, p, b + lane, st, Ex, Ey, Ez, Bx, By, Bz, Jx, Jy, Jz, err, tb,
+        const bool cross = push_one<DIMS, true, XC, XS, PRE>(g, p, b + lane, st, Ex, Ey, Ez, Bx, By, Bz, Jx, Jy, Jz, err, tb,
                                                     bd, Bq, qa);
         const uint32_t m = __ballot_sync(0xffffffffu, cross);
         if (m) {
@@ -538,12 +548,14 @@ __device__ __forceinline__ void move_brick(const GridP &g, const PartF32 &p, con
     TileBox tb;
     int home_lo[3], home_hi[3];
     brick_home<DIMS>(g, bk, b, tb, home_lo, home_hi);
+    tb.gA = bk.nodeA;
+    tb.gB = bk.nodeB;
     // a move is below c per axis; the box is the stored bounds (no margin)
     tile_setup<DIMS, !XS, false, PRE>(g, bk, b, p1 - p0, 0, g.c_f, sm, ts, tb, home_lo, home_hi, Ex, Ey, Ez, Bx, By,
                                       Bz);
     PackedBounds bd;
     bd.init();
-    push_range_tiled<DIMS, XC, XS>(g, p, p0, p1, Ex, Ey, Ez, Bx, By, Bz, Jx, Jy, Jz, err, tb, bd,
+    push_range_tiled<DIMS, XC, XS, PRE>(g, p, p0, p1, Ex, Ey, Ez, Bx, By, Bz, Jx, Jy, Jz, err, tb, bd,
                                    ts.s_q[threadIdx.x >> 5]);
     __syncthreads();
     tile_finish<DIMS, !XS>(g, bk, b, tb, sm, ts, bd.unpack(), home_lo, home_hi, Jx, Jy, Jz);

@@ -12,7 +12,8 @@
 // bounding box, in cells relative to the brick centre and unwrapped across
 // periodic boundaries, of where the brick's particles were after the
 // previous step (Bricks::box, rewritten by the mover for the next step); a
-// box too large for shared memory falls back to the brick plus one cell.
+// box too large for shared memory is cut to as much of it as fits around the
+// brick (at least one cell on each side).
 #pragma once
 
 #include "common.cuh"
@@ -207,6 +208,8 @@ struct TileBox {
     uint32_t oY4, oZ4;  // node-box byte strides of the 16-byte nodes (8-byte nodes: half)
     JOff jo;            // current-box byte offsets
     float S;            // fixed-point scale of the current box
+    const float4 *gA;   // node averages of the whole grid (Bricks::nodeA, nodeB)
+    const float2 *gB;
 };
 
 // Running bounds of the particles' new cells (relative to the brick centre).
@@ -242,6 +245,7 @@ __device__ __forceinline__ PState load_state(const PartF32 &p, uint32_t n)
     return s;
 }
 
+constexpr int kBoxMarginMax = 8;   // cells around its brick of a box cut to fit
 constexpr int kTileThreads = 256;
 constexpr int kTileWarps = kTileThreads / 32;
 
@@ -290,6 +294,14 @@ __device__ __forceinline__ void brick_home(const GridP &g, const Bricks &bk, int
     }
 }
 
+// The box of cells m[0..2] .. -m[3..5] fits the mover's shared memory.
+template <int DIMS>
+__device__ __forceinline__ bool box_fits(const Bricks &bk, const int m[6], int jw)
+{
+    const int cx = 1 - m[3] - m[0], cy = 1 - m[4] - m[1], cz = DIMS == 3 ? 1 - m[5] - m[2] : 1;
+    return cx <= kBoxAxisMax && cy <= kBoxAxisMax && cz <= kBoxAxisMax && box_floats(DIMS, cx, cy, cz, jw) <= bk.smem_floats;
+}
+
 // The boxes of brick b for this step (one CTA, ends with a barrier): the
 // stored bounds widened by `margin` cells on each side (movers that gather a
 // second time at the cell they move to), or the brick +- 1 cell when that is
@@ -313,13 +325,40 @@ __device__ __forceinline__ void tile_setup(const GridP &g, const Bricks &bk, int
     const int *sb = bk.box + 8 * (size_t)b;
     int lo[3] = {ldco(sb) - margin, ldco(sb + 1) - margin, DIMS == 3 ? ldco(sb + 2) - margin : 0};
     int hi[3] = {ldco(sb + 3) + margin, ldco(sb + 4) + margin, DIMS == 3 ? ldco(sb + 5) + margin : 0};
-    if (hi[0] < lo[0] || hi[1] < lo[1] || hi[2] < lo[2] || hi[0] - lo[0] >= kBoxAxisMax ||
-        hi[1] - lo[1] >= kBoxAxisMax || hi[2] - lo[2] >= kBoxAxisMax ||
-        box_floats(DIMS, hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1, WIDE ? 2 : 1) > bk.smem_floats) {
+    // too large: as much of it as fits around the brick, the widest margin
+    // cut first (the brick and one cell around it always fit)
+    {
+        auto fits = [&]() {
+            const int m[6] = {lo[0], lo[1], lo[2], -hi[0], -hi[1], -hi[2]};
+            return hi[0] >= lo[0] && hi[1] >= lo[1] && hi[2] >= lo[2] && box_fits<DIMS>(bk, m, WIDE ? 2 : 1);
+        };
+        if (!fits()) {
 #pragma unroll
-        for (int d = 0; d < DIMS; d++) {
-            lo[d] = home_lo[d] - 1;
-            hi[d] = home_hi[d] + 1;
+            for (int d = 0; d < DIMS; d++) {
+                lo[d] = max(lo[d], home_lo[d] - kBoxMarginMax);
+                hi[d] = min(hi[d], home_hi[d] + kBoxMarginMax);
+                if (hi[d] < lo[d]) {
+                    lo[d] = home_lo[d];
+                    hi[d] = home_hi[d];
+                }
+            }
+            for (int it = 0; it < 6 * kBoxMarginMax && !fits(); it++) {
+                int w = 0;
+#pragma unroll
+                for (int d = 0; d < DIMS; d++) w = max(w, max(home_lo[d] - lo[d], hi[d] - home_hi[d]));
+                bool cut = false;
+#pragma unroll
+                for (int d = 0; d < DIMS; d++) {
+                    if (!cut && hi[d] - home_hi[d] == w) {
+                        hi[d]--;
+                        cut = true;
+                    }
+                    if (!cut && home_lo[d] - lo[d] == w) {
+                        lo[d]++;
+                        cut = true;
+                    }
+                }
+            }
         }
     }
 #pragma unroll

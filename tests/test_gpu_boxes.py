@@ -1,0 +1,66 @@
+"""The FP32 tiled mover when its particles have left their bricks: boxes cut
+to shared memory with particles outside them (2D and 3D, exact charge)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+C = 0.45
+
+
+def _hot(nx, ny, nz, dims, ppc, seed, spread=0.6):
+    from pictor_b200 import Particles
+
+    rng = np.random.Generator(np.random.Philox(key=seed))
+    n = ppc * nx * ny * nz
+    p = Particles.empty(2 * n)
+    for k, m in (("x", nx), ("y", ny), ("z", nz)):
+        a = rng.random(n) * m + (3.0 if k != "z" or dims == 3 else 1.0)
+        getattr(p, k)[:] = np.concatenate([a, a])
+    for k in "uvw":
+        getattr(p, k)[:] = rng.normal(scale=spread, size=2 * n)
+    p.q[:n], p.q[n:] = 1.0, -1.0
+    p.flv[:n], p.flv[n:] = 1, 2
+    return p
+
+
+def _cfg(shape, dims, ppc, period, precision="fp32", **kw):
+    from pictor_b200 import PicConfig, init_scale
+
+    sc = init_scale(C, 2.0, ppc)
+    n = 2 * ppc * shape[0] * shape[1] * shape[2]
+    return PicConfig(nx=shape[0], ny=shape[1], nz=shape[2], dims=dims, c=C, qi=sc["qi"], precision=precision,
+                     capacity=int(n * (1.1 if precision == "fp32" else 3)) + 4096, reorder_period=period, **kw), sc
+
+
+@pytest.mark.parametrize("shape,dims,ppc,steps,kw", [
+    ((41, 24, 23), 3, 8, 16, {}),                  # about half the particles outside the cut boxes
+    ((24, 24, 24), 3, 2, 9, {"exact_charge": 1}),
+    ((24, 41, 13), 3, 1, 3, {"brick": (8, 8, 8)}),
+    ((96, 75, 1), 2, 8, 60, {"brick": (8, 8, 1)}),
+])
+def test_outgrown_boxes_move_like_the_per_particle_form(shape, dims, ppc, steps, kw):
+    """After `steps` moves without a reorder the boxes have outgrown shared
+    memory.  One more move, tiled, against the per-particle form from the same
+    slots and fields: particles bit for bit, the current (through E) to the
+    FP32 rounding of its sums (64 contributions of a cell, 2^-24 each, within
+    1e-5 of the largest)."""
+    from pictor_b200 import Simulation
+
+    cfg, _ = _cfg(shape, dims, ppc, 0, **kw)
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        a.load_particles(_hot(*shape, dims, ppc, 5))
+        a.reorder()
+        a.step(steps)
+        b.load_particles(a.fetch_particles())
+        b.load_fields(a.fetch_fields())
+        a.step(1)
+        b.step(1)
+        pa, pb = a.fetch_particles(), b.fetch_particles()
+        for k in ("x", "y", "u", "v", "w", "q", "flv") + (("z",) if dims == 3 else ()):
+            assert np.array_equal(getattr(pa, k), getattr(pb, k)), k
+        fa, fb = a.fetch_fields(), b.fetch_fields()
+        for k in ("Ex", "Ey", "Ez"):
+            ea, eb = getattr(fa, k), getattr(fb, k)
+            assert np.abs(ea - eb).max() <= 1e-5 * np.abs(eb).max(), k
+        assert a.device_errors() == 0
