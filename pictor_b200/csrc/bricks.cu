@@ -328,6 +328,13 @@ __global__ void k_brick_finish(Bricks bk, Counters *cnt)
     const long long live = bk.tile_start[bk.ntiles];
     cnt->used = live;
     cnt->np = live;
+    if (bk.over) {   // the first move since the last reorder that left over 1/kOverShare of the boxes too large, 0 = none
+        uint32_t first = 0;
+        for (int j = kOverWords - 2; j >= 1; j--)
+            if (bk.over[1 + j] > (uint32_t)(bk.ntiles / kOverShare)) first = (uint32_t)j;
+        for (int j = 0; j < kOverWords; j++) bk.over[j] = 0;
+        if (first) *(volatile uint32_t *)bk.over_host = first;   // kept until the host has read it
+    }
 }
 
 static unsigned grid_for(long long n)

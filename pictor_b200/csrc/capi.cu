@@ -78,6 +78,14 @@ struct pic_handle {
     size_t stage_bytes = 0;
     cudaEvent_t ev_copied[2] = {nullptr, nullptr}, ev_done[2] = {nullptr, nullptr};
     bool sorted = false;
+    // steps between two groupings of the particles by brick inside pic_step
+    // (step_reorders): the current interval, the steps since the last one, the
+    // longest interval that is not accounted for yet, the clean ones in a row,
+    // and the reorders' report (Bricks::over_host, valid after the event)
+    int group_every = 0, since_group = 0, group_len = 0, group_clean = 0;
+    uint32_t *over_host = nullptr;
+    cudaEvent_t ev_group = nullptr;
+    bool group_reported = false;
     // slab form: device counts of the particles sent through the x faces
     uint32_t *slab_sent = nullptr;
     // phase entry points wait for their work (pic_set_sync)
@@ -463,6 +471,55 @@ int get_graph(pic_handle *h, int cur, bool reorder, cudaGraphExec_t *out)
     return PIC_OK;
 }
 
+// Whether the step about to be enqueued ends with a reorder: every
+// reorder_period steps, as the reference does, and in the FP32 Cartesian form
+// also when the bricks' boxes are about to outgrow the tiled mover's shared
+// memory.  A particle outside its brick's box gathers and deposits through
+// global memory, so a move with many such boxes costs several ordinary ones,
+// while a reorder costs about one (3D, 537 M particles, thermalised beams:
+// moves of 12-14 ms for 7 steps, then 15, 18, 23, ... 63 ms up to the 20th; a
+// reorder 14 ms).  The reorder reports the first move that left over 1/64 of
+// the boxes too large; the next interval ends there, and grows by a step after
+// kGroupClean intervals without one.  The report of a reorder is waited for only when
+// kGroupMin steps behind it are enqueued, so the device does not run dry.
+constexpr int kGroupMin = 3, kGroupClean = 4;
+int step_reorders(pic_handle *h, bool *reorder)
+{
+    const int period = h->cfg.reorder_period;
+    *reorder = period > 0 && (h->t % period) == 0;
+    h->since_group++;
+    if (*reorder || !h->over_host || !h->sorted || period <= kGroupMin || h->since_group < kGroupMin) return PIC_OK;
+    if (h->group_reported) {
+        CK(cudaEventSynchronize(h->ev_group));
+        // no later reorder is enqueued yet, so nothing writes the word now
+        const int first = (int)*(volatile uint32_t *)h->over_host;
+        *(volatile uint32_t *)h->over_host = 0;
+        if (h->group_every < 1 || h->group_every > period) h->group_every = period;
+        if (first > 0) {
+            h->group_every = std::max(kGroupMin, std::min(first, period));
+            h->group_clean = 0;
+        } else if (h->group_len >= h->group_every && ++h->group_clean >= kGroupClean) {
+            h->group_every = std::min(period, h->group_every + 1);
+            h->group_clean = 0;
+        }
+        h->group_reported = false;
+        h->group_len = 0;
+    }
+    *reorder = h->group_every > 0 && h->since_group >= h->group_every;
+    return PIC_OK;
+}
+
+// A reorder was enqueued on h->s.
+int note_reorder(pic_handle *h)
+{
+    h->group_len = std::max(h->group_len, h->since_group);
+    h->since_group = 0;
+    if (!h->over_host) return PIC_OK;
+    CK(cudaEventRecord(h->ev_group, h->s));
+    h->group_reported = true;
+    return PIC_OK;
+}
+
 // pic_step with an event pair around every phase of every step (no graphs).
 int step_profiled(pic_handle *h, int32_t nsteps)
 {
@@ -472,7 +529,8 @@ int step_profiled(pic_handle *h, int32_t nsteps)
     int rc = PIC_OK;
     for (int32_t i = 0; i < nsteps && rc == PIC_OK; i++) {
         h->t += 1;
-        const bool reorder = h->cfg.reorder_period > 0 && (h->t % h->cfg.reorder_period) == 0;
+        bool reorder = false;
+        if ((rc = step_reorders(h, &reorder)) != PIC_OK) break;
         cudaEvent_t *e = &ev[(size_t)i * NE];
         cudaEventRecord(e[0], h->s);
         for (int ph = 0; ph < PIC_PHASE_COUNT; ph++) {
@@ -483,6 +541,7 @@ int step_profiled(pic_handle *h, int32_t nsteps)
         if (reorder) {
             h->cur ^= 1;
             if (h->fp32 || h->tiled64) h->sorted = true;  // eager launches: no graph to drop
+            if ((rc = note_reorder(h)) != PIC_OK) break;
         }
         h->prof_steps += 1;
         if (cudaGetLastError() != cudaSuccess) rc = PIC_ERR_CUDA;
@@ -517,14 +576,17 @@ int enqueue_graph_step(pic_handle *h)
 {
     NvtxRange range("pic_step");
     h->t += 1;
-    const bool reorder = h->cfg.reorder_period > 0 && (h->t % h->cfg.reorder_period) == 0;
+    bool reorder = false;
+    int r = step_reorders(h, &reorder);
+    if (r) return r;
     cudaGraphExec_t ge = nullptr;
-    int r = get_graph(h, h->cur, reorder, &ge);
+    r = get_graph(h, h->cur, reorder, &ge);
     if (r) return r;
     CK(cudaGraphLaunch(ge, h->s));
     h->launches += h->graph_kernels[reorder ? 1 : 0][h->cur];
     if (reorder) {
         h->cur ^= 1;
+        if ((r = note_reorder(h)) != PIC_OK) return r;
         if ((h->fp32 || h->tiled64) && !h->sorted) {  // tile ranges are valid from now on
             CK(cudaStreamSynchronize(h->s));
             set_sorted(h, true);
@@ -914,6 +976,8 @@ void pic_destroy(pic_handle *h)
         if (h->ev_copied[b]) cudaEventDestroy(h->ev_copied[b]);
         if (h->ev_done[b]) cudaEventDestroy(h->ev_done[b]);
     }
+    if (h->ev_group) cudaEventDestroy(h->ev_group);
+    if (h->over_host) cudaFreeHost(h->over_host);
     for (void *p : h->allocs) cudaFree(p);
     if (h->cs) cudaStreamDestroy(h->cs);
     if (h->s) cudaStreamDestroy(h->s);
@@ -1064,6 +1128,18 @@ int pic_create(const pic_config *cfg, pic_handle **out)
         if (!r && g.geom == PIC_GEOM_CARTESIAN &&
             !(r = dalloc(h, (char **)&bk.nodeA, (size_t)g.ncell * sizeof(float4))))
             r = dalloc(h, (char **)&bk.nodeB, (size_t)g.ncell * sizeof(float2));
+        // the boxes' report to step_reorders
+        if (!r && g.geom == PIC_GEOM_CARTESIAN && !g.x_external) {
+            if (!(r = dalloc(h, &bk.over, (size_t)kOverWords)) &&
+                (cudaHostAlloc((void **)&h->over_host, sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess ||
+                 cudaHostGetDevicePointer((void **)&bk.over_host, h->over_host, 0) != cudaSuccess ||
+                 cudaEventCreateWithFlags(&h->ev_group, cudaEventDisableTiming) != cudaSuccess))
+                r = PIC_ERR_CUDA;
+            if (!r) {
+                *h->over_host = 0;
+                cudaMemsetAsync(bk.over, 0, kOverWords * sizeof(uint32_t), h->s);
+            }
+        }
     }
     if (!r) r = dalloc(h, &h->cnt, 1);
     if (!r) r = dalloc(h, &h->err, 1);
@@ -1877,7 +1953,8 @@ int pic_reorder(pic_handle *h)
                            h->tiled64 ? &h->t64 : nullptr);
     h->cur ^= 1;
     set_sorted(h, h->fp32 || h->tiled64);
-    return finish_phase(h);
+    const int r = note_reorder(h);
+    return r ? r : finish_phase(h);
 }
 
 int pic_set_step(pic_handle *h, int64_t t)

@@ -106,6 +106,11 @@ struct Bricks {
     uint32_t *wmax_bits;    // max |w| of the live particles (FP32 bits), set by the reorder
     float4 *nodeA;          // node-averaged Ex, Ey, Ez, Bx (+ bext) at every interior node, or null
     float2 *nodeB;          // node-averaged By, Bz (+ bext); both written before each tiled move
+    // Boxes that no longer fit the mover's shared memory, per move since the
+    // reorder (kOverWords words: [0] the moves, [1 + j] the bricks after move
+    // j), and the first move that left many of them, written to host memory
+    // by the next reorder (null where pic_step does not use it)
+    uint32_t *over, *over_host;
     int t[3], nb[3], ntiles;
     unsigned int tmagic[3];   // x / t[d] = fast_div(x, tmagic[d], tshift[d]) for t[d] >= 2 (div_magic)
     int tshift[3];
@@ -124,6 +129,7 @@ __host__ __device__ inline long long box_floats(int dims, int cx, int cy, int cz
 // cylindrical form, whose weights grow with the radius (a 32-bit scale set by
 // the largest weight leaves too few bits for the currents near the axis).
 __host__ __device__ inline int box_current_words(const GridP &g) { return g.geom == PIC_GEOM_CYLINDRICAL ? 2 : 1; }
+constexpr int kOverWords = 64, kOverShare = 64;
 constexpr int kBoxAxisMax = 64;   // cells per axis of a mover box
 // Brick shape: `req` (all > 0) if given, else about 4096 particles per brick
 // at ppc particles per cell.  Returns false if the brick plus one cell on

@@ -69,8 +69,10 @@ template <int DIMS>
 __global__ void __launch_bounds__(kThreads) k_node_avg(GridP g, const float *__restrict__ Ex, const float *__restrict__ Ey,
                                                        const float *__restrict__ Ez, const float *__restrict__ Bx,
                                                        const float *__restrict__ By, const float *__restrict__ Bz,
-                                                       float4 *nodeA, float2 *nodeB)
+                                                       float4 *nodeA, float2 *nodeB, uint32_t *over)
 {
+    if (over && blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x + threadIdx.y == 0)
+        *over += 1;   // this move's number since the reorder (tile_finish)
     const int sy = (int)g.sy, sz = (int)g.sz;
     const int i = 3 + blockIdx.x * 32 + threadIdx.x, j = 3 + blockIdx.y * 8 + threadIdx.y;
     if (i > g.nx + 2 || j > g.ny + 2) return;
@@ -191,9 +193,9 @@ void launch_move_deposit_f32_tiled(const GridP &g, const PartF32 &p, const Brick
                         (unsigned)(g.dims == 3 ? (g.nz + kNodeKz - 1) / kNodeKz : 1)),
             block(32, 8, 1);
         if (g.dims == 3)
-            k_node_avg<3><<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], bk.nodeA, bk.nodeB);
+            k_node_avg<3><<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], bk.nodeA, bk.nodeB, bk.over);
         else
-            k_node_avg<2><<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], bk.nodeA, bk.nodeB);
+            k_node_avg<2><<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], bk.nodeA, bk.nodeB, bk.over);
         count_launches(1);
     }
 #define PIC_MOVE_TILED(D, X, P)                                                                                      \

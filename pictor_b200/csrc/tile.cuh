@@ -513,6 +513,8 @@ __device__ __forceinline__ void tile_finish(const GridP &g, const Bricks &bk, in
                 ob[d + 3] = -m[d + 3];
             }
         }
+        if (bk.over && !empty && !box_fits<DIMS>(bk, m, WIDE ? 2 : 1))
+            atomicAdd(bk.over + 1 + min(ldco(bk.over), (uint32_t)kOverWords - 2u), 1u);
     }
 }
 

@@ -1,5 +1,6 @@
 """The FP32 tiled mover when its particles have left their bricks: boxes cut
-to shared memory with particles outside them (2D and 3D, exact charge)."""
+to shared memory with particles outside them (2D and 3D, exact charge), and
+the reorders pic_step adds before that happens."""
 import numpy as np
 import pytest
 
@@ -64,3 +65,34 @@ def test_outgrown_boxes_move_like_the_per_particle_form(shape, dims, ppc, steps,
             ea, eb = getattr(fa, k), getattr(fb, k)
             assert np.abs(ea - eb).max() <= 1e-5 * np.abs(eb).max(), k
         assert a.device_errors() == 0
+
+
+def test_pic_step_reorders_before_the_boxes_are_outgrown():
+    """A hot run is reordered more often than the period, also across calls;
+    a cold one is not; the hot run's energies stay the FP64 run's (FP32
+    rounding of 40 steps: 1e-4)."""
+    from pictor_b200 import Simulation
+
+    shape, ppc = (48, 32, 32), 8
+
+    def run(precision, spread):
+        cfg, sc = _cfg(shape, 3, ppc, 20, precision)
+        with Simulation(cfg) as s:
+            s.load_particles(_hot(*shape, 3, ppc, 7, spread))
+            s.reorder()
+            s.profile(True)
+            s.phase_times()
+            for n in (20, 1, 1, 11, 7):
+                s.step(n)
+            t = s.phase_times()
+            d = s.diagnostics(sc["masse"])
+        return t["launches"]["reorder"], d
+
+    hot, d32 = run("fp32", 0.6)
+    cold, _ = run("fp32", 0.01)
+    per = cold // 2
+    assert cold == 2 * per and hot >= 4 * per
+    _, d64 = run("fp64", 0.6)
+    for k in ("B2", "E2"):
+        assert abs(d32[k] - d64[k]) <= 1e-4 * d64[k]
+    assert np.allclose(d32["kinetic"], d64["kinetic"], rtol=1e-4)
