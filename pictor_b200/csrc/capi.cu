@@ -46,7 +46,7 @@ struct pic_handle {
     // cylindrical modal form: the fields on modes m = 0, 1, (mx, 3, mz) each;
     // E and B above are kept equal to their theta-gridded synthesis
     bool modal = false;
-    void *Em[3] = {}, *Bm[3] = {}, *Jm[3] = {};   // the handle's precision
+    void *Em[3] = {}, *Bm[3] = {};   // the handle's precision
     PartF64 p64[2] = {};
     PartF32 p32[2] = {};
     int cur = 0;
@@ -237,63 +237,39 @@ void field_ptrs(pic_handle *h, T *E[3], T *B[3], T *J[3])
 // The modal field phases (cyl_modes = 2) in the handle's precision T: each
 // leaves the theta-gridded E / B equal to the synthesis of the modes.
 template <typename T>
-void modal_ptrs(pic_handle *h, T *Em[3], T *Bm[3], T *Jm[3])
+void modal_ptrs(pic_handle *h, T *Em[3], T *Bm[3])
 {
     for (int k = 0; k < 3; k++) {
         Em[k] = (T *)h->Em[k];
         Bm[k] = (T *)h->Bm[k];
-        Jm[k] = (T *)h->Jm[k];
     }
 }
 template <typename T>
 void modal_bhalf(pic_handle *h)
 {
-    T *E[3], *B[3], *J[3], *Em[3], *Bm[3], *Jm[3];
+    T *E[3], *B[3], *J[3], *Em[3], *Bm[3];
     field_ptrs(h, E, B, J);
-    modal_ptrs(h, Em, Bm, Jm);
-    launch_modal_bhalf<T>(h->g, Em, Bm, h->s);
-    launch_modal_synth<T>(h->g, Bm, B, h->s);
+    modal_ptrs(h, Em, Bm);
+    launch_modal_bhalf<T>(h->g, B, Em, Bm, h->s);
 }
+// mode 0: the E update; 2: AddCurrent of the (folded) theta-gridded J,
+// projected onto the modes; 1: the E phase of a step, both with the fold and
+// the zeroing of J.
 template <typename T>
-void modal_update_e(pic_handle *h)
+void modal_efield(pic_handle *h, int mode)
 {
-    T *E[3], *B[3], *J[3], *Em[3], *Bm[3], *Jm[3];
+    T *E[3], *B[3], *J[3], *Em[3], *Bm[3];
     field_ptrs(h, E, B, J);
-    modal_ptrs(h, Em, Bm, Jm);
-    launch_modal_efield<T>(h->g, 0, Em, Bm, Jm, h->s);
-    launch_modal_synth<T>(h->g, Em, E, h->s);
-}
-// AddCurrent of the (folded) theta-gridded J, projected onto the modes.
-template <typename T>
-void modal_add_current(pic_handle *h)
-{
-    T *E[3], *B[3], *J[3], *Em[3], *Bm[3], *Jm[3];
-    field_ptrs(h, E, B, J);
-    modal_ptrs(h, Em, Bm, Jm);
-    launch_modal_project<T>(h->g, J, Jm, h->s);
-    launch_modal_efield<T>(h->g, 2, Em, Bm, Jm, h->s);
-    launch_modal_synth<T>(h->g, Em, E, h->s);
-}
-// The E phase of a step: E update, fold, projection, AddCurrent, synthesis.
-template <typename T>
-void modal_efield_phase(pic_handle *h)
-{
-    T *E[3], *B[3], *J[3], *Em[3], *Bm[3], *Jm[3];
-    field_ptrs(h, E, B, J);
-    modal_ptrs(h, Em, Bm, Jm);
-    launch_modal_efield<T>(h->g, 0, Em, Bm, Jm, h->s);
-    launch_cyl_fold<T>(h->g, J, h->s);
-    launch_modal_project<T>(h->g, J, Jm, h->s);
-    launch_modal_efield<T>(h->g, 2, Em, Bm, Jm, h->s);
-    launch_modal_synth<T>(h->g, Em, E, h->s);
+    modal_ptrs(h, Em, Bm);
+    launch_modal_efield<T>(h->g, mode, E, J, Em, Bm, h->s);
 }
 // Loaded theta-gridded fields -> their modes m = 0, 1; E, B become the synthesis.
 template <typename T>
 void modal_load(pic_handle *h)
 {
-    T *E[3], *B[3], *J[3], *Em[3], *Bm[3], *Jm[3];
+    T *E[3], *B[3], *J[3], *Em[3], *Bm[3];
     field_ptrs(h, E, B, J);
-    modal_ptrs(h, Em, Bm, Jm);
+    modal_ptrs(h, Em, Bm);
     launch_modal_project<T>(h->g, E, Em, h->s);
     launch_modal_project<T>(h->g, B, Bm, h->s);
     launch_modal_synth<T>(h->g, Em, E, h->s);
@@ -326,14 +302,8 @@ int enqueue_phase(pic_handle *h, int cur, bool reorder, int phase)
             case PIC_PHASE_EXCHANGE:
                 break;
             case PIC_PHASE_EFIELD:
-                if (h->modal) {
-                    modal_efield_phase<float>(h);
-                } else {
-                    launch_cyl_efield<float>(g, 0, E, B, J, h->s);
-                    launch_cyl_fold<float>(g, J, h->s);
-                    launch_cyl_efield<float>(g, 2, E, B, J, h->s);
-                }
-                for (int c = 0; c < 3; c++) cudaMemsetAsync(J[c], 0, (size_t)g.ncell * sizeof(float), h->s);
+                if (h->modal) modal_efield<float>(h, 1);
+                else launch_cyl_efield<float>(g, 1, E, B, J, h->s);
                 break;
             case PIC_PHASE_REORDER:
                 if (reorder)
@@ -359,14 +329,8 @@ int enqueue_phase(pic_handle *h, int cur, bool reorder, int phase)
                 launch_exchange_f64(g, h->p64[cur], h->cnt, h->sc, h->capacity, h->err, h->s);
                 break;
             case PIC_PHASE_EFIELD:  // UpdateEfield, halo, fold, AddCurrent, halo, ResetCurrent
-                if (h->modal) {
-                    modal_efield_phase<double>(h);
-                } else {
-                    launch_cyl_efield(g, 0, E, B, J, h->s);
-                    launch_cyl_fold(g, J, h->s);
-                    launch_cyl_efield(g, 2, E, B, J, h->s);
-                }
-                for (int c = 0; c < 3; c++) cudaMemsetAsync(J[c], 0, (size_t)g.ncell * sizeof(double), h->s);
+                if (h->modal) modal_efield<double>(h, 1);
+                else launch_cyl_efield(g, 1, E, B, J, h->s);
                 break;
             case PIC_PHASE_REORDER:
                 if (reorder)
@@ -1102,13 +1066,10 @@ int pic_create(const pic_config *cfg, pic_handle **out)
         h->modal = true;
         const size_t nm = (size_t)g.mx * 3 * (size_t)g.mz, esz = h->fp32 ? sizeof(float) : sizeof(double);
         for (int k = 0; k < 3 && !r; k++)
-            if ((r = dalloc(h, (char **)&h->Em[k], nm * esz)) || (r = dalloc(h, (char **)&h->Bm[k], nm * esz)) ||
-                (r = dalloc(h, (char **)&h->Jm[k], nm * esz)))
-                break;
+            if ((r = dalloc(h, (char **)&h->Em[k], nm * esz)) || (r = dalloc(h, (char **)&h->Bm[k], nm * esz))) break;
         for (int k = 0; k < 3 && !r; k++) {
             cudaMemsetAsync(h->Em[k], 0, nm * esz, h->s);
             cudaMemsetAsync(h->Bm[k], 0, nm * esz, h->s);
-            cudaMemsetAsync(h->Jm[k], 0, nm * esz, h->s);
         }
     }
     if (!r) r = alloc_particles(h);
@@ -1503,8 +1464,8 @@ int pic_update_e(pic_handle *h)
 {
     if (!h) return PIC_ERR_INVALID;
     if (h->modal) {
-        if (h->fp32) modal_update_e<float>(h);
-        else modal_update_e<double>(h);
+        if (h->fp32) modal_efield<float>(h, 0);
+        else modal_efield<double>(h, 0);
     } else if (h->g.geom == PIC_GEOM_CYLINDRICAL && h->fp32) {
         float *E[3], *B[3], *J[3];
         field_ptrs(h, E, B, J);
@@ -1573,8 +1534,8 @@ int pic_add_current(pic_handle *h)
 {
     if (!h) return PIC_ERR_INVALID;
     if (h->modal) {
-        if (h->fp32) modal_add_current<float>(h);
-        else modal_add_current<double>(h);
+        if (h->fp32) modal_efield<float>(h, 2);
+        else modal_efield<double>(h, 2);
     } else if (h->g.geom == PIC_GEOM_CYLINDRICAL && h->fp32) {
         float *E[3], *B[3], *J[3];
         field_ptrs(h, E, B, J);

@@ -15,6 +15,7 @@
 // operation order; the file is compiled without FMA contraction, so fields,
 // momenta and positions equal the serial CPU build bit for bit.
 #include "common.cuh"
+#include "field_math.cuh"
 #include "kernels.cuh"
 #include "tile64.cuh"
 #include "particle_math.cuh"
@@ -71,55 +72,75 @@ __device__ __forceinline__ T lgz(const GridP &g, const T *F, long long c0)
     return r;
 }
 
-// UpdateBfieldHalf main loop (cyl_em_update.F90:66-83): i 4..mx-1, j 1..my-1,
-// k 1..mz-1 (Lehe: k 2..mz-2, see the oracle for why).  T = double is the
-// reference form; T = float the FP32 form (same expressions).
-// Each thread walks kCylZChunk consecutive k of its (i, j) column, so the
-// planes its stencil reads above and below were loaded by its CTA one step
-// earlier and come from L1 rather than L2.
-constexpr int kCylZChunk = 16;
-
-// i from 4 on the rank holding the axis (its cells 3 take the axis
-// updates), from 1 elsewhere (cyl_em_update.F90:49-51).
-template <typename T, int FDTD>
-__global__ void k_cyl_bhalf(GridP g, CylP cp, const T *__restrict__ Ex, const T *__restrict__ Ey,
-                            const T *__restrict__ Ez, T *Bx, T *By, T *Bz)
+// The field phases write every periodic image with the cell itself: the
+// halo (y faces over all x, then z faces over all x and y) of an update that
+// only reads other fields is a copy of the interior cell to its theta and z
+// images, so it needs no launch of its own.  The columns of r that an update
+// leaves alone (ghosts, the axis) copy their images too, as the halo does.
+// The axis conditions read the updated cells next to the axis of two
+// opposite theta and follow in a small launch (k_cyl_axis).  With separate
+// launches for axis, halo, fold and the zeroing of J a step had 49 of them
+// (nr 64, 8 theta, nz 512, FP64: 314 us of a 868 us step; now 6 and
+// 92 us).
+template <typename T>
+__device__ __forceinline__ void store_yz(const GridP &g, T *F, int i, int j, int k, T v, bool own = true)
 {
-    const int i = (g.inc_axis ? 4 : 1) + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    if (i > g.mx - 1 || j > g.my - 1) return;
-    const int k0 = (FDTD == PIC_FDTD_LEHE ? 2 : 1) + blockIdx.z * kCylZChunk;
-    const int k1 = min(k0 + kCylZChunk - 1, FDTD == PIC_FDTD_LEHE ? g.mz - 2 : g.mz - 1);
+    const int jj = image_of(j, g.my), kk = image_of(k, g.mz);
+    if (own) F[cidx(g, i, j, k)] = v;
+    if (jj) F[cidx(g, i, jj, k)] = v;
+    if (kk) F[cidx(g, i, j, kk)] = v;
+    if (jj && kk) F[cidx(g, i, jj, kk)] = v;
+}
+template <typename T>
+__device__ __forceinline__ void copy_yz(const GridP &g, T *F, int i, int j, int k)
+{
+    if (image_of(j, g.my) || image_of(k, g.mz)) store_yz(g, F, i, j, k, F[cidx(g, i, j, k)], false);
+}
+
+// UpdateBfieldHalf main loop (cyl_em_update.F90:66-83; Lehe
+// cyl_em_update_lehe.F90:62-118) on the interior theta and z: i 4..mx-1 on
+// the rank holding the axis (its cells 3 take the axis updates), from 1
+// elsewhere (cyl_em_update.F90:49-51).  T = double is the reference form; T =
+// float the FP32 form (same expressions).  Each thread walks kCylZChunk
+// consecutive k of its (i, j) column, so the planes its stencil reads above
+// and below were loaded by its CTA one step earlier and come from L1 rather
+// than L2.
+constexpr int kCylZChunk = 4;
+
+template <typename T, int FDTD>
+__global__ void __launch_bounds__(256) k_cyl_bhalf(GridP g, CylP cp, const T *__restrict__ Ex, const T *__restrict__ Ey,
+                                                   const T *__restrict__ Ez, T *Bx, T *By, T *Bz)
+{
+    const int i = 1 + blockIdx.x * 32 + threadIdx.x, j = 3 + blockIdx.y * 8 + threadIdx.y;
+    if (i > g.mx || j > g.my - 3) return;
+    const bool upd = i >= (g.inc_axis ? 4 : 1) && i <= g.mx - 1;
+    const int k0 = 3 + blockIdx.z * kCylZChunk, k1 = min(k0 + kCylZChunk - 1, g.mz - 3);
     const T h = (T)g.h, dtheta = (T)cp.dtheta;
     const T r = (((T)i - (T)3.0) + (T)cp.rmin) * (T)1.0;
     const T rp_half = r + (T)0.5 * (T)1.0, rp = r + (T)1.0;
     const long long sy = g.sy, sz = g.sz;
     for (int k = k0; k <= k1; k++) {
         const long long c0 = cidx(g, i, j, k);
-        if (FDTD == PIC_FDTD_YEE) {
-            Bx[c0] = (Bx[c0] - (h * (ldd(Ez + c0 + sy) - ldd(Ez + c0))) / (r * dtheta)) + (h * (T)1.0) * (ldd(Ey + c0 + sz) - ldd(Ey + c0));
-            By[c0] = (By[c0] - (h * (T)1.0) * (ldd(Ex + c0 + sz) - ldd(Ex + c0))) + (h * (T)1.0) * (ldd(Ez + c0 + 1) - ldd(Ez + c0));
-            Bz[c0] = Bz[c0] - (h * (((T)1.0 * (rp * ldd(Ey + c0 + 1) - r * ldd(Ey + c0))) - (ldd(Ex + c0 + sy) - ldd(Ex + c0)) / dtheta)) / rp_half;
-        } else {
-            Bx[c0] = (Bx[c0] - (h * lgy(g, Ez, c0)) / (r * dtheta)) + (h * (T)1.0) * lgz(g, Ey, c0);
-            By[c0] = (By[c0] - (h * (T)1.0) * lgz(g, Ex, c0)) + (h * (T)1.0) * lgx(g, Ez, c0);
-            Bz[c0] = Bz[c0] - (h * (((T)1.0 * lgx1(g, Ey, c0, rp, r)) - lgy(g, Ex, c0) / dtheta)) / rp_half;
+        if (!upd) {
+            copy_yz(g, Bx, i, j, k);
+            copy_yz(g, By, i, j, k);
+            copy_yz(g, Bz, i, j, k);
+            continue;
         }
+        T bx, by, bz;
+        if (FDTD == PIC_FDTD_YEE) {
+            bx = (Bx[c0] - (h * (ldd(Ez + c0 + sy) - ldd(Ez + c0))) / (r * dtheta)) + (h * (T)1.0) * (ldd(Ey + c0 + sz) - ldd(Ey + c0));
+            by = (By[c0] - (h * (T)1.0) * (ldd(Ex + c0 + sz) - ldd(Ex + c0))) + (h * (T)1.0) * (ldd(Ez + c0 + 1) - ldd(Ez + c0));
+            bz = Bz[c0] - (h * (((T)1.0 * (rp * ldd(Ey + c0 + 1) - r * ldd(Ey + c0))) - (ldd(Ex + c0 + sy) - ldd(Ex + c0)) / dtheta)) / rp_half;
+        } else {
+            bx = (Bx[c0] - (h * lgy(g, Ez, c0)) / (r * dtheta)) + (h * (T)1.0) * lgz(g, Ey, c0);
+            by = (By[c0] - (h * (T)1.0) * lgz(g, Ex, c0)) + (h * (T)1.0) * lgx(g, Ez, c0);
+            bz = Bz[c0] - (h * (((T)1.0 * lgx1(g, Ey, c0, rp, r)) - lgy(g, Ex, c0) / dtheta)) / rp_half;
+        }
+        store_yz(g, Bx, i, j, k, bx);
+        store_yz(g, By, i, j, k, by);
+        store_yz(g, Bz, i, j, k, bz);
     }
-}
-
-// UpdateBzAxis (cyl_em_update.F90:231-246) + Bz(3,j,k) = Bz_ax(k): one
-// thread per k sums Ey(4,j,k) over j in the reference's order.
-template <typename T>
-__global__ void k_cyl_bz_axis(GridP g, CylP cp, const T *__restrict__ Ey, T *Bz)
-{
-    const int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > g.mz - 1) return;
-    const T hax = (T)(g.h * cp.ax_perm_area);
-    T s = (T)0.0;
-    for (int j = 3; j <= g.my - 3; j++) s = s - hax * Ey[cidx(g, 4, j, k)];
-    const T v = Bz[cidx(g, 3, 3, k)] + s;
-    for (int j = 1; j <= g.my - 1; j++) Bz[cidx(g, 3, j, k)] = v;
 }
 
 __device__ __forceinline__ int axis_partner(const GridP &g, int j)
@@ -129,82 +150,110 @@ __device__ __forceinline__ int axis_partner(const GridP &g, int j)
     return p;
 }
 
-// UpdateBFldAxis (cyl_em_update.F90:187-227), all j, k.
+// The axis conditions and their images, one thread per interior (theta, z):
+// UpdateBFldAxis (cyl_em_update.F90:187-227) and, by the thread of the first
+// theta, UpdateBzAxis (:231-246: the circulation of Ey(4) summed over theta
+// in the reference's order) with Bz(3,j,k) = Bz_ax(k).
 template <typename T>
-__global__ void k_cyl_b_axis(GridP g, T *Bx, T *By, T *Bz)
+__global__ void k_cyl_b_axis(GridP g, CylP cp, const T *__restrict__ Ey, T *Bx, T *By, T *Bz)
 {
-    const int j = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = 1 + blockIdx.y;
-    if (j > g.my) return;
+    const int j = 3 + blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = 3 + blockIdx.y * blockDim.y + threadIdx.y;
+    if (j > g.my - 3 || k > g.mz - 3) return;
+    if (j == 3) {
+        const T hax = (T)(g.h * cp.ax_perm_area);
+        T s = (T)0.0;
+        for (int t = 3; t <= g.my - 3; t++) s = s - hax * Ey[cidx(g, 4, t, k)];
+        const T v = Bz[cidx(g, 3, 3, k)] + s;
+        for (int t = 3; t <= g.my - 3; t++) store_yz(g, Bz, 3, t, k, v);
+    }
     const int jpp = axis_partner(g, j);
-    By[cidx(g, 3, j, k)] = (T)0.5 * (By[cidx(g, 4, j, k)] - By[cidx(g, 4, jpp, k)]);
-    By[cidx(g, 2, j, k)] = -By[cidx(g, 4, jpp, k)];
-    Bx[cidx(g, 3, j, k)] = -Bx[cidx(g, 4, jpp, k)];
-    Bz[cidx(g, 2, j, k)] = Bz[cidx(g, 4, jpp, k)];
+    const T by = By[cidx(g, 4, j, k)], byp = By[cidx(g, 4, jpp, k)];
+    store_yz(g, By, 3, j, k, (T)0.5 * (by - byp));
+    store_yz(g, By, 2, j, k, -byp);
+    store_yz(g, Bx, 3, j, k, -Bx[cidx(g, 4, jpp, k)]);
+    store_yz(g, Bz, 2, j, k, Bz[cidx(g, 4, jpp, k)]);
 }
 
-// UpdateEFldAxis (cyl_em_update.F90:143-185), all j, k.
+// UpdateEFldAxis (cyl_em_update.F90:143-185) and its images.
 template <typename T>
 __global__ void k_cyl_e_axis(GridP g, T *Ex, T *Ey, T *Ez)
 {
-    const int j = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = 1 + blockIdx.y;
-    if (j > g.my) return;
+    const int j = 3 + blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = 3 + blockIdx.y * blockDim.y + threadIdx.y;
+    if (j > g.my - 3 || k > g.mz - 3) return;
     const int jpp = axis_partner(g, j);
-    Ex[cidx(g, 3, j, k)] = (T)0.5 * (Ex[cidx(g, 4, j, k)] - Ex[cidx(g, 4, jpp, k)]);
-    Ex[cidx(g, 2, j, k)] = -Ex[cidx(g, 4, jpp, k)];
-    Ey[cidx(g, 3, j, k)] = -Ey[cidx(g, 4, jpp, k)];
-    Ez[cidx(g, 3, j, k)] = Ez[cidx(g, 4, jpp, k)];
+    const T ex = Ex[cidx(g, 4, j, k)], exp_ = Ex[cidx(g, 4, jpp, k)];
+    store_yz(g, Ex, 3, j, k, (T)0.5 * (ex - exp_));
+    store_yz(g, Ex, 2, j, k, -exp_);
+    store_yz(g, Ey, 3, j, k, -Ey[cidx(g, 4, jpp, k)]);
+    store_yz(g, Ez, 3, j, k, Ez[cidx(g, 4, jpp, k)]);
 }
 
-// UpdateEfield (MODE 0, cyl_em_update.F90:24-41) or AddCurrent (MODE 2,
-// :128-137): i 4..mx-3 on the rank holding the axis, 3..mx-3 elsewhere;
-// j, k 3..m-3.
-template <typename T, int MODE>
-__global__ void k_cyl_e(GridP g, CylP cp, T *Ex, T *Ey, T *Ez, const T *__restrict__ Bx, const T *__restrict__ By,
-                        const T *__restrict__ Bz, const T *__restrict__ Jx, const T *__restrict__ Jy,
-                        const T *__restrict__ Jz)
+// The current of (i, j, k) with its periodic images: z first, then theta, as
+// the fold's two passes add them.
+template <typename T>
+__device__ __forceinline__ T fold_yz(const GridP &g, const T *J, int i, int j, int k)
 {
-    const int i = (g.inc_axis ? 4 : 3) + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 3 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = 3 + blockIdx.z;
-    if (i > g.mx - 3 || j > g.my - 3) return;
-    const T dtheta = (T)cp.dtheta;
-    const T r = (((T)i - (T)3.0) + (T)cp.rmin) * (T)1.0;
-    const T rp_half = r + (T)0.5 * (T)1.0, rm_half = r - (T)0.5 * (T)1.0;
-    const long long c0 = cidx(g, i, j, k);
-    if (MODE == 0) {
-        const T fc = (T)g.fc;
-        Ex[c0] = (Ex[c0] + (fc * (ldd(Bz + c0) - ldd(Bz + c0 - g.sy))) / (rp_half * dtheta)) - (fc * (T)1.0) * (ldd(By + c0) - ldd(By + c0 - g.sz));
-        Ey[c0] = (Ey[c0] + (fc * (T)1.0) * (ldd(Bx + c0) - ldd(Bx + c0 - g.sz))) - (fc * (T)1.0) * (ldd(Bz + c0) - ldd(Bz + c0 - 1));
-        Ez[c0] = (Ez[c0] + ((fc * (T)1.0) * (rp_half * ldd(By + c0) - rm_half * ldd(By + c0 - 1))) / r) - (fc * (ldd(Bx + c0) - ldd(Bx + c0 - g.sy))) / (r * dtheta);
-    } else {
-        Ex[c0] = Ex[c0] - (ldd(Jx + c0) * (T)1.0) / (rp_half * dtheta);
-        Ey[c0] = Ey[c0] - (ldd(Jy + c0) * (T)1.0) * (T)1.0;
-        Ez[c0] = Ez[c0] - (ldd(Jz + c0) * (T)1.0) / (r * dtheta);
+    const int jj = image_of(j, g.my), kk = image_of(k, g.mz);
+    T v = J[cidx(g, i, j, k)];
+    if (kk) v = v + J[cidx(g, i, j, kk)];
+    if (jj) {
+        T w = J[cidx(g, i, jj, k)];
+        if (kk) w = w + J[cidx(g, i, jj, kk)];
+        v = v + w;
     }
+    return v;
 }
 
-// Halo along y over x 1..mx and z 3..mz-3, then along z over all x, y.
-template <typename T>
-__global__ void k_cyl_halo_y(GridP g, T *F)
+// UpdateEfield (cyl_em_update.F90:24-41, MODE 0), AddCurrent of a folded J
+// (:128-137, MODE 2), or both with the fold of J and its zeroing (MODE 1, the
+// step): i 4..mx-3 on the rank holding the axis, 3..mx-3 elsewhere.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256) k_cyl_e(GridP g, CylP cp, T *Ex, T *Ey, T *Ez, const T *__restrict__ Bx,
+                                               const T *__restrict__ By, const T *__restrict__ Bz, T *Jx, T *Jy, T *Jz)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = 3 + blockIdx.y;
-    if (i > g.mx) return;
-    const int m = g.my;
-    for (int l = 0; l < 3; l++) F[cidx(g, i, m - 2 + l, k)] = F[cidx(g, i, 3 + l, k)];
-    for (int l = 0; l < 2; l++) F[cidx(g, i, 1 + l, k)] = F[cidx(g, i, m - 4 + l, k)];
-}
-template <typename T>
-__global__ void k_cyl_halo_z(GridP g, T *F)
-{
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y;
-    if (i > g.mx) return;
-    const int m = g.mz;
-    for (int l = 0; l < 3; l++) F[cidx(g, i, j, m - 2 + l)] = F[cidx(g, i, j, 3 + l)];
-    for (int l = 0; l < 2; l++) F[cidx(g, i, j, 1 + l)] = F[cidx(g, i, j, m - 4 + l)];
+    const int i = 1 + blockIdx.x * 32 + threadIdx.x, j = 3 + blockIdx.y * 8 + threadIdx.y, k = 3 + blockIdx.z;
+    if (i > g.mx || j > g.my - 3) return;
+    const long long c0 = cidx(g, i, j, k);
+    if (i >= (g.inc_axis ? 4 : 3) && i <= g.mx - 3) {
+        const T dtheta = (T)cp.dtheta;
+        const T r = (((T)i - (T)3.0) + (T)cp.rmin) * (T)1.0;
+        const T rp_half = r + (T)0.5 * (T)1.0, rm_half = r - (T)0.5 * (T)1.0;
+        T ex = Ex[c0], ey = Ey[c0], ez = Ez[c0], jx = (T)0, jy = (T)0, jz = (T)0;
+        if (MODE == 1) {
+            jx = fold_yz(g, Jx, i, j, k);
+            jy = fold_yz(g, Jy, i, j, k);
+            jz = fold_yz(g, Jz, i, j, k);
+        } else if (MODE == 2) {
+            jx = Jx[c0];
+            jy = Jy[c0];
+            jz = Jz[c0];
+        }
+        if (MODE != 2) {
+            const T fc = (T)g.fc;
+            ex = (ex + (fc * (ldd(Bz + c0) - ldd(Bz + c0 - g.sy))) / (rp_half * dtheta)) - (fc * (T)1.0) * (ldd(By + c0) - ldd(By + c0 - g.sz));
+            ey = (ey + (fc * (T)1.0) * (ldd(Bx + c0) - ldd(Bx + c0 - g.sz))) - (fc * (T)1.0) * (ldd(Bz + c0) - ldd(Bz + c0 - 1));
+            ez = (ez + ((fc * (T)1.0) * (rp_half * ldd(By + c0) - rm_half * ldd(By + c0 - 1))) / r) - (fc * (ldd(Bx + c0) - ldd(Bx + c0 - g.sy))) / (r * dtheta);
+        }
+        if (MODE != 0) {
+            ex = ex - (jx * (T)1.0) / (rp_half * dtheta);
+            ey = ey - (jy * (T)1.0) * (T)1.0;
+            ez = ez - (jz * (T)1.0) / (r * dtheta);
+        }
+        store_yz(g, Ex, i, j, k, ex);
+        store_yz(g, Ey, i, j, k, ey);
+        store_yz(g, Ez, i, j, k, ez);
+    } else {
+        copy_yz(g, Ex, i, j, k);
+        copy_yz(g, Ey, i, j, k);
+        copy_yz(g, Ez, i, j, k);
+    }
+    if (MODE == 1) {   // ResetCurrent
+        store_yz(g, Jx, i, j, k, (T)0);
+        store_yz(g, Jy, i, j, k, (T)0);
+        store_yz(g, Jz, i, j, k, (T)0);
+    }
 }
 
 // Current fold: z faces over all x, y, then y faces over x 1..mx, z 3..mz-3.
@@ -246,50 +295,43 @@ static CylP cyl_params(const GridP &g)
     return c;
 }
 
-template <typename T>
-static void halo(const GridP &g, T *const F[3], cudaStream_t s)
-{
-    for (int c = 0; c < 3; c++) {
-        k_cyl_halo_y<T><<<dim3((g.mx + 127) / 128, g.mz - 5), 128, 0, s>>>(g, F[c]);
-        k_cyl_halo_z<T><<<dim3((g.mx + 127) / 128, g.my), 128, 0, s>>>(g, F[c]);
-    }
-    count_launches(6);
-}
+// Grid of the (theta, z) threads of an axis kernel.
+static dim3 axis_grid(const GridP &g, dim3 block) { return dim3((g.ny + block.x - 1) / block.x, (g.nz + block.y - 1) / block.y); }
+constexpr int kAxisJ = 8, kAxisK = 16;
 
 template <typename T>
 void launch_cyl_bhalf(const GridP &g, T *const E[3], T *const B[3], cudaStream_t s)
 {
     const CylP cp = cyl_params(g);
-    const int nk = g.fdtd == PIC_FDTD_LEHE ? g.mz - 3 : g.mz - 1;
-    const int ni = g.mx - (g.inc_axis ? 4 : 1);   // i .. mx-1
-    const dim3 grid((ni + 31) / 32, (g.my - 1 + 3) / 4, (nk + kCylZChunk - 1) / kCylZChunk), block(32, 4, 1);
+    const dim3 grid((g.mx + 31) / 32, (g.ny + 7) / 8, (g.nz + kCylZChunk - 1) / kCylZChunk), block(32, 8, 1);
     if (g.fdtd == PIC_FDTD_LEHE)
         k_cyl_bhalf<T, PIC_FDTD_LEHE><<<grid, block, 0, s>>>(g, cp, E[0], E[1], E[2], B[0], B[1], B[2]);
     else
         k_cyl_bhalf<T, PIC_FDTD_YEE><<<grid, block, 0, s>>>(g, cp, E[0], E[1], E[2], B[0], B[1], B[2]);
     count_launches(1);
     if (g.inc_axis) {   // cyl_em_update.F90:85-105
-        k_cyl_bz_axis<T><<<(g.mz + 127) / 128, 128, 0, s>>>(g, cp, E[1], B[2]);
-        k_cyl_b_axis<T><<<dim3((g.my + 127) / 128, g.mz), 128, 0, s>>>(g, B[0], B[1], B[2]);
-        count_launches(2);
+        const dim3 ab(kAxisJ, kAxisK);
+        k_cyl_b_axis<T><<<axis_grid(g, ab), ab, 0, s>>>(g, cp, E[1], B[0], B[1], B[2]);
+        count_launches(1);
     }
-    halo<T>(g, B, s);
 }
 
 template <typename T>
 void launch_cyl_efield(const GridP &g, int mode, T *const E[3], T *const B[3], T *const J[3], cudaStream_t s)
 {
     const CylP cp = cyl_params(g);
-    const int ni = g.mx - 2 - (g.inc_axis ? 4 : 3);   // i .. mx-3
-    const dim3 grid((ni + 31) / 32, (g.my - 5 + 7) / 8, g.mz - 5), block(32, 8, 1);
-    if (mode == 0) k_cyl_e<T, 0><<<grid, block, 0, s>>>(g, cp, E[0], E[1], E[2], B[0], B[1], B[2], J[0], J[1], J[2]);
-    else k_cyl_e<T, 2><<<grid, block, 0, s>>>(g, cp, E[0], E[1], E[2], B[0], B[1], B[2], J[0], J[1], J[2]);
+    const dim3 grid((g.mx + 31) / 32, (g.ny + 7) / 8, g.nz), block(32, 8, 1);
+#define LE(M) k_cyl_e<T, M><<<grid, block, 0, s>>>(g, cp, E[0], E[1], E[2], B[0], B[1], B[2], J[0], J[1], J[2])
+    if (mode == 0) LE(0);
+    else if (mode == 1) LE(1);
+    else LE(2);
+#undef LE
     count_launches(1);
     if (g.inc_axis) {   // UpdateEFldAxis
-        k_cyl_e_axis<T><<<dim3((g.my + 127) / 128, g.mz), 128, 0, s>>>(g, E[0], E[1], E[2]);
+        const dim3 ab(kAxisJ, kAxisK);
+        k_cyl_e_axis<T><<<axis_grid(g, ab), ab, 0, s>>>(g, E[0], E[1], E[2]);
         count_launches(1);
     }
-    halo<T>(g, E, s);
 }
 
 template <typename T>

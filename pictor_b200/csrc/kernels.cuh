@@ -39,9 +39,10 @@ template <typename T>
 void launch_cyl_fold(const GridP &g, T *const J[3], cudaStream_t s);
 // modal.cu: the cylindrical field solve on azimuthal modes m = 0, 1 (arrays (mx, 3, mz))
 template <typename T>
-void launch_modal_bhalf(const GridP &g, T *const Em[3], T *const Bm[3], cudaStream_t s);
+void launch_modal_bhalf(const GridP &g, T *const B[3], T *const Em[3], T *const Bm[3], cudaStream_t s);
 template <typename T>
-void launch_modal_efield(const GridP &g, int mode, T *const Em[3], T *const Bm[3], T *const Jm[3], cudaStream_t s);
+void launch_modal_efield(const GridP &g, int mode, T *const E[3], T *const J[3], T *const Em[3], T *const Bm[3],
+                         cudaStream_t s);
 template <typename T>
 void launch_modal_synth(const GridP &g, T *const Fm[3], T *const F[3], cudaStream_t s);
 template <typename T>

@@ -20,7 +20,7 @@
 // On fields whose theta content is m <= 1 the result equals the
 // theta-gridded update to round-off.  The particles keep the reference's
 // theta-gridded mover: the theta-gridded E and B it gathers from are
-// synthesised from the modes after every field update, and the current it
+// synthesised from the modes by every field update, and the current it
 // deposits (after the fold) is projected onto the modes before AddCurrent.
 // The projection of a charge-conserving current is charge-conserving mode by
 // mode (the continuity equation is theta-shift invariant), so the truncated
@@ -28,6 +28,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "field_math.cuh"
 #include "kernels.cuh"
 
 namespace pic {
@@ -127,146 +128,196 @@ __device__ __forceinline__ M3<T> mgz(const GridP &gm, const ModalP &m, const T *
     return r;
 }
 
-// B half step (cyl_em_update.F90:66-83; Lehe :62-118): i 4..mx-1, k 1..mz-1
-// (Lehe 2..mz-2).
+// cos and sin of the ny theta angles, in the block's shared memory (dynamic,
+// 2 ny doubles): the synthesis of a column needs all of them, and sincospi in
+// FP64 costs more than the rest of the update.
+__device__ __forceinline__ void theta_table(const ModalP &m, double *cs, double *sn)
+{
+    for (int t = threadIdx.x + blockDim.x * threadIdx.y; t < m.ny; t += blockDim.x * blockDim.y)
+        sincospi(2.0 * (double)t / (double)m.ny, &sn[t], &cs[t]);
+    __syncthreads();
+}
+
+// v into the planes Fm and its synthesis into the theta-gridded F at (i, k),
+// with the z images of both and the theta ghosts.
+template <typename T>
+__device__ __forceinline__ void emit(const GridP &g, const GridP &gm, const double *cs, const double *sn, T *Fm, T *F,
+                                     int i, int k, M3<T> v)
+{
+    const int kk = image_of(k, g.mz);
+    st3(gm, Fm, i, k, v);
+    if (kk) st3(gm, Fm, i, kk, v);
+    for (int j = 3; j <= g.my - 3; j++) {
+        const T f = v.a + v.b * (T)cs[j - 3] + v.c * (T)sn[j - 3];
+        const int jj = image_of(j, g.my);
+        F[cidx(g, i, j, k)] = f;
+        if (jj) F[cidx(g, i, jj, k)] = f;
+        if (kk) F[cidx(g, i, j, kk)] = f;
+        if (jj && kk) F[cidx(g, i, jj, kk)] = f;
+    }
+}
+
+// The B and E phases: one thread per interior (r, z) updates the planes of
+// its cell, applies the axis conditions (the thread next to the axis, whose
+// new values they are made of) and writes the planes, their theta-gridded
+// synthesis and all images; the columns an update leaves alone are emitted as
+// they are.  With launches for the update, the axis, the halo, the synthesis,
+// the fold and the projection each, a step had 43 of them (nr 128, nz 1024,
+// FP32: 379 us of a 877 us step; now 3 and 114 us).
+
+// B half step (cyl_em_update.F90:66-83; Lehe :62-118): i 4..mx-1; then
+// UpdateBzAxis (:231-246: the circulation of Ey(4, :, k) is ny times its m = 0
+// plane, and Bz on the axis has no m = 1 part) and UpdateBFldAxis (:187-227).
 template <typename T, int FDTD>
-__global__ void k_modal_bhalf(GridP gm, ModalP m, const T *__restrict__ Ex, const T *__restrict__ Ey,
-                              const T *__restrict__ Ez, T *Bx, T *By, T *Bz)
+__global__ void __launch_bounds__(128) k_modal_bhalf(GridP g, GridP gm, ModalP m, const T *__restrict__ Ex,
+                                                     const T *__restrict__ Ey, const T *__restrict__ Ez, T *Bx, T *By,
+                                                     T *Bz, T *Fx, T *Fy, T *Fz)
 {
-    const int i = 4 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = (FDTD == PIC_FDTD_LEHE ? 2 : 1) + blockIdx.y;
-    if (i > gm.mx - 1) return;
-    const T h = (T)gm.h, dtheta = (T)m.dtheta;
-    const T r = ((T)i - (T)3.0) + (T)m.rmin;
-    const T rp_half = r + (T)0.5, rp = r + (T)1.0;
-    if (FDTD == PIC_FDTD_YEE) {
-        const M3<T> ez = ld3(gm, Ez, i, k), ex = ld3(gm, Ex, i, k), ey = ld3(gm, Ey, i, k);
-        const M3<T> bx = ld3(gm, Bx, i, k) - (h * (tp(m, ez) - ez)) / (r * dtheta) + h * (ld3(gm, Ey, i, k + 1) - ey);
-        const M3<T> by = ld3(gm, By, i, k) - h * (ld3(gm, Ex, i, k + 1) - ex) + h * (ld3(gm, Ez, i + 1, k) - ez);
-        const M3<T> bz = ld3(gm, Bz, i, k) - (h * ((rp * ld3(gm, Ey, i + 1, k) - r * ey) - (tp(m, ex) - ex) / dtheta)) / rp_half;
-        st3(gm, Bx, i, k, bx);
-        st3(gm, By, i, k, by);
-        st3(gm, Bz, i, k, bz);
-    } else {
-        const M3<T> bx = ld3(gm, Bx, i, k) - (h * mgy(gm, m, Ez, i, k)) / (r * dtheta) + h * mgz(gm, m, Ey, i, k);
-        const M3<T> by = ld3(gm, By, i, k) - h * mgz(gm, m, Ex, i, k) + h * mgx(gm, Ez, i, k);
-        const M3<T> bz = ld3(gm, Bz, i, k) - (h * (mgx1(gm, Ey, i, k, rp, r) - mgy(gm, m, Ex, i, k) / dtheta)) / rp_half;
-        st3(gm, Bx, i, k, bx);
-        st3(gm, By, i, k, by);
-        st3(gm, Bz, i, k, bz);
+    extern __shared__ double tab[];
+    const double *cs = tab, *sn = tab + m.ny;
+    theta_table(m, tab, tab + m.ny);
+    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, k = 3 + blockIdx.y * blockDim.y + threadIdx.y;
+    if (i > gm.mx || k > gm.mz - 3 || i == 3) return;   // column 3 belongs to the thread of column 4
+    M3<T> bx = ld3(gm, Bx, i, k), by = ld3(gm, By, i, k), bz = ld3(gm, Bz, i, k);
+    if (i >= 4 && i <= gm.mx - 1) {
+        const T h = (T)gm.h, dtheta = (T)m.dtheta;
+        const T r = ((T)i - (T)3.0) + (T)m.rmin;
+        const T rp_half = r + (T)0.5, rp = r + (T)1.0;
+        if (FDTD == PIC_FDTD_YEE) {
+            const M3<T> ez = ld3(gm, Ez, i, k), ex = ld3(gm, Ex, i, k), ey = ld3(gm, Ey, i, k);
+            bx = bx - (h * (tp(m, ez) - ez)) / (r * dtheta) + h * (ld3(gm, Ey, i, k + 1) - ey);
+            by = by - h * (ld3(gm, Ex, i, k + 1) - ex) + h * (ld3(gm, Ez, i + 1, k) - ez);
+            bz = bz - (h * ((rp * ld3(gm, Ey, i + 1, k) - r * ey) - (tp(m, ex) - ex) / dtheta)) / rp_half;
+        } else {
+            bx = bx - (h * mgy(gm, m, Ez, i, k)) / (r * dtheta) + h * mgz(gm, m, Ey, i, k);
+            by = by - h * mgz(gm, m, Ex, i, k) + h * mgx(gm, Ez, i, k);
+            bz = bz - (h * (mgx1(gm, Ey, i, k, rp, r) - mgy(gm, m, Ex, i, k) / dtheta)) / rp_half;
+        }
     }
+    if (i == 4) {
+        const T s = -(T)(gm.h * m.ax_perm_area) * ((T)m.ny * ld3(gm, Ey, 4, k).a);
+        emit<T>(g, gm, cs, sn, Bz, Fz, 3, k, {ld3(gm, Bz, 3, k).a + s, (T)0, (T)0});
+        emit(g, gm, cs, sn, By, Fy, 3, k, ((T)0.5 * (by - partner(by))));
+        emit<T>(g, gm, cs, sn, By, Fy, 2, k, {-by.a, by.b, by.c});
+        emit<T>(g, gm, cs, sn, Bx, Fx, 3, k, {-bx.a, bx.b, bx.c});
+        emit(g, gm, cs, sn, Bz, Fz, 2, k, partner(bz));
+    }
+    emit(g, gm, cs, sn, Bx, Fx, i, k, bx);
+    if (i == 2) return;   // By and Bz of column 2: above
+    emit(g, gm, cs, sn, By, Fy, i, k, by);
+    emit(g, gm, cs, sn, Bz, Fz, i, k, bz);
 }
 
-// UpdateBzAxis (cyl_em_update.F90:231-246): the circulation of Ey(4, :, k)
-// is ny times its m = 0 plane; Bz on the axis has no m = 1 part.
-template <typename T>
-__global__ void k_modal_bz_axis(GridP gm, ModalP m, const T *__restrict__ Ey, T *Bz)
+// Modes of the theta-gridded J at (i, k): a = mean, b = 2/ny sum J cos, c =
+// 2/ny sum J sin over the ny interior theta cells (summed in FP64); FOLD: of
+// J with its periodic images added (z first, then theta).
+template <typename T, bool FOLD>
+__device__ __forceinline__ M3<T> project(const GridP &g, const ModalP &m, const double *cs, const double *sn, const T *J,
+                                         int i, int k)
 {
-    const int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > gm.mz - 1) return;
-    const T s = -(T)(gm.h * m.ax_perm_area) * ((T)m.ny * ld3(gm, Ey, 4, k).a);
-    st3<T>(gm, Bz, 3, k, {ld3(gm, Bz, 3, k).a + s, (T)0, (T)0});
+    const int kk = FOLD ? image_of(k, g.mz) : 0;
+    double a = 0.0, b = 0.0, c = 0.0;
+    for (int t = 0; t < m.ny; t++) {
+        const int j = 3 + t;
+        T f = J[cidx(g, i, j, k)];
+        if (FOLD) {
+            const int jj = image_of(j, g.my);
+            if (kk) f = f + J[cidx(g, i, j, kk)];
+            if (jj) {
+                T w = J[cidx(g, i, jj, k)];
+                if (kk) w = w + J[cidx(g, i, jj, kk)];
+                f = f + w;
+            }
+        }
+        const double v = (double)f;
+        a += v;
+        b += v * cs[t];
+        c += v * sn[t];
+    }
+    const double inv = 1.0 / (double)m.ny;
+    return {(T)(a * inv), (T)(2.0 * b * inv), (T)(2.0 * c * inv)};
 }
 
-// UpdateBFldAxis / UpdateEFldAxis (cyl_em_update.F90:143-227) on modes.
-template <typename T>
-__global__ void k_modal_b_axis(GridP gm, T *Bx, T *By, T *Bz)
-{
-    const int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > gm.mz) return;
-    const M3<T> by4 = ld3(gm, By, 4, k), bx4 = ld3(gm, Bx, 4, k), bz4 = ld3(gm, Bz, 4, k);
-    st3(gm, By, 3, k, (T)0.5 * (by4 - partner(by4)));
-    st3<T>(gm, By, 2, k, {-by4.a, by4.b, by4.c});
-    st3<T>(gm, Bx, 3, k, {-bx4.a, bx4.b, bx4.c});
-    st3(gm, Bz, 2, k, partner(bz4));
-}
-template <typename T>
-__global__ void k_modal_e_axis(GridP gm, T *Ex, T *Ey, T *Ez)
-{
-    const int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > gm.mz) return;
-    const M3<T> ex4 = ld3(gm, Ex, 4, k), ey4 = ld3(gm, Ey, 4, k), ez4 = ld3(gm, Ez, 4, k);
-    st3(gm, Ex, 3, k, (T)0.5 * (ex4 - partner(ex4)));
-    st3<T>(gm, Ex, 2, k, {-ex4.a, ex4.b, ex4.c});
-    st3<T>(gm, Ey, 3, k, {-ey4.a, ey4.b, ey4.c});
-    st3(gm, Ez, 3, k, partner(ez4));
-}
-
-// UpdateEfield (MODE 0, cyl_em_update.F90:24-41) or AddCurrent (MODE 2,
-// :128-137) on modes: i 4..mx-3, k 3..mz-3.
+// UpdateEfield (cyl_em_update.F90:24-41, MODE 0), AddCurrent of a folded J
+// (:128-137, MODE 2), or both with the fold and the zeroing of J (MODE 1, the
+// step) on modes: i 4..mx-3; then UpdateEFldAxis (:143-185).
 template <typename T, int MODE>
-__global__ void k_modal_e(GridP gm, ModalP m, T *Ex, T *Ey, T *Ez, const T *__restrict__ Bx, const T *__restrict__ By,
-                          const T *__restrict__ Bz, const T *__restrict__ Jx, const T *__restrict__ Jy,
-                          const T *__restrict__ Jz)
+__global__ void __launch_bounds__(128) k_modal_e(GridP g, GridP gm, ModalP m, T *Ex, T *Ey, T *Ez,
+                                                 const T *__restrict__ Bx, const T *__restrict__ By,
+                                                 const T *__restrict__ Bz, T *Jx, T *Jy, T *Jz, T *Fx, T *Fy, T *Fz)
 {
-    const int i = 4 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = 3 + blockIdx.y;
-    if (i > gm.mx - 3) return;
-    const T dtheta = (T)m.dtheta;
-    const T r = ((T)i - (T)3.0) + (T)m.rmin;
-    const T rp_half = r + (T)0.5, rm_half = r - (T)0.5;
-    if (MODE == 0) {
-        const T fc = (T)gm.fc;
-        const M3<T> bz = ld3(gm, Bz, i, k), by = ld3(gm, By, i, k), bx = ld3(gm, Bx, i, k);
-        st3(gm, Ex, i, k, ld3(gm, Ex, i, k) + (fc * (bz - tm(m, bz))) / (rp_half * dtheta) - fc * (by - ld3(gm, By, i, k - 1)));
-        st3(gm, Ey, i, k, ld3(gm, Ey, i, k) + fc * (bx - ld3(gm, Bx, i, k - 1)) - fc * (bz - ld3(gm, Bz, i - 1, k)));
-        st3(gm, Ez, i, k,
-            ld3(gm, Ez, i, k) + (fc * (rp_half * by - rm_half * ld3(gm, By, i - 1, k))) / r - (fc * (bx - tm(m, bx))) / (r * dtheta));
-    } else {
-        st3(gm, Ex, i, k, ld3(gm, Ex, i, k) - ld3(gm, Jx, i, k) / (rp_half * dtheta));
-        st3(gm, Ey, i, k, ld3(gm, Ey, i, k) - ld3(gm, Jy, i, k));
-        st3(gm, Ez, i, k, ld3(gm, Ez, i, k) - ld3(gm, Jz, i, k) / (r * dtheta));
+    extern __shared__ double tab[];
+    const double *cs = tab, *sn = tab + m.ny;
+    theta_table(m, tab, tab + m.ny);
+    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, k = 3 + blockIdx.y * blockDim.y + threadIdx.y;
+    if (i > gm.mx || k > gm.mz - 3) return;
+    M3<T> ex = ld3(gm, Ex, i, k), ey = ld3(gm, Ey, i, k), ez = ld3(gm, Ez, i, k);
+    if (i >= 4 && i <= gm.mx - 3) {
+        const T dtheta = (T)m.dtheta;
+        const T r = ((T)i - (T)3.0) + (T)m.rmin;
+        const T rp_half = r + (T)0.5, rm_half = r - (T)0.5;
+        if (MODE != 2) {
+            const T fc = (T)gm.fc;
+            const M3<T> bz = ld3(gm, Bz, i, k), by = ld3(gm, By, i, k), bx = ld3(gm, Bx, i, k);
+            ex = ex + (fc * (bz - tm(m, bz))) / (rp_half * dtheta) - fc * (by - ld3(gm, By, i, k - 1));
+            ey = ey + fc * (bx - ld3(gm, Bx, i, k - 1)) - fc * (bz - ld3(gm, Bz, i - 1, k));
+            ez = ez + (fc * (rp_half * by - rm_half * ld3(gm, By, i - 1, k))) / r - (fc * (bx - tm(m, bx))) / (r * dtheta);
+        }
+        if (MODE != 0) {
+            ex = ex - project<T, MODE == 1>(g, m, cs, sn, Jx, i, k) / (rp_half * dtheta);
+            ey = ey - project<T, MODE == 1>(g, m, cs, sn, Jy, i, k);
+            ez = ez - project<T, MODE == 1>(g, m, cs, sn, Jz, i, k) / (r * dtheta);
+        }
     }
+    if (MODE == 1) {   // ResetCurrent
+        const int kk = image_of(k, g.mz);
+        for (int j = 1; j <= g.my; j++) {
+            const long long c = cidx(g, i, j, k);
+            Jx[c] = Jy[c] = Jz[c] = (T)0;
+            if (kk) {
+                const long long d = cidx(g, i, j, kk);
+                Jx[d] = Jy[d] = Jz[d] = (T)0;
+            }
+        }
+    }
+    if (i == 3) return;   // column 3 belongs to the thread of column 4
+    if (i == 4) {
+        emit(g, gm, cs, sn, Ex, Fx, 3, k, (T)0.5 * (ex - partner(ex)));
+        emit<T>(g, gm, cs, sn, Ex, Fx, 2, k, {-ex.a, ex.b, ex.c});
+        emit<T>(g, gm, cs, sn, Ey, Fy, 3, k, {-ey.a, ey.b, ey.c});
+        emit(g, gm, cs, sn, Ez, Fz, 3, k, partner(ez));
+    }
+    if (i != 2) emit(g, gm, cs, sn, Ex, Fx, i, k, ex);   // Ex of column 2: above
+    emit(g, gm, cs, sn, Ey, Fy, i, k, ey);
+    emit(g, gm, cs, sn, Ez, Fz, i, k, ez);
 }
 
-// Periodic z halo of the modal planes (the layer map of cyl.cu's halo).
-template <typename T>
-__global__ void k_modal_halo_z(GridP gm, T *F)
-{
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int p = 1 + blockIdx.y;
-    if (i > gm.mx) return;
-    const int mz = gm.mz;
-    for (int l = 0; l < 3; l++) F[cidx(gm, i, p, mz - 2 + l)] = F[cidx(gm, i, p, 3 + l)];
-    for (int l = 0; l < 2; l++) F[cidx(gm, i, p, 1 + l)] = F[cidx(gm, i, p, mz - 4 + l)];
-}
-
-// Theta-gridded F(i, j, k) for every ghosted j from the modes at (i, k).
+// Theta-gridded F(i, j, k) for every ghosted j from the modes at (i, k)
+// (loaded fields).
 template <typename T>
 __global__ void k_modal_synth(GridP g, GridP gm, ModalP m, const T *__restrict__ Fm, T *F)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = 1 + blockIdx.y;
-    if (i > g.mx) return;
+    extern __shared__ double tab[];
+    theta_table(m, tab, tab + m.ny);
+    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, k = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+    if (i > g.mx || k > g.mz) return;
     const M3<T> v = ld3(gm, Fm, i, k);
     for (int j = 1; j <= g.my; j++) {
         int t = (j - 3) % m.ny;
         if (t < 0) t += m.ny;
-        double sn, cs;
-        sincospi(2.0 * (double)t / (double)m.ny, &sn, &cs);
-        F[cidx(g, i, j, k)] = v.a + v.b * (T)cs + v.c * (T)sn;
+        F[cidx(g, i, j, k)] = v.a + v.b * (T)tab[t] + v.c * (T)tab[m.ny + t];
     }
 }
 
-// Modes of the theta-gridded F over its ny interior theta cells:
-// a = mean, b = 2/ny sum F cos, c = 2/ny sum F sin (summed in FP64).
+// The modes of a theta-gridded component (loaded fields).
 template <typename T>
 __global__ void k_modal_project(GridP g, GridP gm, ModalP m, const T *__restrict__ F, T *Fm)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = 1 + blockIdx.y;
-    if (i > g.mx) return;
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int t = 0; t < m.ny; t++) {
-        const double v = (double)F[cidx(g, i, 3 + t, k)];
-        double sn, cs;
-        sincospi(2.0 * (double)t / (double)m.ny, &sn, &cs);
-        a += v;
-        b += v * cs;
-        c += v * sn;
-    }
-    const double inv = 1.0 / (double)m.ny;
-    st3<T>(gm, Fm, i, k, {(T)(a * inv), (T)(2.0 * b * inv), (T)(2.0 * c * inv)});
+    extern __shared__ double tab[];
+    theta_table(m, tab, tab + m.ny);
+    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, k = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+    if (i > g.mx || k > g.mz) return;
+    st3<T>(gm, Fm, i, k, project<T, false>(g, m, tab, tab + m.ny, F, i, k));
 }
 
 GridP modal_grid(const GridP &g)
@@ -292,43 +343,45 @@ static ModalP modal_params(const GridP &g)
     return m;
 }
 
-template <typename T>
-static void modal_halo(const GridP &gm, T *const F[3], cudaStream_t s)
+static void modal_shape(const GridP &g, dim3 &grid, dim3 &block, size_t &smem)
 {
-    for (int c = 0; c < 3; c++) k_modal_halo_z<T><<<dim3((gm.mx + 127) / 128, 3), 128, 0, s>>>(gm, F[c]);
-    count_launches(3);
+    block = dim3(32, 4);
+    grid = dim3((g.mx + 31) / 32, (g.nz + 3) / 4);
+    smem = 2 * sizeof(double) * (size_t)g.ny;
+}
+template <typename K>
+static void allow_smem(K k, size_t smem)   // beyond 3072 theta cells
+{
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 template <typename T>
-void launch_modal_bhalf(const GridP &g, T *const Em[3], T *const Bm[3], cudaStream_t s)
+void launch_modal_bhalf(const GridP &g, T *const B[3], T *const Em[3], T *const Bm[3], cudaStream_t s)
 {
     const GridP gm = modal_grid(g);
     const ModalP m = modal_params(g);
-    const int nk = g.fdtd == PIC_FDTD_LEHE ? g.mz - 3 : g.mz - 1;
-    const dim3 grid((g.mx - 4 + 127) / 128, nk);
-    if (g.fdtd == PIC_FDTD_LEHE)
-        k_modal_bhalf<T, PIC_FDTD_LEHE><<<grid, 128, 0, s>>>(gm, m, Em[0], Em[1], Em[2], Bm[0], Bm[1], Bm[2]);
-    else
-        k_modal_bhalf<T, PIC_FDTD_YEE><<<grid, 128, 0, s>>>(gm, m, Em[0], Em[1], Em[2], Bm[0], Bm[1], Bm[2]);
-    k_modal_bz_axis<T><<<(g.mz + 127) / 128, 128, 0, s>>>(gm, m, Em[1], Bm[2]);
-    k_modal_b_axis<T><<<(g.mz + 127) / 128, 128, 0, s>>>(gm, Bm[0], Bm[1], Bm[2]);
-    count_launches(3);
-    modal_halo<T>(gm, Bm, s);
+    dim3 grid, block;
+    size_t sm;
+    modal_shape(g, grid, block, sm);
+    auto k = g.fdtd == PIC_FDTD_LEHE ? k_modal_bhalf<T, PIC_FDTD_LEHE> : k_modal_bhalf<T, PIC_FDTD_YEE>;
+    allow_smem(k, sm);
+    k<<<grid, block, sm, s>>>(g, gm, m, Em[0], Em[1], Em[2], Bm[0], Bm[1], Bm[2], B[0], B[1], B[2]);
+    count_launches(1);
 }
 
 template <typename T>
-void launch_modal_efield(const GridP &g, int mode, T *const Em[3], T *const Bm[3], T *const Jm[3], cudaStream_t s)
+void launch_modal_efield(const GridP &g, int mode, T *const E[3], T *const J[3], T *const Em[3], T *const Bm[3],
+                         cudaStream_t s)
 {
     const GridP gm = modal_grid(g);
     const ModalP m = modal_params(g);
-    const dim3 grid((g.mx - 6 + 127) / 128, g.mz - 5);
-    if (mode == 0)
-        k_modal_e<T, 0><<<grid, 128, 0, s>>>(gm, m, Em[0], Em[1], Em[2], Bm[0], Bm[1], Bm[2], Jm[0], Jm[1], Jm[2]);
-    else
-        k_modal_e<T, 2><<<grid, 128, 0, s>>>(gm, m, Em[0], Em[1], Em[2], Bm[0], Bm[1], Bm[2], Jm[0], Jm[1], Jm[2]);
-    k_modal_e_axis<T><<<(g.mz + 127) / 128, 128, 0, s>>>(gm, Em[0], Em[1], Em[2]);
-    count_launches(2);
-    modal_halo<T>(gm, Em, s);
+    dim3 grid, block;
+    size_t sm;
+    modal_shape(g, grid, block, sm);
+    auto k = mode == 0 ? k_modal_e<T, 0> : mode == 1 ? k_modal_e<T, 1> : k_modal_e<T, 2>;
+    allow_smem(k, sm);
+    k<<<grid, block, sm, s>>>(g, gm, m, Em[0], Em[1], Em[2], Bm[0], Bm[1], Bm[2], J[0], J[1], J[2], E[0], E[1], E[2]);
+    count_launches(1);
 }
 
 template <typename T>
@@ -336,7 +389,10 @@ void launch_modal_synth(const GridP &g, T *const Fm[3], T *const F[3], cudaStrea
 {
     const GridP gm = modal_grid(g);
     const ModalP m = modal_params(g);
-    for (int c = 0; c < 3; c++) k_modal_synth<T><<<dim3((g.mx + 127) / 128, g.mz), 128, 0, s>>>(g, gm, m, Fm[c], F[c]);
+    const dim3 block(32, 4), grid((g.mx + 31) / 32, (g.mz + 3) / 4);
+    const size_t sm = 2 * sizeof(double) * (size_t)g.ny;
+    allow_smem(k_modal_synth<T>, sm);
+    for (int c = 0; c < 3; c++) k_modal_synth<T><<<grid, block, sm, s>>>(g, gm, m, Fm[c], F[c]);
     count_launches(3);
 }
 
@@ -345,16 +401,20 @@ void launch_modal_project(const GridP &g, T *const F[3], T *const Fm[3], cudaStr
 {
     const GridP gm = modal_grid(g);
     const ModalP m = modal_params(g);
-    for (int c = 0; c < 3; c++) k_modal_project<T><<<dim3((g.mx + 127) / 128, g.mz), 128, 0, s>>>(g, gm, m, F[c], Fm[c]);
+    const dim3 block(32, 4), grid((g.mx + 31) / 32, (g.mz + 3) / 4);
+    const size_t sm = 2 * sizeof(double) * (size_t)g.ny;
+    allow_smem(k_modal_project<T>, sm);
+    for (int c = 0; c < 3; c++) k_modal_project<T><<<grid, block, sm, s>>>(g, gm, m, F[c], Fm[c]);
     count_launches(3);
 }
 
-template void launch_modal_bhalf<double>(const GridP &, double *const[3], double *const[3], cudaStream_t);
-template void launch_modal_bhalf<float>(const GridP &, float *const[3], float *const[3], cudaStream_t);
-template void launch_modal_efield<double>(const GridP &, int, double *const[3], double *const[3], double *const[3],
-                                          cudaStream_t);
-template void launch_modal_efield<float>(const GridP &, int, float *const[3], float *const[3], float *const[3],
+template void launch_modal_bhalf<double>(const GridP &, double *const[3], double *const[3], double *const[3],
                                          cudaStream_t);
+template void launch_modal_bhalf<float>(const GridP &, float *const[3], float *const[3], float *const[3], cudaStream_t);
+template void launch_modal_efield<double>(const GridP &, int, double *const[3], double *const[3], double *const[3],
+                                          double *const[3], cudaStream_t);
+template void launch_modal_efield<float>(const GridP &, int, float *const[3], float *const[3], float *const[3],
+                                         float *const[3], cudaStream_t);
 template void launch_modal_synth<double>(const GridP &, double *const[3], double *const[3], cudaStream_t);
 template void launch_modal_synth<float>(const GridP &, float *const[3], float *const[3], cudaStream_t);
 template void launch_modal_project<double>(const GridP &, double *const[3], double *const[3], cudaStream_t);
