@@ -34,7 +34,7 @@ struct pic_handle {
     cudaStream_t s = nullptr;
     bool fp32 = false;
     void *E[3] = {}, *B[3] = {}, *J[3] = {};
-    void *Jtmp = nullptr;
+    void *Jtmp[3] = {};   // the current filter's second buffer
     double *open_col = nullptr;   // den, vel per (j, k) column of an 'open' particle face (2 my mz)
     // convolutional PML: per-axis tables (6 doubles and a flag per index),
     // twelve psi grids in the handle's precision (E psi1 x,y,z, psi2 x,y,z,
@@ -362,9 +362,8 @@ int enqueue_phase(pic_handle *h, int cur, bool reorder, int phase)
                     launch_efield<double>(g, 1, E, B, J, h->s);
                 } else {
                     launch_fold<double>(g, J, h->s);
-                    for (int k = 0; k < h->cfg.curr_filter; k++) launch_filter<double>(g, J, (double *)h->Jtmp, h->s);
-                    launch_efield<double>(g, 3, E, B, J, h->s);
-                    for (int c = 0; c < 3; c++) cudaMemsetAsync(J[c], 0, (size_t)g.ncell * sizeof(double), h->s);
+                    double *const tmp[3] = {(double *)h->Jtmp[0], (double *)h->Jtmp[1], (double *)h->Jtmp[2]};
+                    launch_efield_filtered<double>(g, E, B, launch_filter<double>(g, h->cfg.curr_filter, J, tmp, h->s), J, h->s);
                 }
                 break;
             case PIC_PHASE_REORDER:  // MAIN.F90:259-265
@@ -394,9 +393,8 @@ int enqueue_phase(pic_handle *h, int cur, bool reorder, int phase)
                     launch_efield<float>(g, 1, E, B, J, h->s);
                 } else {
                     launch_fold<float>(g, J, h->s);
-                    for (int k = 0; k < h->cfg.curr_filter; k++) launch_filter<float>(g, J, (float *)h->Jtmp, h->s);
-                    launch_efield<float>(g, 3, E, B, J, h->s);
-                    for (int c = 0; c < 3; c++) cudaMemsetAsync(J[c], 0, (size_t)g.ncell * sizeof(float), h->s);
+                    float *const tmp[3] = {(float *)h->Jtmp[0], (float *)h->Jtmp[1], (float *)h->Jtmp[2]};
+                    launch_efield_filtered<float>(g, E, B, launch_filter<float>(g, h->cfg.curr_filter, J, tmp, h->s), J, h->s);
                 }
                 break;
             case PIC_PHASE_REORDER:
@@ -561,6 +559,17 @@ int enqueue_graph_step(pic_handle *h)
 
 size_t field_bytes(const pic_handle *h) { return (size_t)h->g.ncell * (h->fp32 ? sizeof(float) : sizeof(double)); }
 
+int ensure_jtmp(pic_handle *h)
+{
+    for (int c = 0; c < 3; c++) {
+        if (h->Jtmp[c]) continue;
+        const int r = dalloc(h, (char **)&h->Jtmp[c], field_bytes(h));
+        if (r) return r;
+        CK(cudaMemsetAsync(h->Jtmp[c], 0, field_bytes(h), h->s));
+    }
+    return PIC_OK;
+}
+
 int alloc_particles(pic_handle *h)
 {
     const size_t n = (size_t)h->capacity;
@@ -655,6 +664,18 @@ int fetch_array_f32(pic_handle *h, const float *src, double *dst, long long n, i
         CK(cudaEventRecord(h->ev_copied[b], h->cs));
     }
     return PIC_OK;
+}
+
+// The configured filter passes over J, the result left in J.
+template <typename T>
+void filter_current(pic_handle *h)
+{
+    T *E[3], *B[3], *J[3];
+    field_ptrs(h, E, B, J);
+    T *const tmp[3] = {(T *)h->Jtmp[0], (T *)h->Jtmp[1], (T *)h->Jtmp[2]};
+    if (launch_filter<T>(h->g, h->cfg.curr_filter, J, tmp, h->s) != J)
+        for (int c = 0; c < 3; c++)
+            cudaMemcpyAsync(J[c], tmp[c], (size_t)h->g.ncell * sizeof(T), cudaMemcpyDeviceToDevice, h->s);
 }
 
 int sync_both(pic_handle *h)
@@ -1061,7 +1082,7 @@ int pic_create(const pic_config *cfg, pic_handle **out)
         if ((r = dalloc(h, (char **)&h->B[k], fb))) break;
         if ((r = dalloc(h, (char **)&h->J[k], fb))) break;
     }
-    if (!r && c.curr_filter > 0) r = dalloc(h, (char **)&h->Jtmp, fb);
+    if (!r && c.curr_filter > 0) r = ensure_jtmp(h);
     if (!r && c.cyl_modes == 2) {
         h->modal = true;
         const size_t nm = (size_t)g.mx * 3 * (size_t)g.mz, esz = h->fp32 ? sizeof(float) : sizeof(double);
@@ -1512,21 +1533,10 @@ int pic_fold_current(pic_handle *h)
 int pic_filter_current(pic_handle *h)
 {
     if (!h || h->g.geom == PIC_GEOM_CYLINDRICAL) return PIC_ERR_INVALID;
-    if (!h->Jtmp) {
-        int r = dalloc(h, (char **)&h->Jtmp, field_bytes(h));
-        if (r) return r;
-    }
-    for (int k = 0; k < h->cfg.curr_filter; k++) {
-        if (h->fp32) {
-            float *E[3], *B[3], *J[3];
-            field_ptrs(h, E, B, J);
-            launch_filter<float>(h->g, J, (float *)h->Jtmp, h->s);
-        } else {
-            double *E[3], *B[3], *J[3];
-            field_ptrs(h, E, B, J);
-            launch_filter<double>(h->g, J, (double *)h->Jtmp, h->s);
-        }
-    }
+    const int r = ensure_jtmp(h);
+    if (r) return r;
+    if (h->fp32) filter_current<float>(h);
+    else filter_current<double>(h);
     return finish_phase(h);
 }
 

@@ -28,7 +28,10 @@ constexpr uint32_t kCellMask = (1u << kFlvShift) - 1u;
 template <typename T> void launch_bhalf(const GridP &g, T *const E[3], T *const B[3], cudaStream_t s);
 template <typename T> void launch_efield(const GridP &g, int mode, T *const E[3], T *const B[3], T *const J[3], cudaStream_t s);
 template <typename T> void launch_fold(const GridP &g, T *const J[3], cudaStream_t s);
-template <typename T> void launch_filter(const GridP &g, T *const J[3], T *tmp, cudaStream_t s);
+template <typename T>
+T *const *launch_filter(const GridP &g, int passes, T *const J[3], T *const tmp[3], cudaStream_t s);
+template <typename T>
+void launch_efield_filtered(const GridP &g, T *const E[3], T *const B[3], T *const F[3], T *const J[3], cudaStream_t s);
 
 // cyl.cu (cylindrical FP64 form)
 template <typename T>
