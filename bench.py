@@ -768,9 +768,10 @@ def run_adjoint_bench(args, rank, local, peak, peak_kind):
             "roofline": {"bound": "hbm", "achieved": None, "peak": peak, "unit": "GB/s", "frac": None,
                          "traffic": None, "kernel": "k_move_T (mover adjoint), latency/atomic bound at this size",
                          "peak_kind": peak_kind},
-            # forward: 2 B half steps, mover, E update, energy per step; gradient: the 4 kernels of each
-            # recomputed step, the 7 of each reverse step, the parameter reduction and 5 conversions
-            "gpu_launches": 5 * steps + 12 * steps + 6,
+            # forward: 2 B half steps, mover, E update with the energy per step; gradient: the 4 kernels of each
+            # recomputed step (2 of a segment's last), the 5 of each reverse step, the parameter reduction and 5
+            # conversions
+            "gpu_launches": 4 * steps + 9 * steps - 2 * (-(-steps // K)) + 6,
             "clocks": out["fp32"]["clocks"],
             "e2e": {"value": value, "unit": "particle-steps/s", "h2d_bytes_per_step": 0,
                     "d2h_bytes_per_step": 3 * 8 * n / steps,
