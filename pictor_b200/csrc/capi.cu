@@ -355,7 +355,8 @@ int enqueue_phase(pic_handle *h, int cur, bool reorder, int phase)
                     launch_move_deposit_f64(g, h->p64[cur], h->cnt, E, B, J, h->err, h->s, h->exact ? &h->rec : nullptr);
                 break;
             case PIC_PHASE_EXCHANGE:  // MAIN.F90:86-94 + 145-150
-                launch_exchange_f64(g, h->p64[cur], h->cnt, h->sc, h->capacity, h->err, h->s);
+                launch_exchange_f64(g, h->p64[cur], h->cnt, h->sc, h->capacity, h->err, h->s, nullptr, 0, nullptr,
+                                    h->tiled64 && h->sorted);
                 break;
             case PIC_PHASE_EFIELD:  // MAIN.F90:108-110, 124, 158, 170-184
                 if (!filt) {
@@ -1150,6 +1151,8 @@ int pic_create(const pic_config *cfg, pic_handle **out)
             !(r = dalloc(h, &T.box, 8 * (size_t)T.ntiles)) && !(r = dalloc(h, &T.np, 1)) &&
             !(r = dalloc(h, &T.qmax, 1)))
             h->tiled64 = true;
+        T.marks = reinterpret_cast<uint8_t *>(exchange_marks(h->sc));
+        if (!r && g.dims == 3 && g.geom == PIC_GEOM_CARTESIAN) r = dalloc(h, &T.node, 6 * (size_t)g.ncell);
     }
     if (!r && c.exact_current) {
         SegRecords &R = h->rec;

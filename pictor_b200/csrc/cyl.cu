@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_cyl_move_tiled(GridP g, CylP
                                                                    double *Jy, double *Jz, int *err)
 {
     extern __shared__ __align__(16) double smem64[];
-    move_tile64<3, 1>(g, p, T, Ex, Ey, Ez, Bx, By, Bz, Jx, Jy, Jz, 2.0, smem64,
+    move_tile64<3, 1>(g, p, T, Ex, Ey, Ez, Bx, By, Bz, Jx, Jy, Jz, 2.0, smem64, blockIdx.x,
                       [&](const P64 &s, uint32_t n, const Tile64Ctx &ctx, int *nc) {
         auto interp = [&](double x, double y, double z, double pE[3], double pB[3]) {
             const int i = (int)x, j = (int)y, k = (int)z;
@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_cyl_move_tiled(GridP g, CylP
             return false;
         // the particles that stay in the interior bound the next box
         return nc[0] >= 3 && nc[0] <= g.mx - 3 && nc[1] >= 3 && nc[1] <= g.my - 3 && nc[2] >= 3 && nc[2] <= g.mz - 3;
-    });
+    }, [](const Tile64Ctx &) {}, [](const Tile64Ctx &) {});
 }
 
 // AxisCurrentBC (cyl_movdep_strang.F90:570-584), all j, k.

@@ -61,15 +61,16 @@ void launch_cyl_move_deposit_f32(const GridP &g, const PartF32 &p, const Counter
 struct SegRecords;
 // rec == nullptr: the current goes to J by FP64 atomics; otherwise it is
 // summed in the reference's order (pic_config.exact_current, see mover.cu).
-// first (device, may be null): move the slots [*first, used) only.
 void launch_move_deposit_f64(const GridP &g, const PartF64 &p, const Counters *cnt, double *const E[3],
                              double *const B[3], double *const J[3], int *err, cudaStream_t s,
-                             SegRecords *rec = nullptr, const long long *first = nullptr);
+                             SegRecords *rec = nullptr);
 // mover_f64_tiled.cu: the FP64 mover after a reorder, one CTA per tile of H
 // row segments of W consecutive cells (x in [1 + sx W, 1 + (sx+1) W), rows
 // j0 .. j0 + H - 1, plane k; the tiles cover the ghosted grid), whose
 // particles the cell-order reorder leaves in H slot ranges.
-constexpr int kTile64SmemBytes = 110 * 1024;   // node box + FP64 current box of one tile (2 CTAs per SM)
+// Node box + current box of one tile, 2 CTAs per SM: cylindrical, and
+// Cartesian, whose kernel also queues second segments (13 KB).
+constexpr int kTile64SmemBytes = 110 * 1024, kTile64SmemCart = 98 * 1024;
 constexpr int kTile64MaxRows = 8;
 struct Tiles64 {
     uint32_t *range;              // 2 H per tile: first and past-the-end slot of each row segment
@@ -82,6 +83,8 @@ struct Tiles64 {
     int jfirst;                   // rows of the first row group (H, or 2: the low ghost rows alone, so
                                   // that the next groups start at the first interior row)
     int smem_bytes;
+    uint8_t *marks;               // Cartesian: exchange_marks
+    double *node;                 // 3D Cartesian: the 6 node values of every node 2 .. m - 1, or null
 };
 void choose_tiles64(const GridP &g, Tiles64 &T);
 // After a reorder: the tiles' slot ranges from the sorted keys, the boxes.
@@ -206,7 +209,13 @@ struct SegRecords {
 // Slab form (g.x_external): the x leavers go to `out` (out_cap particles of 8
 // doubles) and sent_counts (device) receives {right-bound, right + left-bound}.
 void launch_exchange_f64(const GridP &g, PartF64 &p, Counters *cnt, SortScratch &sc, long long capacity, int *err,
-                         cudaStream_t s, double *out = nullptr, long long out_cap = 0, uint32_t *sent_counts = nullptr);
+                         cudaStream_t s, double *out = nullptr, long long out_cap = 0, uint32_t *sent_counts = nullptr,
+                         bool marked = false);
+// The exchange's face words, one byte per slot, in the radix-sort key buffer
+// that is free between reorders.  marked: the tiled Cartesian mover has just
+// moved every particle and set the byte of those that are not in an interior
+// cell (Tiles64::marks); nothing has moved since.
+inline uint32_t *exchange_marks(const SortScratch &sc) { return sc.key[1]; }
 // bc.cu: walls along x (src/bc/bc_reflect.F90 on one rank), FP64 reference layout
 void launch_wall_reflect(const GridP &g, PartF64 &p, const Counters *cnt, double *const J[3], int side, double pos,
                          long long capacity, cudaStream_t s);

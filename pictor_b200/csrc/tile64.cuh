@@ -33,6 +33,7 @@
 
 namespace pic {
 
+constexpr int kTile64CutMax = 4;   // widest margin tried for a box cut to fit
 constexpr int kT64Threads = 256;   // 8 warps: the item order below covers 256 items
 
 // Tile t -> its row segments: cells x0 .. x1 - 1 (1-based) of rows j0 ..
@@ -103,6 +104,28 @@ __device__ __forceinline__ void gather_box64(const Box64 &bx, const double *sN, 
     }
 }
 
+// The node values of gather() (GatherVecEfld / GatherVecBfld) at offset nd.
+template <int DIMS>
+__device__ __forceinline__ void node_values64(const GridP &g, const double *__restrict__ Ex,
+                                              const double *__restrict__ Ey, const double *__restrict__ Ez,
+                                              const double *__restrict__ Bx, const double *__restrict__ By,
+                                              const double *__restrict__ Bz, long long nd, double v[6])
+{
+    const long long sy = g.sy, sz = g.sz;
+    v[0] = (__ldg(Ex + nd - 1) + __ldg(Ex + nd)) * 0.5;
+    v[1] = (__ldg(Ey + nd - sy) + __ldg(Ey + nd)) * 0.5;
+    if (DIMS == 3) {
+        v[2] = (__ldg(Ez + nd - sz) + __ldg(Ez + nd)) * 0.5;
+        v[3] = (((__ldg(Bx + nd - sy - sz) + __ldg(Bx + nd - sz)) + __ldg(Bx + nd - sy)) + __ldg(Bx + nd)) * 0.25 + g.bext[0];
+        v[4] = (((__ldg(By + nd - 1 - sz) + __ldg(By + nd - 1)) + __ldg(By + nd - sz)) + __ldg(By + nd)) * 0.25 + g.bext[1];
+    } else {
+        v[2] = __ldg(Ez + nd);
+        v[3] = (__ldg(Bx + nd - sy) + __ldg(Bx + nd)) * 0.5 + g.bext[0];
+        v[4] = (__ldg(By + nd - 1) + __ldg(By + nd)) * 0.5 + g.bext[1];
+    }
+    v[5] = (((__ldg(Bz + nd - 1 - sy) + __ldg(Bz + nd - 1)) + __ldg(Bz + nd - sy)) + __ldg(Bz + nd)) * 0.25 + g.bext[2];
+}
+
 // An FP64 value already multiplied by the box's scale, rounded to the
 // nearest integer: adding 1.5 * 2^52 leaves it in the low mantissa bits
 // (exact for |v| < 2^51).
@@ -127,14 +150,14 @@ __device__ __forceinline__ void add_fixed64(unsigned long long *w, long long q)
 
 // The VecJ entries o of a cell whose box current cell is jb, added into the
 // fixed-point box (the scatter offsets of movdep_routines.F90:276-303): each
-// entry times the scale S rounded to an integer.
-template <int DIMS>
+// entry times the scale S (SCALED: already in o) rounded to an integer.
+template <int DIMS, bool SCALED = false>
 __device__ __forceinline__ void deposit_box64(const Box64 &bx, unsigned long long *sJ, int jb, const double *o,
                                               double S)
 {
     unsigned long long *jx = sJ + jb, *jy = sJ + bx.nj + jb, *jz = sJ + 2 * bx.nj + jb;
     const int oy = bx.JX, oz = bx.JXY;
-    auto add = [&](unsigned long long *a, double v) { add_fixed64(a, fixed64(v * S)); };
+    auto add = [&](unsigned long long *a, double v) { add_fixed64(a, fixed64(SCALED ? v : v * S)); };
     if (DIMS == 2) {
         add(jx, o[0]);
         add(jx + oy, o[1]);
@@ -201,25 +224,27 @@ struct Tile64Ctx {
     }
 };
 
-// The CTA's work on tile blockIdx.x (see the file comment).  body(s, n, ctx,
+// The CTA's work on tile t (see the file comment).  body(s, n, ctx,
 // nc) moves the particle s of slot n and returns true with its new cell in
 // nc when that cell bounds the next box.  MARGIN widens the staged box by
 // cells on each side (a body that gathers at the moved position too); bound
 // is the largest VecJ entry a particle of charge q adds to one word, over
 // q qi.  The current box covers the cells of the box without MARGIN (the
 // start cells; a deposit beyond them by one cell lands in its +-1 frame).
+// after() runs for all lanes of a warp after each round of its particles, and
+// last() once at the end, before the current box is read.
 // Shared memory: T.smem_bytes dynamic; smem64 the dynamic array.
-template <int DIMS, int MARGIN, class Body>
+template <int DIMS, int MARGIN, class Body, class After, class Last>
 __device__ __forceinline__ void move_tile64(const GridP &g, const PartF64 &p, const Tiles64 &T,
                                             const double *__restrict__ Ex, const double *__restrict__ Ey,
                                             const double *__restrict__ Ez, const double *__restrict__ Bx,
                                             const double *__restrict__ By, const double *__restrict__ Bz,
                                             double *Jx, double *Jy, double *Jz, double bound, double *smem64,
-                                            Body &&body)
+                                            int t, Body &&body, After &&after, Last &&last)
 {
     __shared__ int s_red[kT64Threads / 32][6];
     __shared__ uint32_t s_rg[2 * kTile64MaxRows];
-    const int t = blockIdx.x, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     const int nseg = T.H * T.D;
     if (tid < 2 * nseg) s_rg[tid] = T.range[2 * (size_t)nseg * t + tid];
     __syncthreads();
@@ -255,16 +280,23 @@ __device__ __forceinline__ void move_tile64(const GridP &g, const PartF64 &p, co
     };
     int nnode = set_box();
     if (!fits(nnode)) {
-        // the particles spread further than shared memory holds: the tile's
-        // own cells plus one on each side (clamped to the ghost frame), the
-        // particles beyond it through global memory
+        // the particles spread further than shared memory holds: as much of
+        // their box as fits around the tile, the widest margin cut first, at
+        // least the tile's own cells plus one on each side (clamped to the
+        // ghost frame); the particles beyond it through global memory
         int x0, x1, j0, nrow, k0, nk;
         tile_cells(g, T, t, x0, x1, j0, nrow, k0, nk);
-        lo[0] = max(x0 - 1, 2); hi[0] = min(x1, g.mx - 2);
-        lo[1] = max(j0 - 1, 2); hi[1] = min(j0 + nrow, g.my - 2);
-        if (DIMS == 3) { lo[2] = max(k0 - 1, 2); hi[2] = min(k0 + nk, g.mz - 2); }
+        const int hl[3] = {x0, j0, DIMS == 3 ? k0 : 1}, hh[3] = {x1 - 1, j0 + nrow - 1, DIMS == 3 ? k0 + nk - 1 : 1};
+        const int m3[3] = {g.mx, g.my, g.mz};
         margin = 0;   // the current box is the node box here
-        nnode = set_box();
+        for (int w = kTile64CutMax; w >= 1; w--) {
+            for (int d = 0; d < DIMS; d++) {
+                lo[d] = max(w == 1 ? hl[d] - 1 : max(lo[d], hl[d] - w), 2);
+                hi[d] = min(w == 1 ? hh[d] + 1 : min(hi[d], hh[d] + w), m3[d] - 2);
+            }
+            nnode = set_box();
+            if (fits(nnode)) break;
+        }
     }
     // the box fits (and lies where the kernel may read and write) or the
     // tile's particles all take the global path
@@ -285,25 +317,26 @@ __device__ __forceinline__ void move_tile64(const GridP &g, const PartF64 &p, co
         if (b > 0.0) ctx.S = 1125899906842624.0 / b * (total > 4096u ? 4096.0 / (double)total : 1.0);
     }
     if (ctx.use_box) {
-        const long long sy = g.sy, sz = g.sz;
         for (int q = tid; q < 3 * bx.nj; q += kT64Threads) sJ[q] = 0ull;
+        // q / NX and r / NY by multiply-high (exact for q < 2^16)
+        const uint32_t mX = 0xffffffffu / (uint32_t)bx.NX + 1u, mY = 0xffffffffu / (uint32_t)(bx.C[1] + 1) + 1u;
         for (int q = tid; q < nnode; q += kT64Threads) {
-            const int a = q % bx.NX, r = q / bx.NX, b = r % (bx.C[1] + 1), c = r / (bx.C[1] + 1);
+            const int r = (int)__umulhi((uint32_t)q, mX), a = q - r * bx.NX;
+            const int c = (int)__umulhi((uint32_t)r, mY), b = r - c * (bx.C[1] + 1);
             const long long nd = cidx(g, lo[0] + a, lo[1] + b, DIMS == 3 ? lo[2] + c : 1);
-            double *v = sN + 6 * q;
-            // the node values of gather() (GatherVecEfld / GatherVecBfld)
-            v[0] = (__ldg(Ex + nd - 1) + __ldg(Ex + nd)) * 0.5;
-            v[1] = (__ldg(Ey + nd - sy) + __ldg(Ey + nd)) * 0.5;
-            if (DIMS == 3) {
-                v[2] = (__ldg(Ez + nd - sz) + __ldg(Ez + nd)) * 0.5;
-                v[3] = (((__ldg(Bx + nd - sy - sz) + __ldg(Bx + nd - sz)) + __ldg(Bx + nd - sy)) + __ldg(Bx + nd)) * 0.25 + g.bext[0];
-                v[4] = (((__ldg(By + nd - 1 - sz) + __ldg(By + nd - 1)) + __ldg(By + nd - sz)) + __ldg(By + nd)) * 0.25 + g.bext[1];
+            double2 *v = reinterpret_cast<double2 *>(sN + 6 * q);
+            if (T.node) {
+                const double2 *src = reinterpret_cast<const double2 *>(T.node + 6 * nd);
+                v[0] = __ldg(src);
+                v[1] = __ldg(src + 1);
+                v[2] = __ldg(src + 2);
             } else {
-                v[2] = __ldg(Ez + nd);
-                v[3] = (__ldg(Bx + nd - sy) + __ldg(Bx + nd)) * 0.5 + g.bext[0];
-                v[4] = (__ldg(By + nd - 1) + __ldg(By + nd)) * 0.5 + g.bext[1];
+                double u[6];
+                node_values64<DIMS>(g, Ex, Ey, Ez, Bx, By, Bz, nd, u);
+                v[0] = make_double2(u[0], u[1]);
+                v[1] = make_double2(u[2], u[3]);
+                v[2] = make_double2(u[4], u[5]);
             }
-            v[5] = (((__ldg(Bz + nd - 1 - sy) + __ldg(Bz + nd - 1)) + __ldg(Bz + nd - sy)) + __ldg(Bz + nd)) * 0.25 + g.bext[2];
         }
     }
     __syncthreads();
@@ -332,37 +365,40 @@ __device__ __forceinline__ void move_tile64(const GridP &g, const PartF64 &p, co
         ncur = slot_of(perm);
         cur = load_p64(p, ncur);
     }
-    for (uint32_t i = perm; i < total; i += kT64Threads) {
+    for (uint32_t base = 0; base < total; base += kT64Threads) {   // all lanes of the CTA step together
         // the next particle loads while this one moves
         P64 nxt;
         nxt.flv = 0;
         uint32_t nn = 0;
-        if (i + kT64Threads < total) {
-            nn = slot_of(i + kT64Threads);
+        if (base + perm + kT64Threads < total) {
+            nn = slot_of(base + perm + kT64Threads);
             nxt = load_p64(p, nn);
         }
         const uint32_t n = ncur;
         const P64 s = cur;
         cur = nxt;
         ncur = nn;
-        if (s.flv == 0) continue;
         int nc[3];
-        if (body(s, n, ctx, nc)) {
+        if (s.flv != 0 && body(s, n, ctx, nc)) {
             blo[0] = min(blo[0], nc[0]); bhi[0] = max(bhi[0], nc[0]);
             blo[1] = min(blo[1], nc[1]); bhi[1] = max(bhi[1], nc[1]);
             blo[2] = min(blo[2], nc[2]); bhi[2] = max(bhi[2], nc[2]);
         }
+        after(ctx);
     }
+    last(ctx);
     __syncthreads();
     if (ctx.use_box) {
         // the box current onto J (one FP64 atomic per nonzero word)
         const int JY = bx.jC[1] + 3;
         const double inv = 1.0 / ctx.S;
+        const uint32_t mX = 0xffffffffu / (uint32_t)bx.JX + 1u, mY = 0xffffffffu / (uint32_t)JY + 1u;
         for (int q = tid; q < bx.nj; q += kT64Threads) {
             const long long ix = (long long)sJ[q], iy = (long long)sJ[bx.nj + q], iz = (long long)sJ[2 * bx.nj + q];
             if (ix == 0 && iy == 0 && iz == 0) continue;
             const double vx = (double)ix * inv, vy = (double)iy * inv, vz = (double)iz * inv;
-            const int a = q % bx.JX, r = q / bx.JX, b = r % JY, cc = r / JY;
+            const int r = (int)__umulhi((uint32_t)q, mX), a = q - r * bx.JX;
+            const int cc = (int)__umulhi((uint32_t)r, mY), b = r - cc * JY;
             const long long off = cidx(g, bx.jlo[0] - 1 + a, bx.jlo[1] - 1 + b, DIMS == 3 ? bx.jlo[2] - 1 + cc : 1);
             if (vx != 0.0) atomicAdd(Jx + off, vx);
             if (vy != 0.0) atomicAdd(Jy + off, vy);
