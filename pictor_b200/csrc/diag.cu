@@ -8,6 +8,7 @@
 // the backward-difference node divergence of CalcDivE.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "tile64.cuh"
 
 namespace pic {
 
@@ -16,17 +17,19 @@ constexpr int kDiagThreads = 256;
 int field_energy_blocks(const GridP &g)
 {
     const long long nint = (long long)g.nx * g.ny * (g.dims == 3 ? g.nz : 1);
-    long long b = (nint + kDiagThreads * 8 - 1) / (kDiagThreads * 8);
+    long long b = (nint + kDiagThreads * 2 - 1) / (kDiagThreads * 2);
     if (b > kSMs * 8) b = kSMs * 8;
     return (int)(b < 1 ? 1 : b);
 }
 
-__device__ __forceinline__ void interior_ijk(const GridP &g, long long t, int &i, int &j, int &k)
+// Interior rows (j, k) of the grid; a warp takes rows gw, gw + nw, ... and its
+// lanes the cells of a row, so no flat index is divided per cell.
+__device__ __forceinline__ int row_count(const GridP &g) { return g.ny * (g.dims == 3 ? g.nz : 1); }
+__device__ __forceinline__ void row_jk(const GridP &g, int r, int &j, int &k)
 {
-    i = 3 + (int)(t % g.nx);
-    const long long r = t / g.nx;
-    j = 3 + (int)(r % g.ny);
-    k = g.dims == 3 ? 3 + (int)(r / g.ny) : 1;
+    const int kk = g.dims == 3 ? r / g.ny : 0;
+    j = 3 + (r - kk * g.ny);
+    k = g.dims == 3 ? 3 + kk : 1;
 }
 
 __device__ __forceinline__ double block_sum(double v, double *red)
@@ -48,23 +51,26 @@ __global__ void __launch_bounds__(kDiagThreads) k_field_energy_partial(GridP g, 
                                                                        double *partials)
 {
     __shared__ double red[kDiagThreads / 32];
-    const long long nint = (long long)g.nx * g.ny * (g.dims == 3 ? g.nz : 1);
     double eb = 0, ee = 0;
     const double dtheta = 2.0 * 3.14159265358979323846264 / g.ny;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        interior_ijk(g, t, i, j, k);
-        const long long c = cidx(g, i, j, k);
-        const double bx = Bx[c], by = By[c], bz = Bz[c], ex = Ex[c], ey = Ey[c], ez = Ez[c];
-        if (g.geom == PIC_GEOM_CYLINDRICAL) {
-            // CalcFldEnergy_cyl (cyl_savedata_routines.F90:8-31): r weights, axis cell excluded
-            if (i < 4) continue;
-            const double r = ((double)i - 3.0) + -0.5, rp = r + 0.5;
-            eb += ((r * (bx * bx) + rp * (by * by)) + rp * (bz * bz)) * dtheta;
-            ee += ((rp * (ex * ex) + r * (ey * ey)) + r * (ez * ez)) * dtheta;
-        } else {
-            eb += (bx * bx + by * by) + bz * bz;
-            ee += (ex * ex + ey * ey) + ez * ez;
+    const int lane = threadIdx.x & 31, nw = gridDim.x * (kDiagThreads / 32), rows = row_count(g);
+    for (int row = blockIdx.x * (kDiagThreads / 32) + (threadIdx.x >> 5); row < rows; row += nw) {
+        int j, k;
+        row_jk(g, row, j, k);
+        const long long c0 = cidx(g, 0, j, k);
+        for (int i = 3 + lane; i < 3 + g.nx; i += 32) {
+            const long long c = c0 + i;
+            const double bx = Bx[c], by = By[c], bz = Bz[c], ex = Ex[c], ey = Ey[c], ez = Ez[c];
+            if (g.geom == PIC_GEOM_CYLINDRICAL) {
+                // CalcFldEnergy_cyl (cyl_savedata_routines.F90:8-31): r weights, axis cell excluded
+                if (i < 4) continue;
+                const double r = ((double)i - 3.0) + -0.5, rp = r + 0.5;
+                eb += ((r * (bx * bx) + rp * (by * by)) + rp * (bz * bz)) * dtheta;
+                ee += ((rp * (ex * ex) + r * (ey * ey)) + r * (ez * ez)) * dtheta;
+            } else {
+                eb += (bx * bx + by * by) + bz * bz;
+                ee += (ex * ex + ey * ey) + ez * ez;
+            }
         }
     }
     const double sb = block_sum(eb, red);
@@ -75,16 +81,22 @@ __global__ void __launch_bounds__(kDiagThreads) k_field_energy_partial(GridP g, 
     }
 }
 
-__global__ void k_sum_partials(const double *__restrict__ partials, int nblocks, double *out2)
+// The partial pairs added in a fixed order: thread t its own stride, then the
+// threads' sums in a tree (one thread walking 1184 pairs took 33 us).
+__global__ void __launch_bounds__(kDiagThreads) k_sum_partials(const double *__restrict__ partials, int nblocks, double *out2)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ double red[kDiagThreads / 32];
     double sb = 0, se = 0;
-    for (int b = 0; b < nblocks; b++) {
+    for (int b = threadIdx.x; b < nblocks; b += kDiagThreads) {
         sb += partials[2 * b];
         se += partials[2 * b + 1];
     }
-    out2[0] = sb;
-    out2[1] = se;
+    const double tb = block_sum(sb, red);
+    const double te = block_sum(se, red);
+    if (threadIdx.x == 0) {
+        out2[0] = tb;
+        out2[1] = te;
+    }
 }
 
 void launch_field_energy(const GridP &g, const void *const E[3], const void *const B[3], bool fp32, double *partials,
@@ -98,7 +110,7 @@ void launch_field_energy(const GridP &g, const void *const E[3], const void *con
         k_field_energy_partial<double><<<nblocks, kDiagThreads, 0, s>>>(
             g, (const double *)E[0], (const double *)E[1], (const double *)E[2], (const double *)B[0],
             (const double *)B[1], (const double *)B[2], partials);
-    k_sum_partials<<<1, 32, 0, s>>>(partials, nblocks, out2);
+    k_sum_partials<<<1, kDiagThreads, 0, s>>>(partials, nblocks, out2);
     count_launches(1);
     count_launches(1);
 }
@@ -107,83 +119,113 @@ void launch_field_energy(const GridP &g, const void *const E[3], const void *con
 // Kinetic energy per species (CalcPrtlEnergy, savedata_routines.F90:283-308),
 // with the particle weight wtp = |q| (charge = weight * FlvrCharge).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void add_species_energy(const GridP &g, double masse, int flv, double q, double u, double v,
-                                                   double w, double *acc)
+__device__ __forceinline__ double species_energy(const GridP &g, double masse, int flv, double q, double u, double v,
+                                                 double w)
 {
     const double c = g.c;
     const double gm = sqrt(((1.0 + u * u) + v * v) + w * w);
     const double wt = fabs(q);
-    if (q > 0) acc[flv] += (((gm - 1.0) * wt) * (q * g.qi / g.qm[flv])) * c * c;
-    if (q < 0) acc[flv] += ((gm - 1.0) * wt) * ((masse * c) * c);
+    if (q > 0) return (((gm - 1.0) * wt) * (q * g.qi / g.qm[flv])) * c * c;
+    if (q < 0) return ((gm - 1.0) * wt) * ((masse * c) * c);
+    return 0.0;
 }
+
+// Sums per flavour: flavours 1 and 2 in registers (an array indexed by the
+// flavour lives in local memory), the others, which few runs have, in shared
+// memory; one atomic per block and flavour.
+struct FlavourSum {
+    double a1 = 0, a2 = 0;
+    __device__ __forceinline__ void add(double *sh, int flv, double e)
+    {
+        a1 += flv == 1 ? e : 0.0;
+        a2 += flv == 2 ? e : 0.0;
+        if (flv > 2) atomicAdd(sh + flv, e);
+    }
+    __device__ void store(double *sh, double *out)
+    {
+        double v[2] = {a1, a2};
+        for (int f = 0; f < 2; f++) {
+            for (int o = 16; o > 0; o >>= 1) v[f] += __shfl_down_sync(0xffffffffu, v[f], o);
+            if ((threadIdx.x & 31) == 0 && v[f] != 0.0) atomicAdd(sh + 1 + f, v[f]);
+        }
+        __syncthreads();
+        const int f = 1 + threadIdx.x;
+        if (f <= PIC_MAX_FLVR && sh[f] != 0.0) atomicAdd(out + f - 1, sh[f]);
+    }
+};
 
 __global__ void __launch_bounds__(kDiagThreads) k_pe_f64(GridP g, PartF64 p, const Counters *__restrict__ cnt, double masse,
                                                          double *out)
 {
-    double acc[PIC_MAX_FLVR + 1];
-    for (int f = 0; f <= PIC_MAX_FLVR; f++) acc[f] = 0;
+    __shared__ double sh[PIC_MAX_FLVR + 1];
+    if (threadIdx.x <= PIC_MAX_FLVR) sh[threadIdx.x] = 0;
+    __syncthreads();
+    FlavourSum acc;
     const long long n = cnt->used;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const int flv = p.flv[i];
         if (flv <= 0 || flv > PIC_MAX_FLVR) continue;
-        add_species_energy(g, masse, flv, p.q[i], p.u[i], p.v[i], p.w[i], acc);
+        acc.add(sh, flv, species_energy(g, masse, flv, p.q[i], p.u[i], p.v[i], p.w[i]));
     }
-    for (int f = 1; f <= PIC_MAX_FLVR; f++) {
-        double v = acc[f];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(out + f - 1, v);
-    }
+    acc.store(sh, out);
 }
 
 __global__ void __launch_bounds__(kDiagThreads) k_pe_f32(GridP g, PartF32 p, const Counters *__restrict__ cnt, double masse,
                                                          double *out)
 {
-    double acc[PIC_MAX_FLVR + 1];
-    for (int f = 0; f <= PIC_MAX_FLVR; f++) acc[f] = 0;
+    __shared__ double sh[PIC_MAX_FLVR + 1];
+    if (threadIdx.x <= PIC_MAX_FLVR) sh[threadIdx.x] = 0;
+    __syncthreads();
+    FlavourSum acc;
     const long long n = cnt->used;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const int flv = (int)(p.key[i] >> kFlvShift);
         if (flv == 0) continue;
-        add_species_energy(g, masse, flv, (double)p.w[i], (double)p.ux[i], (double)p.uy[i], (double)p.uz[i], acc);
+        acc.add(sh, flv, species_energy(g, masse, flv, (double)p.w[i], (double)p.ux[i], (double)p.uy[i], (double)p.uz[i]));
     }
-    for (int f = 1; f <= PIC_MAX_FLVR; f++) {
-        double v = acc[f];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(out + f - 1, v);
-    }
+    acc.store(sh, out);
 }
 
 void launch_particle_energy_f64(const GridP &g, const PartF64 &p, const Counters *cnt, double masse, double *out,
                                 cudaStream_t s)
 {
-    k_pe_f64<<<kSMs * 4, kDiagThreads, 0, s>>>(g, p, cnt, masse, out);
+    k_pe_f64<<<kSMs * 8, kDiagThreads, 0, s>>>(g, p, cnt, masse, out);
     count_launches(1);
 }
 
 void launch_particle_energy_f32(const GridP &g, const PartF32 &p, const Counters *cnt, double masse, double *out,
                                 cudaStream_t s)
 {
-    k_pe_f32<<<kSMs * 4, kDiagThreads, 0, s>>>(g, p, cnt, masse, out);
+    k_pe_f32<<<kSMs * 8, kDiagThreads, 0, s>>>(g, p, cnt, masse, out);
     count_launches(1);
 }
 
 // ---------------------------------------------------------------------------
 // Gauss residual
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void deposit_rho(const GridP &g, double *rho, double *rho_pos, int i, int j, int k, double dx,
-                                            double dy, double dz, double q)
+// The positive and the negative charge are summed apart (the residual wants
+// their sum, the scale the positive one), so a particle adds to one array.
+__device__ __forceinline__ void corner_weights(int dims, double dx, double dy, double dz, double w[8])
 {
-    for (int nn = 0; nn < (g.dims == 3 ? 8 : 4); nn++) {
-        const double w = ((nn & 1) ? dx : 1.0 - dx) * ((nn & 2) ? dy : 1.0 - dy) * ((nn & 4) ? dz : 1.0 - dz);
+#pragma unroll
+    for (int nn = 0; nn < 8; nn++)
+        w[nn] = ((nn & 1) ? dx : 1.0 - dx) * ((nn & 2) ? dy : 1.0 - dy) * ((nn & 4) ? dz : 1.0 - dz);
+}
+__device__ __forceinline__ void deposit_rho(const GridP &g, double *rho, int i, int j, int k, double dx, double dy,
+                                            double dz, double q)
+{
+    double w[8];
+    corner_weights(g.dims, dx, dy, dz, w);
+#pragma unroll
+    for (int nn = 0; nn < 8; nn++) {
+        if (nn >= 4 && g.dims == 2) break;
         const int a = wrap_index(i + (nn & 1), g.mx), b = wrap_index(j + ((nn >> 1) & 1), g.my);
         const int c = g.dims == 3 ? wrap_index(k + ((nn >> 2) & 1), g.mz) : 1;
-        const long long o = cidx(g, a, b, c);
-        atomicAdd(rho + o, q * w);
-        if (q > 0) atomicAdd(rho_pos + o, q * w);
+        atomicAdd(rho + cidx(g, a, b, c), q * w[nn]);
     }
 }
 
-__global__ void k_rho_f64(GridP g, PartF64 p, const Counters *__restrict__ cnt, double *rho, double *rho_pos)
+__global__ void k_rho_f64(GridP g, PartF64 p, const Counters *__restrict__ cnt, double *rho_neg, double *rho_pos)
 {
     const long long n = cnt->used;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -193,38 +235,139 @@ __global__ void k_rho_f64(GridP g, PartF64 p, const Counters *__restrict__ cnt, 
         const int i = (int)floor(x), j = (int)floor(y);
         const int k = g.dims == 3 ? (int)floor(z) : 1;
         if (g.dims == 3 && !(z >= 1.0 && z < g.mz)) continue;
-        deposit_rho(g, rho, rho_pos, i, j, k, x - i, y - j, g.dims == 3 ? z - k : 0.0, p.q[t] * g.qi);
+        const double q = p.q[t] * g.qi;
+        deposit_rho(g, q > 0 ? rho_pos : rho_neg, i, j, k, x - i, y - j, g.dims == 3 ? z - k : 0.0, q);
     }
 }
 
-__global__ void k_rho_f32(GridP g, PartF32 p, const Counters *__restrict__ cnt, double *rho, double *rho_pos)
+__global__ void k_rho_f32(GridP g, PartF32 p, const Counters *__restrict__ cnt, double *rho_neg, double *rho_pos)
 {
     const long long n = cnt->used;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         const uint32_t key = p.key[t];
         if ((key >> kFlvShift) == 0) continue;
-        const int cell = (int)(key & kCellMask);
-        const int i = cell % g.mx + 1, jk = cell / g.mx, j = jk % g.my + 1, k = jk / g.my + 1;
-        deposit_rho(g, rho, rho_pos, i, j, k, (double)p.dx[t], (double)p.dy[t], g.dims == 3 ? (double)p.dz[t] : 0.0,
-                    (double)p.w[t] * g.qi);
+        int i, j, k;
+        decode_cell(g, (int)(key & kCellMask), i, j, k);
+        const double q = (double)p.w[t] * g.qi;
+        deposit_rho(g, q > 0 ? rho_pos : rho_neg, i, j, k, (double)p.dx[t], (double)p.dy[t],
+                    g.dims == 3 ? (double)p.dz[t] : 0.0, q);
     }
+}
+
+// The same after a reorder, one CTA per brick (bricks.cu): the brick's charge
+// is summed in shared memory over the nodes of its box as 64-bit fixed-point
+// words (the scale of tile64.cuh: a unit is at most 2^-50 of the largest
+// charge, below the FP64 rounding of the sums), each added as two 32-bit
+// atomics, and the box is added to the grid once.  A particle outside the box
+// adds to the grid.  537 M particles 6.7 ms, and with the energies below the
+// diagnostics 11.9 ms (23.8 ms with 12 FP64 atomics into L2 per particle).
+constexpr int kRhoNodes = 3072;   // 48 KB, 4 CTAs per SM
+template <int DIMS>
+__global__ void __launch_bounds__(256) k_rho_f32_bricks(GridP g, PartF32 p, Bricks bk, double *rho_neg, double *rho_pos)
+{
+    extern __shared__ unsigned long long s_rho[];   // positive, then negative charge
+    const int b = blockIdx.x;
+    const uint32_t p0 = bk.tile_start[b], p1 = bk.tile_start[b + 1];
+    if (p0 >= p1) return;
+    const int bx = b % bk.nb[0], byz = b / bk.nb[0], by = byz % bk.nb[1], bz = byz / bk.nb[1];
+    const int n3[3] = {g.nx, g.ny, g.nz}, bi[3] = {bx, by, bz};
+    int hc[3], lo[3], N[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        hc[d] = d < DIMS ? 3 + bi[d] * bk.t[d] + (bk.t[d] >> 1) : 1;
+        lo[d] = d < DIMS ? bk.box[8 * (size_t)b + d] : 0;
+        N[d] = d < DIMS ? bk.box[8 * (size_t)b + 3 + d] - lo[d] + 2 : 1;   // nodes
+    }
+    const bool fits = N[0] > 1 && N[1] > 1 && (DIMS == 2 || N[2] > 1) && N[0] <= kBoxAxisMax && N[1] <= kBoxAxisMax &&
+                      N[2] <= kBoxAxisMax && N[0] * N[1] * N[2] <= kRhoNodes;
+    const int nn = fits ? N[0] * N[1] * N[2] : 0;
+    for (int q = threadIdx.x; q < 2 * nn; q += 256) s_rho[q] = 0ull;
+    const double qmax = (double)__uint_as_float(*bk.wmax_bits) * g.qi;
+    const uint32_t np = p1 - p0;
+    const double S = qmax > 0.0 ? 1125899906842624.0 / qmax * (np > 4096u ? 4096.0 / (double)np : 1.0) : 1.0;
+    __syncthreads();
+    for (uint32_t t = p0 + threadIdx.x; t < p1; t += 256) {
+        const uint32_t key = p.key[t];
+        if ((key >> kFlvShift) == 0) continue;
+        int i, j, k;
+        decode_cell(g, (int)(key & kCellMask), i, j, k);
+        const double q = (double)p.w[t] * g.qi;
+        const double dx = p.dx[t], dy = p.dy[t], dz = DIMS == 3 ? (double)p.dz[t] : 0.0;
+        auto un = [](int a, int c, int n) {
+            int u = a - c;
+            const int half = n >> 1;
+            if (u >= n - half) u -= n;
+            else if (u < -half) u += n;
+            return u;
+        };
+        const int lx = un(i, hc[0], n3[0]) - lo[0], ly = un(j, hc[1], n3[1]) - lo[1],
+                  lz = DIMS == 3 ? un(k, hc[2], n3[2]) - lo[2] : 0;
+        if (!fits || (unsigned)lx >= (unsigned)(N[0] - 1) || (unsigned)ly >= (unsigned)(N[1] - 1) ||
+            (DIMS == 3 && (unsigned)lz >= (unsigned)(N[2] - 1))) {
+            deposit_rho(g, q > 0 ? rho_pos : rho_neg, i, j, k, dx, dy, dz, q);
+            continue;
+        }
+        double w[8];
+        corner_weights(DIMS, dx, dy, dz, w);
+        unsigned long long *at = s_rho + (q > 0 ? 0 : nn) + lx + N[0] * (ly + N[1] * lz);
+        const double qS = q * S;
+#pragma unroll
+        for (int c = 0; c < (DIMS == 3 ? 8 : 4); c++)
+            add_fixed64(at + (c & 1) + ((c >> 1) & 1) * N[0] + ((c >> 2) & 1) * N[0] * N[1], fixed64(qS * w[c]));
+    }
+    __syncthreads();
+    const double inv = 1.0 / S;
+    const uint32_t mX = 0xffffffffu / (uint32_t)N[0] + 1u, mY = 0xffffffffu / (uint32_t)N[1] + 1u;
+    for (int q = threadIdx.x; q < nn; q += 256) {
+        const long long vp = (long long)s_rho[q], vn = (long long)s_rho[nn + q];
+        if (vp == 0 && vn == 0) continue;
+        const int r = (int)__umulhi((uint32_t)q, mX), xx = q - r * N[0];
+        const int zz = (int)__umulhi((uint32_t)r, mY), yy = r - zz * N[1];
+        const int c[3] = {hc[0] + lo[0] + xx, hc[1] + lo[1] + yy, DIMS == 3 ? hc[2] + lo[2] + zz : 1};
+        int cc[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            int a = c[d] - 3;
+            if (d < DIMS) {
+                a %= n3[d];
+                if (a < 0) a += n3[d];
+                cc[d] = 3 + a;
+            } else {
+                cc[d] = 1;
+            }
+        }
+        const long long o = cidx(g, cc[0], cc[1], cc[2]);
+        if (vp != 0) atomicAdd(rho_pos + o, (double)vp * inv);
+        if (vn != 0) atomicAdd(rho_neg + o, (double)vn * inv);
+    }
+}
+
+// rho_neg += rho_pos: the total density.
+__global__ void k_rho_total(long long n, double *rho_neg, const double *__restrict__ rho_pos)
+{
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
+        rho_neg[t] += rho_pos[t];
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kDiagThreads) k_gauss_max(GridP g, const T *__restrict__ Ex, const T *__restrict__ Ey,
-                                                            const T *__restrict__ Ez, const double *__restrict__ rho,
+                                                            const T *__restrict__ Ez, const double *__restrict__ rho_neg,
                                                             const double *__restrict__ rho_pos, double *out2)
 {
-    const long long nint = (long long)g.nx * g.ny * (g.dims == 3 ? g.nz : 1);
     double res = 0, rm = 0;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        interior_ijk(g, t, i, j, k);
-        const long long c = cidx(g, i, j, k);
-        double div = ((double)Ex[c] - (double)Ex[c - 1]) + ((double)Ey[c] - (double)Ey[c - g.sy]);
-        if (g.dims == 3) div = div + ((double)Ez[c] - (double)Ez[c - g.sz]);
-        res = fmax(res, fabs(div - rho[c]));
-        rm = fmax(rm, fabs(rho_pos[c]));
+    const int lane = threadIdx.x & 31, nw = gridDim.x * (kDiagThreads / 32), rows = row_count(g);
+    for (int row = blockIdx.x * (kDiagThreads / 32) + (threadIdx.x >> 5); row < rows; row += nw) {
+        int j, k;
+        row_jk(g, row, j, k);
+        const long long c0 = cidx(g, 0, j, k);
+        for (int i = 3 + lane; i < 3 + g.nx; i += 32) {
+            const long long c = c0 + i;
+            double div = ((double)Ex[c] - (double)Ex[c - 1]) + ((double)Ey[c] - (double)Ey[c - g.sy]);
+            if (g.dims == 3) div = div + ((double)Ez[c] - (double)Ez[c - g.sz]);
+            const double rp = rho_pos[c];
+            res = fmax(res, fabs(div - (rho_neg[c] + rp)));
+            rm = fmax(rm, fabs(rp));
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         res = fmax(res, __shfl_down_sync(0xffffffffu, res, o));
@@ -237,43 +380,64 @@ __global__ void __launch_bounds__(kDiagThreads) k_gauss_max(GridP g, const T *__
     }
 }
 
+static void zero_rho(const GridP &g, double *rho, double *rho_pos, cudaStream_t s)
+{
+    const size_t bytes = (size_t)g.ncell * sizeof(double);
+    if (rho_pos == rho + g.ncell) {   // the two arrays of one block
+        cudaMemsetAsync(rho, 0, 2 * bytes, s);
+    } else {
+        cudaMemsetAsync(rho, 0, bytes, s);
+        cudaMemsetAsync(rho_pos, 0, bytes, s);
+    }
+}
+static void deposit_f64(const GridP &g, const PartF64 &p, const Counters *cnt, double *rho, double *rho_pos, cudaStream_t s)
+{
+    zero_rho(g, rho, rho_pos, s);
+    k_rho_f64<<<kSMs * 8, 256, 0, s>>>(g, p, cnt, rho, rho_pos);
+    count_launches(1);
+}
+static void deposit_f32(const GridP &g, const PartF32 &p, const Counters *cnt, const Bricks *bk, double *rho,
+                        double *rho_pos, cudaStream_t s)
+{
+    zero_rho(g, rho, rho_pos, s);
+    const size_t sm = 2 * kRhoNodes * sizeof(unsigned long long);
+    if (bk && g.dims == 3) k_rho_f32_bricks<3><<<bk->ntiles, 256, sm, s>>>(g, p, *bk, rho, rho_pos);
+    else if (bk) k_rho_f32_bricks<2><<<bk->ntiles, 256, sm, s>>>(g, p, *bk, rho, rho_pos);
+    else k_rho_f32<<<kSMs * 8, 256, 0, s>>>(g, p, cnt, rho, rho_pos);
+    count_launches(1);
+}
+static void total_density(const GridP &g, double *rho, const double *rho_pos, cudaStream_t s)
+{
+    k_rho_total<<<kSMs * 8, 256, 0, s>>>(g.ncell, rho, rho_pos);
+    count_launches(1);
+}
+
 // The CIC charge density alone (the initial Gauss solve, poisson.cu).
 void launch_rho_f64(const GridP &g, const PartF64 &p, const Counters *cnt, double *rho, double *rho_pos, cudaStream_t s)
 {
-    cudaMemsetAsync(rho, 0, (size_t)g.ncell * sizeof(double), s);
-    cudaMemsetAsync(rho_pos, 0, (size_t)g.ncell * sizeof(double), s);
-    k_rho_f64<<<kSMs * 8, 256, 0, s>>>(g, p, cnt, rho, rho_pos);
-    count_launches(1);
+    deposit_f64(g, p, cnt, rho, rho_pos, s);
+    total_density(g, rho, rho_pos, s);
 }
 
 void launch_rho_f32(const GridP &g, const PartF32 &p, const Counters *cnt, double *rho, double *rho_pos, cudaStream_t s)
 {
-    cudaMemsetAsync(rho, 0, (size_t)g.ncell * sizeof(double), s);
-    cudaMemsetAsync(rho_pos, 0, (size_t)g.ncell * sizeof(double), s);
-    k_rho_f32<<<kSMs * 8, 256, 0, s>>>(g, p, cnt, rho, rho_pos);
-    count_launches(1);
+    deposit_f32(g, p, cnt, nullptr, rho, rho_pos, s);
+    total_density(g, rho, rho_pos, s);
 }
 
+// out2 must be zero.
 void launch_gauss_f64(const GridP &g, const PartF64 &p, const Counters *cnt, const double *const E[3], double *rho,
                       double *rho_pos, double *out2, cudaStream_t s)
 {
-    cudaMemsetAsync(rho, 0, (size_t)g.ncell * sizeof(double), s);
-    cudaMemsetAsync(rho_pos, 0, (size_t)g.ncell * sizeof(double), s);
-    cudaMemsetAsync(out2, 0, 2 * sizeof(double), s);
-    k_rho_f64<<<kSMs * 8, 256, 0, s>>>(g, p, cnt, rho, rho_pos);
-    count_launches(1);
+    deposit_f64(g, p, cnt, rho, rho_pos, s);
     k_gauss_max<double><<<field_energy_blocks(g), kDiagThreads, 0, s>>>(g, E[0], E[1], E[2], rho, rho_pos, out2);
     count_launches(1);
 }
 
-void launch_gauss_f32(const GridP &g, const PartF32 &p, const Counters *cnt, const float *const E[3], double *rho,
-                      double *rho_pos, double *out2, cudaStream_t s)
+void launch_gauss_f32(const GridP &g, const PartF32 &p, const Counters *cnt, const Bricks *bk, const float *const E[3],
+                      double *rho, double *rho_pos, double *out2, cudaStream_t s)
 {
-    cudaMemsetAsync(rho, 0, (size_t)g.ncell * sizeof(double), s);
-    cudaMemsetAsync(rho_pos, 0, (size_t)g.ncell * sizeof(double), s);
-    cudaMemsetAsync(out2, 0, 2 * sizeof(double), s);
-    k_rho_f32<<<kSMs * 8, 256, 0, s>>>(g, p, cnt, rho, rho_pos);
-    count_launches(1);
+    deposit_f32(g, p, cnt, bk, rho, rho_pos, s);
     k_gauss_max<float><<<field_energy_blocks(g), kDiagThreads, 0, s>>>(g, E[0], E[1], E[2], rho, rho_pos, out2);
     count_launches(1);
 }

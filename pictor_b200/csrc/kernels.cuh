@@ -291,6 +291,7 @@ void launch_reorder_f32(const GridP &g, const PartF32 &p, const PartF32 &out, Co
 void launch_f64_to_f32(const GridP &g, const PartF64 &in, const PartF32 &out, long long n, int *err, cudaStream_t s);
 void launch_f32_to_f64(const GridP &g, const PartF32 &in, const PartF64 &out, long long n, cudaStream_t s);
 void launch_array_f64_to_f32(const double *in, float *out, long long n, cudaStream_t s);
+void launch_arrays_f32_to_f64(const float *const *in, int m, double *out, long long n, cudaStream_t s);
 void launch_array_f32_to_f64(const float *in, double *out, long long n, cudaStream_t s);
 // Device Weibel loader.
 struct WeibelParams {
@@ -339,7 +340,8 @@ int solve_gauss(const GridP &g, void *const E[3], bool fp32, const double *rho, 
                 cudaStream_t s, int *iters, double *rel_res, double *rho_mean);
 void launch_gauss_f64(const GridP &g, const PartF64 &p, const Counters *cnt, const double *const E[3], double *rho,
                       double *rho_pos, double *out2, cudaStream_t s);
-void launch_gauss_f32(const GridP &g, const PartF32 &p, const Counters *cnt, const float *const E[3], double *rho,
-                      double *rho_pos, double *out2, cudaStream_t s);
+// bk: the bricks of the last reorder, or null when the particles are in any order
+void launch_gauss_f32(const GridP &g, const PartF32 &p, const Counters *cnt, const Bricks *bk, const float *const E[3],
+                      double *rho, double *rho_pos, double *out2, cudaStream_t s);
 
 }  // namespace pic

@@ -95,40 +95,8 @@ __global__ void k_scan_add(uint32_t *out, size_t n, const uint32_t *__restrict__
     if (i < n) out[i] += offs[i / kScanTile];
 }
 
-// The scan of up to kScanOne values by one block, a contiguous run of at most
-// 32 per thread: one launch (4 us at 18 k values) where the two levels take
-// three (10 us).
-constexpr size_t kScanOne = 32 * kScanBlock;
-__global__ void __launch_bounds__(kScanBlock) k_scan_one(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *total)
-{
-    __shared__ uint32_t warp_tot[kScanBlock / 32];
-    const uint32_t per = (n + kScanBlock - 1) / kScanBlock;
-    const uint32_t b = min(threadIdx.x * per, n), e = min(b + per, n);
-    uint32_t acc = 0;
-#pragma unroll 8
-    for (uint32_t i = b; i < e; i++) acc += in[i];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t incl = warp_incl_scan(acc);
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) warp_tot[lane] = warp_incl_scan(warp_tot[lane]);
-    __syncthreads();
-    uint32_t run = (incl - acc) + (warp > 0 ? warp_tot[warp - 1] : 0u);
-    for (uint32_t i = b; i < e; i++) {
-        const uint32_t v = in[i];
-        out[i] = run;
-        run += v;
-    }
-    if (threadIdx.x == kScanBlock - 1 && total) *total = run;
-}
-
 void scan_exclusive_u32(const uint32_t *in, uint32_t *out, size_t n, uint32_t *tmp, uint32_t *total, cudaStream_t s)
 {
-    if (n > kScanTile && n <= kScanOne) {
-        k_scan_one<<<1, kScanBlock, 0, s>>>(in, out, (uint32_t)n, total);
-        count_launches(1);
-        return;
-    }
     const size_t nb = (n + kScanTile - 1) / kScanTile;
     if (nb <= 1) {
         k_scan_block<<<1, kScanBlock, 0, s>>>(in, out, n, nullptr, total);
@@ -398,7 +366,7 @@ __device__ __forceinline__ int append_slot(const GridP &g, int face)
 // state.  The append order is slot order within each face (LoadPrtlOutliers
 // walks the array in order).  With blocks of 4096 slots, four rounds each, and
 // every position read: 2.1 M particles 68 us per step, 104 k particles 43 us;
-// now 46 and 24 us.
+// now 36 and 23 us.
 constexpr int kExchTile = 1024;
 static size_t exch_tiles(long long capacity) { return (size_t)((capacity + kExchTile - 1) / kExchTile) + 1; }
 __device__ __forceinline__ void load_quad_f64(const double *a, long long i, long long n, double v[4])
@@ -474,26 +442,82 @@ __device__ __forceinline__ void remove_prtl(const PartF64 &p, long long i)
 // (right-bound first, then left-bound; 8 doubles each: q, x, y, z, u, v, w,
 // flv, x already in the receiver's coordinates), and the y / z leavers are
 // appended after the local particles from scan position offs[2 ntiles] on.
-// The scatter stops before moving anything when the appended particles would
-// pass the capacity or the x leavers the outbox; the count then stays as it
-// was (and the overflow bit is set), so no stale slot becomes live.  The last
-// block to finish (cnt->scratch[0] counts them) updates the count, which
-// every block reads when it starts.
+// The scatter moves nothing when the appended particles would pass the
+// capacity or the x leavers the outbox; the count then stays as it was (and
+// the overflow bit is set), so no stale slot becomes live.  cnt->scratch[0] is
+// the count the appended particles follow, scratch[1] the overflow.
+__device__ __forceinline__ void exch_finish(Counters *cnt, long long total, long long sent, long long capacity,
+                                            long long out_cap, int *err)
+{
+    const long long n = cnt->used, t = total - sent;
+    const bool over = n + t > capacity || sent > out_cap;
+    cnt->scratch[0] = n;
+    cnt->scratch[1] = over;
+    cnt->append = t;
+    if (over) raise_error(err, PIC_DEVERR_OVERFLOW);
+    else cnt->used = n + t;
+}
+
+// Scan of the counts of the blocks that hold particles, face by face, and the
+// new particle count, by one block: 4096 counts per round.
+constexpr size_t kExchScanOne = 65536;   // counts; beyond it the multi-block scan
+__global__ void __launch_bounds__(kScanBlock) k_exch_scan(Counters *cnt, uint32_t *counts, uint32_t ntiles, int external,
+                                                          long long capacity, long long out_cap, int *err)
+{
+    __shared__ uint32_t warp_tot[kScanBlock / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t nu = min((uint32_t)((cnt->used + kExchTile - 1) / kExchTile), ntiles), n = 6 * nu;
+    uint32_t carry = 0, sent = 0;
+    // an empty first tile keeps the slab's sent counts defined
+    if (nu == 0 && threadIdx.x < 6) counts[(size_t)threadIdx.x * ntiles] = 0;
+    for (uint32_t base = 0; base < n; base += 4 * kScanBlock) {
+        uint32_t v[4], acc = 0;
+        uint32_t at[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t e = base + 4 * threadIdx.x + k, f = e < n ? e / nu : 0u;
+            at[k] = f * ntiles + (e - f * nu);
+            v[k] = e < n ? counts[at[k]] : 0u;
+            acc += v[k];
+        }
+        const uint32_t incl = warp_incl_scan(acc);
+        if (lane == 31) warp_tot[warp] = incl;
+        __syncthreads();
+        if (warp == 0) warp_tot[lane] = warp_incl_scan(warp_tot[lane]);
+        __syncthreads();
+        uint32_t run = carry + (incl - acc) + (warp > 0 ? warp_tot[warp - 1] : 0u);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t e = base + 4 * threadIdx.x + k;
+            if (e < n) counts[at[k]] = run;
+            run += v[k];
+        }
+        carry += warp_tot[kScanBlock / 32 - 1];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        if (external) sent = nu ? counts[2 * (size_t)ntiles] : 0u;
+        exch_finish(cnt, carry, sent, capacity, out_cap, err);
+    }
+}
+__global__ void k_exch_finish(Counters *cnt, const uint32_t *__restrict__ total, const uint32_t *__restrict__ sent,
+                              long long capacity, long long out_cap, int *err)
+{
+    exch_finish(cnt, *total, sent ? (long long)*sent : 0, capacity, out_cap, err);
+}
+
 template <int DIMS>
 __global__ void __launch_bounds__(256) k_exch_scatter(GridP g, PartF64 p, Counters *cnt, const uint32_t *__restrict__ offs,
-                                                      const uint32_t *__restrict__ total,
-                                                      const uint32_t *__restrict__ faces, size_t ntiles,
-                                                      long long capacity, int *err, double *out, long long out_cap)
+                                                      const uint32_t *__restrict__ faces, size_t ntiles, double *out)
 {
     constexpr int kWarps = 8;   // a warp takes 128 consecutive slots of the block
     __shared__ uint32_t wh[kWarps][6];
-    const long long n = cnt->used;
+    const long long n = cnt->scratch[0];
+    if ((long long)blockIdx.x * kExchTile >= n || cnt->scratch[1]) return;
     const uint32_t sent = g.x_external ? offs[2 * ntiles] : 0u;   // particles leaving through the x faces
-    const bool over = (long long)(*total - sent) + n > capacity || (long long)sent > out_cap;
-    if (over && blockIdx.x == 0 && threadIdx.x == 0) raise_error(err, PIC_DEVERR_OVERFLOW);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long q = (long long)blockIdx.x * (kExchTile / 4) + threadIdx.x;
-    const uint32_t word = !over && 4 * q < n ? faces[q] : 0u;
+    const uint32_t word = 4 * q < n ? faces[q] : 0u;
     if (__syncthreads_or(word != 0u)) {
         int sl[4];
 #pragma unroll
@@ -574,16 +598,6 @@ __global__ void __launch_bounds__(256) k_exch_scatter(GridP g, PartF64 p, Counte
             remove_prtl<DIMS>(p, i);
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd((unsigned long long *)&cnt->scratch[0], 1ull) == gridDim.x - 1) {
-            cnt->scratch[0] = 0;
-            const long long t = (long long)*total - (long long)sent;
-            cnt->append = t;
-            if (!over) cnt->used = n + t;
-        }
-    }
 }
 
 void launch_exchange_f64(const GridP &g, PartF64 &p, Counters *cnt, SortScratch &sc, long long capacity, int *err,
@@ -597,13 +611,15 @@ void launch_exchange_f64(const GridP &g, PartF64 &p, Counters *cnt, SortScratch 
     else if (g.dims == 3) k_exch_count<3, false><<<(unsigned)ntiles, 256, 0, s>>>(g, p, &cnt->used, counts, faces, ntiles);
     else if (marked) k_exch_count<2, true><<<(unsigned)ntiles, 256, 0, s>>>(g, p, &cnt->used, counts, faces, ntiles);
     else k_exch_count<2, false><<<(unsigned)ntiles, 256, 0, s>>>(g, p, &cnt->used, counts, faces, ntiles);
-    scan_exclusive_u32(counts, counts, 6 * ntiles, sc.scan_tmp, total, s);
-    if (g.dims == 3)
-        k_exch_scatter<3><<<(unsigned)ntiles, 256, 0, s>>>(g, p, cnt, counts, total, faces, ntiles, capacity, err, out,
-                                                          out_cap);
-    else
-        k_exch_scatter<2><<<(unsigned)ntiles, 256, 0, s>>>(g, p, cnt, counts, total, faces, ntiles, capacity, err, out,
-                                                          out_cap);
+    if (6 * ntiles <= kExchScanOne) {
+        k_exch_scan<<<1, kScanBlock, 0, s>>>(cnt, counts, (uint32_t)ntiles, g.x_external, capacity, out_cap, err);
+    } else {
+        scan_exclusive_u32(counts, counts, 6 * ntiles, sc.scan_tmp, total, s);
+        k_exch_finish<<<1, 1, 0, s>>>(cnt, total, g.x_external ? counts + 2 * ntiles : nullptr, capacity, out_cap, err);
+    }
+    count_launches(1);
+    if (g.dims == 3) k_exch_scatter<3><<<(unsigned)ntiles, 256, 0, s>>>(g, p, cnt, counts, faces, ntiles, out);
+    else k_exch_scatter<2><<<(unsigned)ntiles, 256, 0, s>>>(g, p, cnt, counts, faces, ntiles, out);
     if (g.x_external && sent_counts) {
         // right-bound (face 2, slot 0) and right + left-bound particle counts
         cudaMemcpyAsync(sent_counts, counts + ntiles, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
@@ -692,6 +708,26 @@ void launch_array_f64_to_f32(const double *in, float *out, long long n, cudaStre
 {
     if (n > 0) k_array_f64_to_f32<<<stream_grid(n), kThreads, 0, s>>>(in, out, n);
     count_launches(n > 0 ? 1 : 0);
+}
+
+struct FloatArrays {
+    const float *a[9];
+};
+__global__ void k_arrays_f32_to_f64(FloatArrays in, double *out, long long n)
+{
+    const float *__restrict__ a = in.a[blockIdx.y];
+    double *__restrict__ o = out + (size_t)blockIdx.y * n;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        o[i] = (double)a[i];
+}
+// m <= 9 arrays of n values, one after the other in out.
+void launch_arrays_f32_to_f64(const float *const *in, int m, double *out, long long n, cudaStream_t s)
+{
+    FloatArrays f = {};
+    for (int k = 0; k < m; k++) f.a[k] = in[k];
+    const long long b = (n + 255) / 256;
+    k_arrays_f32_to_f64<<<dim3((unsigned)(b < kSMs * 8 ? b : kSMs * 8), (unsigned)m), 256, 0, s>>>(f, out, n);
+    count_launches(1);
 }
 
 void launch_array_f32_to_f64(const float *in, double *out, long long n, cudaStream_t s)
