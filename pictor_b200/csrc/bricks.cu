@@ -406,14 +406,14 @@ bool choose_bricks(const GridP &g, double ppc, const int req[3], Bricks &bk)
         if (bk.t[d] >= 2) div_magic((unsigned)bk.t[d], bk.tmagic[d], bk.tshift[d]);
     }
     bk.ntiles = bk.nb[0] * bk.nb[1] * bk.nb[2];
-    bk.smem_floats = kBrickSmemBytes / 4;
+    bk.smem_floats = (g.geom == PIC_GEOM_CYLINDRICAL ? kBrickSmemCyl : kBrickSmemBytes) / 4;
     // the fallback box (brick + 1 cell per side) must fit, and the per-cell
     // counters of the in-brick order must fit beside its staging words
     for (int d = 0; d < g.dims; d++)
         if (bk.t[d] + 2 > kBoxAxisMax) return false;
     if ((long long)bk.t[0] * bk.t[1] * bk.t[2] * 4 > 32 * 1024) return false;
     return box_floats(g.dims, bk.t[0] + 2, bk.t[1] + 2, g.dims == 3 ? bk.t[2] + 2 : 1, box_current_words(g)) <=
-           bk.smem_floats;
+           kBrickSmemBytes / 4;
 }
 
 }  // namespace pic

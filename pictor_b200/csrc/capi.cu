@@ -1117,10 +1117,9 @@ int pic_create(const pic_config *cfg, pic_handle **out)
             (r = dalloc(h, &bk.scan_tmp, scan_tmp_len(nt + 1))) ||
             (r = dalloc(h, &bk.wmax_bits, 1))) {
         }
-        // the node averages of the Cartesian tiled mover, computed once per
-        // move instead of by every brick for its box
-        if (!r && g.geom == PIC_GEOM_CARTESIAN &&
-            !(r = dalloc(h, (char **)&bk.nodeA, (size_t)g.ncell * sizeof(float4))))
+        // the node averages of the tiled movers, computed once per move
+        // instead of by every brick for its box
+        if (!r && !(r = dalloc(h, (char **)&bk.nodeA, (size_t)g.ncell * sizeof(float4))))
             r = dalloc(h, (char **)&bk.nodeB, (size_t)g.ncell * sizeof(float2));
         // the boxes' report to step_reorders
         if (!r && g.geom == PIC_GEOM_CARTESIAN && !g.x_external) {
@@ -1163,7 +1162,7 @@ int pic_create(const pic_config *cfg, pic_handle **out)
             !(r = dalloc(h, &T.qmax, 1)))
             h->tiled64 = true;
         T.marks = reinterpret_cast<uint8_t *>(exchange_marks(h->sc));
-        if (!r && g.dims == 3 && g.geom == PIC_GEOM_CARTESIAN) r = dalloc(h, &T.node, 6 * (size_t)g.ncell);
+        if (!r && g.dims == 3) r = dalloc(h, &T.node, 6 * (size_t)g.ncell);
     }
     if (!r && c.exact_current) {
         SegRecords &R = h->rec;

@@ -665,8 +665,13 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_cyl_move_tiled(GridP g, CylP
                 double wt[8];
                 weights<double, 3>(x - i, y - j, z - k, wt);
                 gather_box64<3>(ctx.bx, ctx.sN, nb, wt, pE, pB);
-            } else {
-                interp3(g, Ex, Ey, Ez, Bx, By, Bz, x, y, z, pE, pB);
+            } else {   // from the node array, as a box of the whole grid
+                Box64 whole;
+                whole.NX = g.mx;
+                whole.NXY = (int)g.sz;
+                double wt[8];
+                weights<double, 3>(x - i, y - j, z - k, wt);
+                gather_box64<3>(whole, T.node + 6 * cidx(g, i, j, k), 0, wt, pE, pB);
             }
         };
         auto dep = [&](int i, int j, int k, const double *o, bool far) {
@@ -707,6 +712,7 @@ void launch_cyl_move_deposit(const GridP &g, const PartF64 &p, const Counters *c
             cudaFuncSetAttribute(k_cyl_move_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, kTile64SmemBytes);
             attr_set = true;
         }
+        launch_node_f64(g, *T, E, B, s);
         k_cyl_move_tiled<<<T->ntiles, kT64Threads, T->smem_bytes, s>>>(g, cp, p, *T, E[0], E[1], E[2], B[0], B[1],
                                                                         B[2], J[0], J[1], J[2], err);
         count_launches(1);
@@ -767,6 +773,21 @@ __device__ __forceinline__ void interp3f(const GridP &g, const float *__restrict
         pB[0] = fmaf(wt[nn], vbx, pB[0]);
         pB[1] = fmaf(wt[nn], vby, pB[1]);
         pB[2] = fmaf(wt[nn], vbz, pB[2]);
+    }
+}
+
+// The same from the node averages of the grid (the same values, one load pair
+// per node instead of 20): theta and z of the node wrapped to the interior.
+__device__ __forceinline__ void interp_nodes(const GridP &g, const TileBox &tb, int ip, int jp, int kp, float dx, float dy,
+                                             float dz, float pE[3], float pB[3])
+{
+    float wt[8];
+    weights_f32<3>(dx, dy, dz, wt);
+    pE[0] = pE[1] = pE[2] = pB[0] = pB[1] = pB[2] = 0.f;
+#pragma unroll
+    for (int nn = 0; nn < 8; nn++) {
+        const long long nd = cidx(g, ip + (nn & 1), wrap_index(jp + ((nn >> 1) & 1), g.my), wrap_index(kp + ((nn >> 2) & 1), g.mz));
+        accum(wt[nn], ldro(tb.gA + nd), ldro(tb.gB + nd), pE, pB);
     }
 }
 
@@ -914,6 +935,8 @@ __device__ __forceinline__ void cyl_push_f32(const GridP &g, const CylP &cp, con
             weights_f32<3>(dx, dy, dz, wt);
             pE[0] = pE[1] = pE[2] = pB[0] = pB[1] = pB[2] = 0.f;
             gather_box<3>(tb, l0 + tb.NX * l1 + tb.NXY * l2, wt, pE, pB);
+        } else if (TILED) {
+            interp_nodes(g, tb, i, j, k, dx, dy, dz, pE, pB);
         } else {
             interp3f(g, Ex, Ey, Ez, Bx, By, Bz, i, j, k, dx, dy, dz, pE, pB);
         }
@@ -959,6 +982,8 @@ __device__ __forceinline__ void cyl_push_f32(const GridP &g, const CylP &cp, con
             weights_f32<3>(ox, oy, oz, wt);
             pE[0] = pE[1] = pE[2] = pB[0] = pB[1] = pB[2] = 0.f;
             gather_box<3>(tb, (l0 + sx) + tb.NX * (l1 + sy) + tb.NXY * (l2 + sz), wt, pE, pB);
+        } else if (TILED) {
+            interp_nodes(g, tb, ni, nj, nk, ox, oy, oz, pE, pB);
         } else {
             interp3f(g, Ex, Ey, Ez, Bx, By, Bz, ni, nj, nk, ox, oy, oz, pE, pB);
         }
@@ -1169,7 +1194,9 @@ __global__ void __launch_bounds__(kTileThreads, 2)
     int home_lo[3], home_hi[3];
     brick_home<3>(g, bk, b, tb, home_lo, home_hi);
     // a Strang move is below one cell per axis, a sub-stepped one below two
-    tile_setup<3, false, true>(g, bk, b, p1 - p0, 1, 2.f, sm, ts, tb, home_lo, home_hi, Ex, Ey, Ez, Bx, By, Bz);
+    tb.gA = bk.nodeA;
+    tb.gB = bk.nodeB;
+    tile_setup<3, false, true, true>(g, bk, b, p1 - p0, 1, 2.f, sm, ts, tb, home_lo, home_hi, Ex, Ey, Ez, Bx, By, Bz);
     Bounds bd;
     bd.init();
     JAcc acc;
@@ -1205,12 +1232,13 @@ void launch_cyl_move_deposit_f32_tiled(const GridP &g, const PartF32 &p, const B
 {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_cyl_move_f32_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, kBrickSmemBytes);
+        cudaFuncSetAttribute(k_cyl_move_f32_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, kBrickSmemCyl);
         attr_set = true;
     }
     const CylP cp = cyl_params(g);
     // the queue of near-axis slots: the brick-id scratch of the reorder, its
     // length in the scan scratch (both free between reorders)
+    launch_node_avg(g, bk, E, B, s);
     cudaMemsetAsync(bk.count, 0, sizeof(uint32_t), s);
     k_cyl_move_f32_tiled<<<bk.ntiles, kTileThreads, bk.smem_floats * 4, s>>>(g, cp, p, bk, E[0], E[1], E[2], B[0],
                                                                             B[1], B[2], J[0], J[1], J[2], err);

@@ -84,12 +84,13 @@ struct Tiles64 {
                                   // that the next groups start at the first interior row)
     int smem_bytes;
     uint8_t *marks;               // Cartesian: exchange_marks
-    double *node;                 // 3D Cartesian: the 6 node values of every node 2 .. m - 1, or null
+    double *node;                 // 3D: the 6 node values of every node 2 .. m - 1, or null
 };
 void choose_tiles64(const GridP &g, Tiles64 &T);
 // After a reorder: the tiles' slot ranges from the sorted keys, the boxes.
 void launch_tiles64_after_reorder(const GridP &g, const uint32_t *keys, const Counters *cnt, Tiles64 &T,
                                   cudaStream_t s);
+void launch_node_f64(const GridP &g, const Tiles64 &T, double *const E[3], double *const B[3], cudaStream_t s);
 void launch_move_deposit_f64_tiled(const GridP &g, const PartF64 &p, const Counters *cnt, const Tiles64 &T,
                                    double *const E[3], double *const B[3], double *const J[3], int *err,
                                    cudaStream_t s);
@@ -101,7 +102,9 @@ void launch_move_deposit_f32(const GridP &g, const PartF32 &p, const Counters *c
 // [tile_start[b], tile_start[b+1]); box[8b..8b+5] holds the lower and upper
 // cell bounds (relative to the brick centre 3 + nb*t + t/2, unwrapped) of
 // where the brick's particles are, which the tiled mover reads and rewrites.
-constexpr int kBrickSmemBytes = 64 * 1024;   // dynamic shared memory of the tiled mover (node + current box)
+// Dynamic shared memory of a tiled mover (node + current box): 3 CTAs per SM;
+// the cylindrical mover, whose registers allow 2, takes the room of 2.
+constexpr int kBrickSmemBytes = 64 * 1024, kBrickSmemCyl = 100 * 1024;
 struct Bricks {
     uint32_t *tile_start;   // ntiles + 1
     int *box;               // 8 per brick
@@ -142,6 +145,8 @@ constexpr int kBoxAxisMax = 64;   // cells per axis of a mover box
 // at ppc particles per cell.  Returns false if the brick plus one cell on
 // each side would not fit the mover's shared memory.
 bool choose_bricks(const GridP &g, double ppc, const int req[3], Bricks &bk);
+// The node averages the tiled FP32 movers read (mover_f32.cu).
+void launch_node_avg(const GridP &g, const Bricks &bk, float *const E[3], float *const B[3], cudaStream_t s);
 // Tiled FP32 mover: one CTA per brick.
 // One run of a batch of FP32 runs stepped by shared kernels (one launch per
 // phase for all runs).  `cur` is the run's current particle buffer; a

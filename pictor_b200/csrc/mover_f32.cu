@@ -62,20 +62,23 @@ __global__ void __launch_bounds__(kTileThreads, 3)
 }
 
 // The node averages of every interior node (node_avg, the same expressions
-// as the bricks' own staging), for the tiled mover's boxes.  A (32, 8) block
-// covers 32 x 8 nodes of kNodeKz consecutive z planes (3D).
+// as the bricks' own staging), for the tiled movers' boxes; along x of the
+// nodes i0 .. i1 (the cylinder's radius is not periodic: its boxes reach into
+// the ghost columns).  A (32, 8) block covers 32 x 8 nodes of kNodeKz
+// consecutive z planes (3D).
 constexpr int kNodeKz = 4;
 template <int DIMS>
 __global__ void __launch_bounds__(kThreads) k_node_avg(GridP g, const float *__restrict__ Ex, const float *__restrict__ Ey,
                                                        const float *__restrict__ Ez, const float *__restrict__ Bx,
                                                        const float *__restrict__ By, const float *__restrict__ Bz,
-                                                       float4 *nodeA, float2 *nodeB, uint32_t *over)
+                                                       float4 *nodeA, float2 *nodeB, uint32_t *over, int i0,
+                                                       int i1)
 {
     if (over && blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x + threadIdx.y == 0)
         *over += 1;   // this move's number since the reorder (tile_finish)
     const int sy = (int)g.sy, sz = (int)g.sz;
-    const int i = 3 + blockIdx.x * 32 + threadIdx.x, j = 3 + blockIdx.y * 8 + threadIdx.y;
-    if (i > g.nx + 2 || j > g.ny + 2) return;
+    const int i = i0 + blockIdx.x * 32 + threadIdx.x, j = 3 + blockIdx.y * 8 + threadIdx.y;
+    if (i > i1 || j > g.ny + 2) return;
     for (int z = 0; z < (DIMS == 3 ? kNodeKz : 1); z++) {
         const int k = DIMS == 3 ? 3 + blockIdx.z * kNodeKz + z : 1;
         if (DIMS == 3 && k > g.nz + 2) break;
@@ -86,6 +89,20 @@ __global__ void __launch_bounds__(kThreads) k_node_avg(GridP g, const float *__r
         nodeA[nd] = A;
         nodeB[nd] = Bv;
     }
+}
+
+void launch_node_avg(const GridP &g, const Bricks &bk, float *const E[3], float *const B[3], cudaStream_t s)
+{
+    const bool cyl = g.geom == PIC_GEOM_CYLINDRICAL;
+    const int i0 = cyl ? 1 : 3, i1 = cyl ? g.mx : g.nx + 2;
+    const dim3 grid((unsigned)((i1 - i0 + 32) / 32), (unsigned)((g.ny + 7) / 8),
+                    (unsigned)(g.dims == 3 ? (g.nz + kNodeKz - 1) / kNodeKz : 1)),
+        block(32, 8, 1);
+    if (g.dims == 3)
+        k_node_avg<3><<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], bk.nodeA, bk.nodeB, bk.over, i0, i1);
+    else
+        k_node_avg<2><<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], bk.nodeA, bk.nodeB, bk.over, i0, i1);
+    count_launches(1);
 }
 
 // The tiled mover for all runs of a batch in one launch: CTA b takes brick b
@@ -188,16 +205,7 @@ void launch_move_deposit_f32_tiled(const GridP &g, const PartF32 &p, const Brick
         return;
     }
     const bool pre = bk.nodeA != nullptr;
-    if (pre) {
-        const dim3 grid((unsigned)((g.nx + 31) / 32), (unsigned)((g.ny + 7) / 8),
-                        (unsigned)(g.dims == 3 ? (g.nz + kNodeKz - 1) / kNodeKz : 1)),
-            block(32, 8, 1);
-        if (g.dims == 3)
-            k_node_avg<3><<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], bk.nodeA, bk.nodeB, bk.over);
-        else
-            k_node_avg<2><<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], bk.nodeA, bk.nodeB, bk.over);
-        count_launches(1);
-    }
+    if (pre) launch_node_avg(g, bk, E, B, s);
 #define PIC_MOVE_TILED(D, X, P)                                                                                      \
     k_move_f32_tiled<D, X, P><<<bk.ntiles, kTileThreads, bytes, s>>>(g, p, bk, E[0], E[1], E[2], B[0], B[1], B[2], J[0], \
                                                                     J[1], J[2], err)

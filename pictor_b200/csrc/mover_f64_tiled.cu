@@ -64,24 +64,6 @@ __global__ void k_tile_starts(GridP g, Tiles64 T, const uint32_t *__restrict__ k
     }
 }
 
-// The node values of every node 2 .. m - 1 (3D), which the tiles copy and the
-// particles outside their tile's box read: 3 loads per node instead of 20.
-__global__ void __launch_bounds__(256) k_node_f64(GridP g, const double *__restrict__ Ex, const double *__restrict__ Ey,
-                                                  const double *__restrict__ Ez, const double *__restrict__ Bx,
-                                                  const double *__restrict__ By, const double *__restrict__ Bz,
-                                                  double *node)
-{
-    const int i = 2 + blockIdx.x * 32 + threadIdx.x, j = 2 + blockIdx.y * 8 + threadIdx.y, k = 2 + blockIdx.z;
-    if (i > g.mx - 1 || j > g.my - 1 || k > g.mz - 1) return;
-    const long long nd = cidx(g, i, j, k);
-    double v[6];
-    node_values64<3>(g, Ex, Ey, Ez, Bx, By, Bz, nd, v);
-    double2 *o = reinterpret_cast<double2 *>(node + 6 * nd);
-    o[0] = make_double2(v[0], v[1]);
-    o[1] = make_double2(v[2], v[3]);
-    o[2] = make_double2(v[4], v[5]);
-}
-
 // A particle's move: the current of its start cell (a particle that stays in
 // its cell: both segments) goes to the box at once, the second segment of one
 // that crosses a face is queued per warp (warp's queue rows: F x, y, z, W x,
@@ -270,7 +252,32 @@ __global__ void __launch_bounds__(kT64Threads, 2)
     }, [&](const Tile64Ctx &ctx) { drain(ctx); });
 }
 
+// The node values of every node 2 .. m - 1 (3D), which the tiles copy and the
+// particles outside their tile's box read: 3 loads per node instead of 20.
+__global__ void __launch_bounds__(256) k_node_f64(GridP g, const double *__restrict__ Ex, const double *__restrict__ Ey,
+                                                  const double *__restrict__ Ez, const double *__restrict__ Bx,
+                                                  const double *__restrict__ By, const double *__restrict__ Bz,
+                                                  double *node)
+{
+    const int i = 2 + blockIdx.x * 32 + threadIdx.x, j = 2 + blockIdx.y * 8 + threadIdx.y, k = 2 + blockIdx.z;
+    if (i > g.mx - 1 || j > g.my - 1 || k > g.mz - 1) return;
+    const long long nd = cidx(g, i, j, k);
+    double v[6];
+    node_values64<3>(g, Ex, Ey, Ez, Bx, By, Bz, nd, v);
+    double2 *o = reinterpret_cast<double2 *>(node + 6 * nd);
+    o[0] = make_double2(v[0], v[1]);
+    o[1] = make_double2(v[2], v[3]);
+    o[2] = make_double2(v[4], v[5]);
+}
+
 }  // namespace
+
+void launch_node_f64(const GridP &g, const Tiles64 &T, double *const E[3], double *const B[3], cudaStream_t s)
+{
+    const dim3 block(32, 8, 1), grid((g.mx - 2 + 31) / 32, (g.my - 2 + 7) / 8, g.mz - 2);
+    k_node_f64<<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], T.node);
+    count_launches(1);
+}
 
 void choose_tiles64(const GridP &g, Tiles64 &T)
 {
@@ -312,11 +319,7 @@ void launch_move_deposit_f64_tiled(const GridP &g, const PartF64 &p, const Count
         cudaFuncSetAttribute(k_move_f64_tiled<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTile64SmemCart);
         attr_set = true;
     }
-    if (T.node) {
-        const dim3 block(32, 8, 1), grid((g.mx - 2 + 31) / 32, (g.my - 2 + 7) / 8, g.mz - 2);
-        k_node_f64<<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], T.node);
-        count_launches(1);
-    }
+    if (T.node) launch_node_f64(g, T, E, B, s);
     const int blocks = kAppendBlocks + T.ntiles;
     if (g.dims == 3)
         k_move_f64_tiled<3><<<blocks, kT64Threads, T.smem_bytes, s>>>(g, p, T, cnt, E[0], E[1], E[2], B[0], B[1], B[2],
