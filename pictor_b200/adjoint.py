@@ -96,7 +96,7 @@ class Adjoint:
         check(self.L.pic_adj_fetch_particles(self.h, C.byref(n), None, None, None, None, None, None, None, None, None),
               "pic_adj_fetch_particles")
         n = n.value
-        out = {k: np.zeros(n) for k in ("u", "v", "w", "x", "y")}
+        out = {k: np.empty(n) for k in ("u", "v", "w", "x", "y")}   # filled below
         par = np.zeros(3)
         t = np.asarray(temp if temp is not None else self.temp, dtype=np.float64)
         check(self.L.pic_adj_gradient(self.h, float(self.drift if drift is None else drift), dptr(t), dptr(out["u"]),

@@ -366,7 +366,7 @@ void launch_reorder_f32(const GridP &g, const PartF32 &p, const PartF32 &out, Co
 }
 
 // Brick shape for a fill of ppc particles per cell: about 4096 particles per
-// brick, in 2D fewer where that leaves less than two bricks per SM (down to
+// brick, in 2D fewer where that leaves less than a brick per SM (down to
 // 512, two rounds of a CTA: 64^2 cells of 8 particles as 64 bricks instead of
 // 16 move in 15.5 instead of 21.8 us; in 3D a smaller brick's box is mostly
 // margin), x first, up to 8x8x8 (3D) / 32x32 (2D) so that the boxes of the
@@ -383,7 +383,7 @@ bool choose_bricks(const GridP &g, double ppc, const int req[3], Bricks &bk)
             if (t[d] < 1) return false;
     } else {
         const double fill = ppc > 0.5 ? ppc : 0.5;
-        const double share = fill * g.nx * g.ny * (g.dims == 3 ? g.nz : 1) / (2 * kSMs);
+        const double share = fill * g.nx * g.ny * (g.dims == 3 ? g.nz : 1) / kSMs;
         const double target = (g.dims == 3 || share > 4096.0 ? 4096.0 : share > 512.0 ? share : 512.0) / fill;
         const int ns = g.dims == 3 ? 4 : 5;
         int pick = ns - 1;

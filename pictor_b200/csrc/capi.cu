@@ -200,6 +200,58 @@ void maxbolt_table(int n, std::vector<double> &X, std::vector<double> &P)
 
 constexpr int kPinWords = 80, kPinErr = 64, kPinCount = 65, kPinOver = 66;
 
+// Pinned words of the handles, one block of kPinSlots slots shared by all of
+// them (pinning memory takes milliseconds, most of what creating a small run
+// costs): allocated with the first handle, freed with the last.  A handle
+// beyond the slots pins its own.
+constexpr int kPinSlots = 256;
+struct PinPool {
+    std::mutex mu;
+    double *base = nullptr;
+    std::vector<int> free_slots;
+    int live = 0;
+};
+PinPool g_pins;
+
+double *pin_take()
+{
+    std::lock_guard<std::mutex> lk(g_pins.mu);
+    if (!g_pins.base) {
+        if (cudaHostAlloc((void **)&g_pins.base, (size_t)kPinSlots * kPinWords * sizeof(double),
+                          cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            g_pins.base = nullptr;
+            return nullptr;
+        }
+        g_pins.free_slots.clear();
+        for (int k = kPinSlots - 1; k >= 0; k--) g_pins.free_slots.push_back(k);
+    }
+    double *p = nullptr;
+    if (!g_pins.free_slots.empty()) {
+        p = g_pins.base + (size_t)g_pins.free_slots.back() * kPinWords;
+        g_pins.free_slots.pop_back();
+    } else if (cudaHostAlloc((void **)&p, kPinWords * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable) !=
+               cudaSuccess) {
+        p = nullptr;
+    }
+    if (p) g_pins.live++;
+    return p;
+}
+
+void pin_return(double *p)
+{
+    if (!p) return;
+    std::lock_guard<std::mutex> lk(g_pins.mu);
+    const size_t words = (size_t)kPinSlots * kPinWords;
+    if (g_pins.base && p >= g_pins.base && p < g_pins.base + words)
+        g_pins.free_slots.push_back((int)((p - g_pins.base) / kPinWords));
+    else
+        cudaFreeHost(p);
+    if (--g_pins.live == 0) {
+        cudaFreeHost(g_pins.base);
+        g_pins.base = nullptr;
+    }
+}
+
 // Finish a synchronous entry point: launch errors, stream errors, device
 // error word (copied behind the work, so one wait covers all three).
 int finish(pic_handle *h)
@@ -973,7 +1025,7 @@ void pic_destroy(pic_handle *h)
         if (h->ev_done[b]) cudaEventDestroy(h->ev_done[b]);
     }
     if (h->ev_group) cudaEventDestroy(h->ev_group);
-    if (h->pin) cudaFreeHost(h->pin);
+    pin_return(h->pin);
     for (void *p : h->allocs) cudaFree(p);
     if (h->cs) cudaStreamDestroy(h->cs);
     if (h->s) cudaStreamDestroy(h->s);
@@ -1087,7 +1139,7 @@ int pic_create(const pic_config *cfg, pic_handle **out)
 
     int r = PIC_OK;
     if (cudaStreamCreateWithFlags(&h->s, cudaStreamNonBlocking) != cudaSuccess) r = PIC_ERR_CUDA;
-    if (!r && cudaHostAlloc((void **)&h->pin, kPinWords * sizeof(double), cudaHostAllocMapped) != cudaSuccess) r = PIC_ERR_OOM;
+    if (!r && !(h->pin = pin_take())) r = PIC_ERR_OOM;
     const size_t fb = field_bytes(h);
     for (int k = 0; k < 3 && !r; k++) {
         if ((r = dalloc(h, (char **)&h->E[k], fb))) break;

@@ -196,7 +196,8 @@ class Simulation:
 
     def fetch_particles(self) -> Particles:
         n = self.particle_count()
-        p = Particles.empty(n)
+        # every value is written below: no zeroing, whose pages would be touched twice
+        p = Particles(*(np.empty(n) for _ in range(7)), np.empty(n, dtype=np.int32))
         got = C.c_int64()
         check(self.L.pic_fetch_particles(self.h, C.byref(got), *[dptr(getattr(p, k)) for k in Particles.NAMES[:7]],
                                          iptr(p.flv)), "pic_fetch_particles")

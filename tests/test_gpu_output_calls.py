@@ -1,0 +1,88 @@
+"""What an output call returns, over the routes it can take: the charge density
+by bricks (after a reorder, boxes kept, cut or outgrown) against the particles
+in any order, the kinetic energy of more flavours than the two kept in
+registers, and the fields of small grids (one conversion, one or more copies)
+and of grids past the staging buffer."""
+import numpy as np
+import pytest
+
+from pictor_b200.simulation import Fields
+
+from .test_gpu_boxes import _cfg, _hot
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape,dims,ppc,steps", [((24, 20, 17), 3, 6, 0), ((41, 24, 23), 3, 6, 14),
+                                                  ((96, 75, 1), 2, 6, 25), ((5, 5, 5), 3, 1, 2)])
+def test_density_by_bricks(shape, dims, ppc, steps):
+    """The diagnostics of a reordered run and of the same slots loaded into
+    one that was not: the density scale and the Gauss residual to the rounding
+    of the sums (1e-12 of the largest density), the energies to 1e-12."""
+    from pictor_b200 import Simulation
+
+    cfg, sc = _cfg(shape, dims, ppc, 0)
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        p = _hot(*shape, dims, ppc, 21)
+        p.q *= np.random.default_rng(2).uniform(0.2, 3.0, size=len(p))
+        a.load_particles(p)
+        a.reorder()
+        a.step(steps)
+        b.load_particles(a.fetch_particles())
+        b.load_fields(a.fetch_fields())
+        da, db = a.diagnostics(sc["masse"]), b.diagnostics(sc["masse"])
+    assert db["rho_max"] > 0
+    for k in ("rho_max", "gauss_linf"):
+        assert abs(da[k] - db[k]) <= 1e-12 * db["rho_max"], k
+    for k in ("B2", "E2"):
+        assert abs(da[k] - db[k]) <= 1e-12 * max(db[k], 1e-300)
+    assert np.allclose(da["kinetic"], db["kinetic"], rtol=1e-12)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_kinetic_energy_of_every_flavour(precision):
+    from pictor_b200 import PicConfig, Simulation
+
+    qm = tuple([1.0, -1.0, 0.5, -1.0, 0.25] + [1.0] * 10)
+    cfg = PicConfig(nx=12, ny=10, dims=2, c=0.45, qi=0.01, qm=qm, precision=precision, capacity=1 << 14)
+    p = _hot(12, 10, 1, 2, 20, 3, 0.3)
+    n = len(p)
+    p.flv[:] = 1 + np.arange(n) % 15
+    p.q[:] = np.where(np.isin(p.flv, (2, 4)), -1.0, 1.0)
+    with Simulation(cfg) as s:
+        s.load_particles(p)
+        got = s.diagnostics(0.02)["kinetic"]
+        f = s.fetch_particles()
+    gm = np.sqrt(1 + f.u ** 2 + f.v ** 2 + f.w ** 2) - 1
+    m = np.where(f.q > 0, f.q * 0.01 / np.array((0.0,) + qm)[f.flv], 0.02) * 0.45 ** 2
+    want = np.array([(gm * m)[f.flv == k].sum() for k in range(1, 16)])
+    assert np.allclose(got, want, rtol=1e-12)
+
+
+@pytest.mark.parametrize("nx,ny", [(5, 5), (64, 33), (900, 700)])
+@pytest.mark.parametrize("layout", ["separate", "contiguous", "gaps"])
+def test_fetched_fields(nx, ny, layout):
+    """Loaded fields come back (as FP32 keeps them) into arrays of their own,
+    into one block, and into rows with gaps; with and without the current.
+    The small grids' arrays fit the staging buffer together, the last one's
+    do not."""
+    from pictor_b200 import PicConfig, Simulation
+
+    cfg = PicConfig(nx=nx, ny=ny, dims=2, c=0.45, qi=0.01, precision="fp32", capacity=4096)
+    n = int(np.prod(cfg.shape))
+    rng = np.random.default_rng(nx)
+    f = Fields(*(np.asfortranarray(rng.normal(size=cfg.shape)) for _ in range(9)))
+    with Simulation(cfg) as s:
+        s.load_fields(f)
+        s.load_current(f.Jx, f.Jy, f.Jz)
+        for with_j in (True, False):
+            row = n if layout == "contiguous" else n + 3
+            buf = np.full((9, row), 7.0)
+            out = None if layout == "separate" else Fields(*(buf[k, :n].reshape(cfg.shape, order="F") for k in range(9)))
+            got = s.fetch_fields(with_j, out=out)
+            for k in ("Ex", "Ey", "Ez", "Bx", "By", "Bz") + (("Jx", "Jy", "Jz") if with_j else ()):
+                assert np.array_equal(getattr(got, k), getattr(f, k).astype(np.float32).astype(np.float64)), k
+            if layout == "gaps":
+                assert (buf[:, n:] == 7.0).all()
+            if not with_j and out is not None:
+                assert (buf[6:] == 7.0).all()
