@@ -323,18 +323,23 @@ __global__ void k_brick_prepare(GridP g, Bricks bk)
     box[6] = box[7] = 0;
 }
 
-__global__ void k_brick_finish(Bricks bk, Counters *cnt)
+__global__ void __launch_bounds__(kOverWords) k_brick_finish(Bricks bk, Counters *cnt)
 {
-    const long long live = bk.tile_start[bk.ntiles];
-    cnt->used = live;
-    cnt->np = live;
-    if (bk.over) {   // the first move since the last reorder that left over 1/kOverShare of the boxes too large, 0 = none
-        uint32_t first = 0;
-        for (int j = kOverWords - 2; j >= 1; j--)
-            if (bk.over[1 + j] > (uint32_t)(bk.ntiles / kOverShare)) first = (uint32_t)j;
-        for (int j = 0; j < kOverWords; j++) bk.over[j] = 0;
-        if (first) *(volatile uint32_t *)bk.over_host = first;   // kept until the host has read it
+    if (threadIdx.x == 0) {
+        const long long live = bk.tile_start[bk.ntiles];
+        cnt->used = live;
+        cnt->np = live;
     }
+    if (!bk.over) return;
+    // the first move since the last reorder that left over 1/kOverShare of the boxes too large, 0 = none
+    __shared__ uint32_t first;
+    const uint32_t j = threadIdx.x;
+    if (j == 0) first = kOverWords;
+    __syncthreads();
+    if (j >= 2 && bk.over[j] > (uint32_t)(bk.ntiles / kOverShare)) atomicMin(&first, j - 1);
+    __syncthreads();
+    bk.over[j] = 0;
+    if (j == 0 && first < kOverWords) *(volatile uint32_t *)bk.over_host = first;   // kept until the host has read it
 }
 
 static unsigned grid_for(long long n)
@@ -361,7 +366,7 @@ void launch_reorder_f32(const GridP &g, const PartF32 &p, const PartF32 &out, Co
         attr_set = true;
     }
     k_brick_order<<<bk.ntiles, kOrderThreads, smem, s>>>(g, bk, p, out, g.dims == 3);
-    k_brick_finish<<<1, 1, 0, s>>>(bk, cnt);
+    k_brick_finish<<<1, kOverWords, 0, s>>>(bk, cnt);
     count_launches(6);
 }
 

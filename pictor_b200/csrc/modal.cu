@@ -157,8 +157,8 @@ __device__ __forceinline__ void emit(const GridP &g, const GridP &gm, const doub
     }
 }
 
-// The B and E phases: one thread per interior (r, z) updates the planes of
-// its cell, applies the axis conditions (the thread next to the axis, whose
+// The B and E phases: one thread per interior (r, z) and component updates
+// the planes of its cell, applies the axis conditions (the thread next to the axis, whose
 // new values they are made of) and writes the planes, their theta-gridded
 // synthesis and all images; the columns an update leaves alone are emitted as
 // they are.  With launches for the update, the axis, the halo, the synthesis,
@@ -178,34 +178,44 @@ __global__ void __launch_bounds__(128) k_modal_bhalf(GridP g, GridP gm, ModalP m
     theta_table(m, tab, tab + m.ny);
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, k = 3 + blockIdx.y * blockDim.y + threadIdx.y;
     if (i > gm.mx || k > gm.mz - 3 || i == 3) return;   // column 3 belongs to the thread of column 4
-    M3<T> bx = ld3(gm, Bx, i, k), by = ld3(gm, By, i, k), bz = ld3(gm, Bz, i, k);
+    const int comp = blockIdx.z;
+    T *B = comp == 0 ? Bx : comp == 1 ? By : Bz, *F = comp == 0 ? Fx : comp == 1 ? Fy : Fz;
+    M3<T> v = ld3(gm, B, i, k);
     if (i >= 4 && i <= gm.mx - 1) {
         const T h = (T)gm.h, dtheta = (T)m.dtheta;
         const T r = ((T)i - (T)3.0) + (T)m.rmin;
         const T rp_half = r + (T)0.5, rp = r + (T)1.0;
         if (FDTD == PIC_FDTD_YEE) {
-            const M3<T> ez = ld3(gm, Ez, i, k), ex = ld3(gm, Ex, i, k), ey = ld3(gm, Ey, i, k);
-            bx = bx - (h * (tp(m, ez) - ez)) / (r * dtheta) + h * (ld3(gm, Ey, i, k + 1) - ey);
-            by = by - h * (ld3(gm, Ex, i, k + 1) - ex) + h * (ld3(gm, Ez, i + 1, k) - ez);
-            bz = bz - (h * ((rp * ld3(gm, Ey, i + 1, k) - r * ey) - (tp(m, ex) - ex) / dtheta)) / rp_half;
+            if (comp == 0) {
+                const M3<T> ez = ld3(gm, Ez, i, k), ey = ld3(gm, Ey, i, k);
+                v = v - (h * (tp(m, ez) - ez)) / (r * dtheta) + h * (ld3(gm, Ey, i, k + 1) - ey);
+            } else if (comp == 1) {
+                const M3<T> ez = ld3(gm, Ez, i, k), ex = ld3(gm, Ex, i, k);
+                v = v - h * (ld3(gm, Ex, i, k + 1) - ex) + h * (ld3(gm, Ez, i + 1, k) - ez);
+            } else {
+                const M3<T> ex = ld3(gm, Ex, i, k), ey = ld3(gm, Ey, i, k);
+                v = v - (h * ((rp * ld3(gm, Ey, i + 1, k) - r * ey) - (tp(m, ex) - ex) / dtheta)) / rp_half;
+            }
         } else {
-            bx = bx - (h * mgy(gm, m, Ez, i, k)) / (r * dtheta) + h * mgz(gm, m, Ey, i, k);
-            by = by - h * mgz(gm, m, Ex, i, k) + h * mgx(gm, Ez, i, k);
-            bz = bz - (h * (mgx1(gm, Ey, i, k, rp, r) - mgy(gm, m, Ex, i, k) / dtheta)) / rp_half;
+            if (comp == 0) v = v - (h * mgy(gm, m, Ez, i, k)) / (r * dtheta) + h * mgz(gm, m, Ey, i, k);
+            else if (comp == 1) v = v - h * mgz(gm, m, Ex, i, k) + h * mgx(gm, Ez, i, k);
+            else v = v - (h * (mgx1(gm, Ey, i, k, rp, r) - mgy(gm, m, Ex, i, k) / dtheta)) / rp_half;
         }
     }
     if (i == 4) {
-        const T s = -(T)(gm.h * m.ax_perm_area) * ((T)m.ny * ld3(gm, Ey, 4, k).a);
-        emit<T>(g, gm, cs, sn, Bz, Fz, 3, k, {ld3(gm, Bz, 3, k).a + s, (T)0, (T)0});
-        emit(g, gm, cs, sn, By, Fy, 3, k, ((T)0.5 * (by - partner(by))));
-        emit<T>(g, gm, cs, sn, By, Fy, 2, k, {-by.a, by.b, by.c});
-        emit<T>(g, gm, cs, sn, Bx, Fx, 3, k, {-bx.a, bx.b, bx.c});
-        emit(g, gm, cs, sn, Bz, Fz, 2, k, partner(bz));
+        if (comp == 0) {
+            emit<T>(g, gm, cs, sn, B, F, 3, k, {-v.a, v.b, v.c});
+        } else if (comp == 1) {
+            emit(g, gm, cs, sn, B, F, 3, k, (T)0.5 * (v - partner(v)));
+            emit<T>(g, gm, cs, sn, B, F, 2, k, {-v.a, v.b, v.c});
+        } else {
+            const T s = -(T)(gm.h * m.ax_perm_area) * ((T)m.ny * ld3(gm, Ey, 4, k).a);
+            emit<T>(g, gm, cs, sn, B, F, 3, k, {ld3(gm, B, 3, k).a + s, (T)0, (T)0});
+            emit(g, gm, cs, sn, B, F, 2, k, partner(v));
+        }
     }
-    emit(g, gm, cs, sn, Bx, Fx, i, k, bx);
-    if (i == 2) return;   // By and Bz of column 2: above
-    emit(g, gm, cs, sn, By, Fy, i, k, by);
-    emit(g, gm, cs, sn, Bz, Fz, i, k, bz);
+    if (i == 2 && comp != 0) return;   // By and Bz of column 2: above
+    emit(g, gm, cs, sn, B, F, i, k, v);
 }
 
 // Modes of the theta-gridded J at (i, k): a = mean, b = 2/ny sum J cos, c =
@@ -251,45 +261,54 @@ __global__ void __launch_bounds__(128) k_modal_e(GridP g, GridP gm, ModalP m, T 
     theta_table(m, tab, tab + m.ny);
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, k = 3 + blockIdx.y * blockDim.y + threadIdx.y;
     if (i > gm.mx || k > gm.mz - 3) return;
-    M3<T> ex = ld3(gm, Ex, i, k), ey = ld3(gm, Ey, i, k), ez = ld3(gm, Ez, i, k);
+    const int comp = blockIdx.z;
+    T *E = comp == 0 ? Ex : comp == 1 ? Ey : Ez, *F = comp == 0 ? Fx : comp == 1 ? Fy : Fz;
+    T *J = comp == 0 ? Jx : comp == 1 ? Jy : Jz;
+    M3<T> v = ld3(gm, E, i, k);
     if (i >= 4 && i <= gm.mx - 3) {
         const T dtheta = (T)m.dtheta;
         const T r = ((T)i - (T)3.0) + (T)m.rmin;
         const T rp_half = r + (T)0.5, rm_half = r - (T)0.5;
         if (MODE != 2) {
             const T fc = (T)gm.fc;
-            const M3<T> bz = ld3(gm, Bz, i, k), by = ld3(gm, By, i, k), bx = ld3(gm, Bx, i, k);
-            ex = ex + (fc * (bz - tm(m, bz))) / (rp_half * dtheta) - fc * (by - ld3(gm, By, i, k - 1));
-            ey = ey + fc * (bx - ld3(gm, Bx, i, k - 1)) - fc * (bz - ld3(gm, Bz, i - 1, k));
-            ez = ez + (fc * (rp_half * by - rm_half * ld3(gm, By, i - 1, k))) / r - (fc * (bx - tm(m, bx))) / (r * dtheta);
+            if (comp == 0) {
+                const M3<T> bz = ld3(gm, Bz, i, k), by = ld3(gm, By, i, k);
+                v = v + (fc * (bz - tm(m, bz))) / (rp_half * dtheta) - fc * (by - ld3(gm, By, i, k - 1));
+            } else if (comp == 1) {
+                const M3<T> bz = ld3(gm, Bz, i, k), bx = ld3(gm, Bx, i, k);
+                v = v + fc * (bx - ld3(gm, Bx, i, k - 1)) - fc * (bz - ld3(gm, Bz, i - 1, k));
+            } else {
+                const M3<T> by = ld3(gm, By, i, k), bx = ld3(gm, Bx, i, k);
+                v = v + (fc * (rp_half * by - rm_half * ld3(gm, By, i - 1, k))) / r - (fc * (bx - tm(m, bx))) / (r * dtheta);
+            }
         }
         if (MODE != 0) {
-            ex = ex - project<T, MODE == 1>(g, m, cs, sn, Jx, i, k) / (rp_half * dtheta);
-            ey = ey - project<T, MODE == 1>(g, m, cs, sn, Jy, i, k);
-            ez = ez - project<T, MODE == 1>(g, m, cs, sn, Jz, i, k) / (r * dtheta);
+            const M3<T> cur = project<T, MODE == 1>(g, m, cs, sn, J, i, k);
+            if (comp == 0) v = v - cur / (rp_half * dtheta);
+            else if (comp == 1) v = v - cur;
+            else v = v - cur / (r * dtheta);
         }
     }
     if (MODE == 1) {   // ResetCurrent
         const int kk = image_of(k, g.mz);
         for (int j = 1; j <= g.my; j++) {
-            const long long c = cidx(g, i, j, k);
-            Jx[c] = Jy[c] = Jz[c] = (T)0;
-            if (kk) {
-                const long long d = cidx(g, i, j, kk);
-                Jx[d] = Jy[d] = Jz[d] = (T)0;
-            }
+            J[cidx(g, i, j, k)] = (T)0;
+            if (kk) J[cidx(g, i, j, kk)] = (T)0;
         }
     }
     if (i == 3) return;   // column 3 belongs to the thread of column 4
     if (i == 4) {
-        emit(g, gm, cs, sn, Ex, Fx, 3, k, (T)0.5 * (ex - partner(ex)));
-        emit<T>(g, gm, cs, sn, Ex, Fx, 2, k, {-ex.a, ex.b, ex.c});
-        emit<T>(g, gm, cs, sn, Ey, Fy, 3, k, {-ey.a, ey.b, ey.c});
-        emit(g, gm, cs, sn, Ez, Fz, 3, k, partner(ez));
+        if (comp == 0) {
+            emit(g, gm, cs, sn, E, F, 3, k, (T)0.5 * (v - partner(v)));
+            emit<T>(g, gm, cs, sn, E, F, 2, k, {-v.a, v.b, v.c});
+        } else if (comp == 1) {
+            emit<T>(g, gm, cs, sn, E, F, 3, k, {-v.a, v.b, v.c});
+        } else {
+            emit(g, gm, cs, sn, E, F, 3, k, partner(v));
+        }
     }
-    if (i != 2) emit(g, gm, cs, sn, Ex, Fx, i, k, ex);   // Ex of column 2: above
-    emit(g, gm, cs, sn, Ey, Fy, i, k, ey);
-    emit(g, gm, cs, sn, Ez, Fz, i, k, ez);
+    if (i == 2 && comp == 0) return;   // Ex of column 2: above
+    emit(g, gm, cs, sn, E, F, i, k, v);
 }
 
 // Theta-gridded F(i, j, k) for every ghosted j from the modes at (i, k)
@@ -346,7 +365,7 @@ static ModalP modal_params(const GridP &g)
 static void modal_shape(const GridP &g, dim3 &grid, dim3 &block, size_t &smem)
 {
     block = dim3(32, 4);
-    grid = dim3((g.mx + 31) / 32, (g.nz + 3) / 4);
+    grid = dim3((g.mx + 31) / 32, (g.nz + 3) / 4, 3);
     smem = 2 * sizeof(double) * (size_t)g.ny;
 }
 template <typename K>
