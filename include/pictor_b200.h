@@ -63,7 +63,10 @@ typedef struct {
     double qi;                   /* charge unit from InitScale (initialise.F90:46)        */
     double bext[3];              /* Bx_ext0, By_ext0, Bz_ext0 (vars.F90:25)               */
     double qm[PIC_MAX_FLVR + 1]; /* flvrqm, index 1..nflvr (vars.F90:87)                  */
-    int32_t reorder_period;      /* prtl_reorder_period (parameters.F90:71); 0 = never    */
+    int32_t reorder_period;      /* prtl_reorder_period (parameters.F90:71); 0 = never.
+                                    In the FP32 Cartesian form pic_step and
+                                    pic_step_many also reorder in between, when
+                                    particles have spread too far from their bricks */
     int32_t curr_filter;         /* passes of the (1/4,1/2,1/4) filter (parameters.F90:22) */
     int64_t capacity;            /* particle slots on the device (gpu_prtl_arr_size)      */
     /* cylindrical (geom = PIC_GEOM_CYLINDRICAL): r of the first interior x cell
@@ -323,7 +326,8 @@ int pic_slab_pack_particles_fixed(pic_handle *h, double *to_left, double *to_rig
 int pic_slab_unpack_particles_fixed(pic_handle *h, const double *from_left, const double *from_right, int64_t cap);
 
 /* nsteps full steps of MAIN.F90:42-284 (reorder every reorder_period steps,
-   counted from the handle's step counter), captured once as a CUDA graph. */
+   counted from the handle's step counter, and see pic_config.reorder_period),
+   captured once as a CUDA graph. */
 int pic_step(pic_handle *h, int32_t nsteps);
 int pic_set_step(pic_handle *h, int64_t t);
 

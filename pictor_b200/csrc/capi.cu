@@ -138,6 +138,17 @@ int dalloc(pic_handle *h, T **p, size_t n)
     return PIC_OK;
 }
 
+// An array the handle does without when the device has no room for it (null).
+template <typename T>
+int dalloc_optional(pic_handle *h, T **p, size_t n)
+{
+    const int r = dalloc(h, p, n);
+    if (r != PIC_ERR_OOM) return r;
+    *p = nullptr;
+    cudaGetLastError();
+    return PIC_OK;
+}
+
 // Lehe coefficients, em_update_lehe.F90:8-25 (grid_dx = dy = dz = 1).
 void lehe_coefficients(int dims, double c, double *o)
 {
@@ -347,7 +358,7 @@ int enqueue_phase(pic_handle *h, int cur, bool reorder, int phase)
                 else launch_cyl_bhalf<float>(g, E, B, h->s);
                 break;
             case PIC_PHASE_MOVE:  // push, deposit and the wrap / outer-radius drop
-                if (h->sorted)
+                if (h->sorted && h->bricks.nodeA)
                     launch_cyl_move_deposit_f32_tiled(g, h->p32[cur], h->bricks, E, B, J, h->err, h->s);
                 else
                     launch_cyl_move_deposit_f32(g, h->p32[cur], h->cnt, E, B, J, h->err, h->s);
@@ -531,6 +542,10 @@ int note_reorder(pic_handle *h)
     h->group_len = std::max(h->group_len, h->since_group);
     h->since_group = 0;
     if (!h->over_host) return PIC_OK;
+    // a caller capturing pic_stream: the event could not be waited for
+    cudaStreamCaptureStatus cap;
+    CK(cudaStreamIsCapturing(h->s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return PIC_OK;
     CK(cudaEventRecord(h->ev_group, h->s));
     h->group_reported = true;
     return PIC_OK;
@@ -1171,8 +1186,8 @@ int pic_create(const pic_config *cfg, pic_handle **out)
         }
         // the node averages of the tiled movers, computed once per move
         // instead of by every brick for its box
-        if (!r && !(r = dalloc(h, (char **)&bk.nodeA, (size_t)g.ncell * sizeof(float4))))
-            r = dalloc(h, (char **)&bk.nodeB, (size_t)g.ncell * sizeof(float2));
+        if (!r && !(r = dalloc_optional(h, (char **)&bk.nodeB, (size_t)g.ncell * sizeof(float2))) && bk.nodeB)
+            r = dalloc_optional(h, (char **)&bk.nodeA, (size_t)g.ncell * sizeof(float4));
         // the boxes' report to step_reorders
         if (!r && g.geom == PIC_GEOM_CARTESIAN && !g.x_external) {
             h->over_host = reinterpret_cast<uint32_t *>(h->pin + kPinOver);
@@ -1214,7 +1229,10 @@ int pic_create(const pic_config *cfg, pic_handle **out)
             !(r = dalloc(h, &T.qmax, 1)))
             h->tiled64 = true;
         T.marks = reinterpret_cast<uint8_t *>(exchange_marks(h->sc));
-        if (!r && g.dims == 3) r = dalloc(h, &T.node, 6 * (size_t)g.ncell);
+        // without the node array the Cartesian tiles average their own nodes;
+        // the cylindrical ones need it
+        if (!r && g.dims == 3) r = dalloc_optional(h, &T.node, 6 * (size_t)g.ncell);
+        if (g.geom == PIC_GEOM_CYLINDRICAL && !T.node) h->tiled64 = false;
     }
     if (!r && c.exact_current) {
         SegRecords &R = h->rec;
@@ -1528,7 +1546,7 @@ int pic_move_deposit(pic_handle *h)
     if (h->g.geom == PIC_GEOM_CYLINDRICAL && h->fp32) {
         float *E[3], *B[3], *J[3];
         field_ptrs(h, E, B, J);
-        if (h->sorted)
+        if (h->sorted && h->bricks.nodeA)
             launch_cyl_move_deposit_f32_tiled(h->g, h->p32[h->cur], h->bricks, E, B, J, h->err, h->s);
         else
             launch_cyl_move_deposit_f32(h->g, h->p32[h->cur], h->cnt, E, B, J, h->err, h->s);
