@@ -210,13 +210,14 @@ __device__ __forceinline__ T fold_yz(const GridP &g, const T *J, int i, int j, i
 // UpdateEfield (cyl_em_update.F90:24-41, MODE 0), AddCurrent of a folded J
 // (:128-137, MODE 2), or both with the fold of J and its zeroing (MODE 1, the
 // step): i 4..mx-3 on the rank holding the axis, 3..mx-3 elsewhere.
-// One component per thread (blockIdx.z: plane x component), as k_cyl_bhalf.
+// One component per thread, as k_cyl_bhalf (blockIdx.y: block of theta x
+// component; z planes have blockIdx.z to themselves, whose limit is 65535).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) k_cyl_e(GridP g, CylP cp, T *Ex, T *Ey, T *Ez, const T *__restrict__ Bx,
                                                const T *__restrict__ By, const T *__restrict__ Bz, T *Jx, T *Jy, T *Jz)
 {
-    const int comp = blockIdx.z % 3;
-    const int i = 1 + blockIdx.x * 32 + threadIdx.x, j = 3 + blockIdx.y * 8 + threadIdx.y, k = 3 + blockIdx.z / 3;
+    const int comp = blockIdx.y % 3;
+    const int i = 1 + blockIdx.x * 32 + threadIdx.x, j = 3 + (blockIdx.y / 3) * 8 + threadIdx.y, k = 3 + blockIdx.z;
     if (i > g.mx || j > g.my - 3) return;
     T *E = comp == 0 ? Ex : comp == 1 ? Ey : Ez, *J = comp == 0 ? Jx : comp == 1 ? Jy : Jz;
     const long long c0 = cidx(g, i, j, k);
@@ -308,7 +309,7 @@ template <typename T>
 void launch_cyl_efield(const GridP &g, int mode, T *const E[3], T *const B[3], T *const J[3], cudaStream_t s)
 {
     const CylP cp = cyl_params(g);
-    const dim3 grid((g.mx + 31) / 32, (g.ny + 7) / 8, 3 * g.nz), block(32, 8, 1);
+    const dim3 grid((g.mx + 31) / 32, 3 * ((g.ny + 7) / 8), g.nz), block(32, 8, 1);
 #define LE(M) k_cyl_e<T, M><<<grid, block, 0, s>>>(g, cp, E[0], E[1], E[2], B[0], B[1], B[2], J[0], J[1], J[2])
     if (mode == 0) LE(0);
     else if (mode == 1) LE(1);
