@@ -478,21 +478,31 @@ int enqueue_step(pic_handle *h, int cur, bool reorder)
     return n;
 }
 
+// A graph of the launches enqueue() makes on s.  A launch that a capture
+// refuses (an invalid configuration) leaves the rest of the graph valid, so
+// the graph is kept only when every launch of it was accepted.
+template <typename F>
+int capture_graph(cudaStream_t s, F enqueue, cudaGraphExec_t *out)
+{
+    *out = nullptr;
+    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    enqueue();
+    const cudaError_t launch = cudaGetLastError();
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamEndCapture(s, &graph);
+    if (launch != cudaSuccess) e = launch;
+    if (e == cudaSuccess && (e = cudaGraphInstantiate(out, graph, 0)) != cudaSuccess) *out = nullptr;
+    if (graph) cudaGraphDestroy(graph);
+    return e == cudaSuccess ? PIC_OK : cuda_status(e);
+}
+
 int get_graph(pic_handle *h, int cur, bool reorder, cudaGraphExec_t *out)
 {
     cudaGraphExec_t &ge = h->graph[reorder ? 1 : 0][cur];
     if (!ge) {
-        cudaGraph_t graph = nullptr;
-        CK(cudaStreamBeginCapture(h->s, cudaStreamCaptureModeThreadLocal));
-        h->graph_kernels[reorder ? 1 : 0][cur] = enqueue_step(h, cur, reorder);
-        cudaError_t e = cudaStreamEndCapture(h->s, &graph);
-        if (e != cudaSuccess) return cuda_status(e);
-        e = cudaGraphInstantiate(&ge, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) {
-            ge = nullptr;
-            return cuda_status(e);
-        }
+        const int r = capture_graph(
+            h->s, [&] { h->graph_kernels[reorder ? 1 : 0][cur] = enqueue_step(h, cur, reorder); }, &ge);
+        if (r) return r;
     }
     *out = ge;
     return PIC_OK;
@@ -939,21 +949,13 @@ static int batch_group_prepare(BatchGroup &G, bool fresh)
     // one step of every run: B half, move + deposit, B half, E + fold + AddCurrent
     const int dims = h0->g.dims, fdtd = h0->g.fdtd;
     g_launches = 0;
-    cudaGraph_t gr = nullptr;
-    CK(cudaStreamBeginCapture(G.s, cudaStreamCaptureModeThreadLocal));
-    launch_batch_bhalf(dims, fdtd, G.druns, G.dstart, n, G.nf, G.s);
-    launch_batch_move(dims, h0->g.exact_charge != 0, G.druns, G.dstart + n + 1, n, G.nm, G.s);
-    launch_batch_bhalf(dims, fdtd, G.druns, G.dstart, n, G.nf, G.s);
-    launch_batch_efield(dims, G.druns, G.dstart, n, G.nf, G.s);
-    G.step_kernels = g_launches;
-    const cudaError_t e = cudaStreamEndCapture(G.s, &gr);
-    const cudaError_t ei = e == cudaSuccess ? cudaGraphInstantiate(&G.ge, gr, 0) : e;
-    if (gr) cudaGraphDestroy(gr);
-    if (ei != cudaSuccess) {
-        G.ge = nullptr;
-        return cuda_status(ei);
-    }
-    return PIC_OK;
+    return capture_graph(G.s, [&] {
+        launch_batch_bhalf(dims, fdtd, G.druns, G.dstart, n, G.nf, G.s);
+        launch_batch_move(dims, h0->g.exact_charge != 0, G.druns, G.dstart + n + 1, n, G.nm, G.s);
+        launch_batch_bhalf(dims, fdtd, G.druns, G.dstart, n, G.nf, G.s);
+        launch_batch_efield(dims, G.druns, G.dstart, n, G.nf, G.s);
+        G.step_kernels = g_launches;
+    }, &G.ge);
 }
 
 static int step_many_batched(pic_handle *const *hs, int32_t n, int32_t nsteps)
@@ -2165,13 +2167,8 @@ static int step_persistent(pic_handle *const *hs, int32_t n, int32_t nsteps, uns
         return launches;
     };
     if (!ge) {
-        cudaGraph_t gr = nullptr;
-        CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        launches = enqueue();
-        const cudaError_t e = cudaStreamEndCapture(s, &gr);
-        const cudaError_t ei = e == cudaSuccess ? cudaGraphInstantiate(&ge, gr, 0) : e;
-        if (gr) cudaGraphDestroy(gr);
-        if (ei != cudaSuccess) return cuda_status(ei);
+        const int r = capture_graph(s, [&] { launches = enqueue(); }, &ge);
+        if (r) return r;
         P.graphs.push_back({key, ge, launches});
     } else {
         // the host-side counters advance as the captured sequence does

@@ -1,5 +1,6 @@
 """Cylinders of many z cells: every launch of the field phases within the grid
-limits for as many planes as the smallest of them allows (65530)."""
+limits for as many planes as the smallest of them allows (65530), and an error
+on every step beyond it."""
 import numpy as np
 import pytest
 
@@ -56,3 +57,18 @@ def test_long_cylinder_repeats_the_short_one(nz, reps, modes, precision):
             s.fold_current()
             s.add_current()
         same()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_a_step_that_cannot_be_launched_fails_every_time(precision):
+    """One z plane more than a launch can index: the step's graph is refused,
+    not kept without that launch, so the second call fails as the first does;
+    a run of another size on the same device is not disturbed."""
+    from pictor_b200._capi import PicError
+
+    with _sim(66000, precision, 0) as s, _sim(12, precision, 0) as t:
+        for _ in range(3):
+            with pytest.raises(PicError, match="CUDA"):
+                s.step(1)
+        t.step(1)
+        assert t.device_errors() == 0
