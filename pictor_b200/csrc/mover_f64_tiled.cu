@@ -13,6 +13,8 @@
 // particle that leaves the interior is wrapped by the exchange and appended
 // after the sorted range; those are moved one per thread by blocks of the
 // same launch.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "particle_math.cuh"
@@ -259,22 +261,26 @@ __global__ void __launch_bounds__(256) k_node_f64(GridP g, const double *__restr
                                                   const double *__restrict__ By, const double *__restrict__ Bz,
                                                   double *node)
 {
-    const int i = 2 + blockIdx.x * 32 + threadIdx.x, j = 2 + blockIdx.y * 8 + threadIdx.y, k = 2 + blockIdx.z;
-    if (i > g.mx - 1 || j > g.my - 1 || k > g.mz - 1) return;
-    const long long nd = cidx(g, i, j, k);
-    double v[6];
-    node_values64<3>(g, Ex, Ey, Ez, Bx, By, Bz, nd, v);
-    double2 *o = reinterpret_cast<double2 *>(node + 6 * nd);
-    o[0] = make_double2(v[0], v[1]);
-    o[1] = make_double2(v[2], v[3]);
-    o[2] = make_double2(v[4], v[5]);
+    const int i = 2 + blockIdx.x * 32 + threadIdx.x, j = 2 + blockIdx.y * 8 + threadIdx.y;
+    if (i > g.mx - 1 || j > g.my - 1) return;
+    for (int k = 2 + blockIdx.z; k <= g.mz - 1; k += gridDim.z) {
+        const long long nd = cidx(g, i, j, k);
+        double v[6];
+        node_values64<3>(g, Ex, Ey, Ez, Bx, By, Bz, nd, v);
+        double2 *o = reinterpret_cast<double2 *>(node + 6 * nd);
+        o[0] = make_double2(v[0], v[1]);
+        o[1] = make_double2(v[2], v[3]);
+        o[2] = make_double2(v[4], v[5]);
+    }
 }
 
 }  // namespace
 
 void launch_node_f64(const GridP &g, const Tiles64 &T, double *const E[3], double *const B[3], cudaStream_t s)
 {
-    const dim3 block(32, 8, 1), grid((g.mx - 2 + 31) / 32, (g.my - 2 + 7) / 8, g.mz - 2);
+    // one plane of nodes per block; there are 3 more of them than z cells, so
+    // at the most cells the field phases launch (65535) the blocks take two
+    const dim3 block(32, 8, 1), grid((g.mx - 2 + 31) / 32, (g.my - 2 + 7) / 8, std::min(g.mz - 2, 65535));
     k_node_f64<<<grid, block, 0, s>>>(g, E[0], E[1], E[2], B[0], B[1], B[2], T.node);
     count_launches(1);
 }

@@ -53,3 +53,23 @@ def test_tiled_steps_keep_the_slots_of_the_per_particle_form(shape, dims, ppc, s
         fa, fb = a.fetch_fields(), b.fetch_fields()
         for k in ("Ex", "Ey", "Ez"):
             assert np.abs(getattr(fa, k) - getattr(fb, k)).max() <= 1e-12 * np.abs(getattr(fb, k)).max(), k
+
+
+def test_tiles_on_the_longest_grid():
+    """65535 z cells, the most the field phases launch: a sparse run stepped
+    after a reorder by either form, bit for bit (particles), ends included."""
+    shape = (5, 5, 65535)
+    a, b = _sims(shape, 3, 1, 1 << 14)
+    p = _hot(5, 5, 40, 3, 2, 3)
+    p.z[:] = 3.0 + (p.z - 3.0) / 40 * 65535
+    p.z[:200] = 3.0 + np.linspace(0, 2, 200)
+    p.z[200:400] = 65538.0 - np.linspace(1e-3, 2, 200)
+    with a, b:
+        for s in (a, b):
+            s.load_particles(p)
+            s.reorder()
+            s.step(1)
+        pa, pb = a.fetch_particles(), b.fetch_particles()
+        for k in pa.NAMES:
+            assert np.array_equal(getattr(pa, k), getattr(pb, k)), k
+        assert a.device_errors() == 0 and len(pa) > len(p)   # some crossed the z ends
