@@ -764,6 +764,21 @@ int fetch_array_f32(pic_handle *h, const float *src, double *dst, long long n, i
     return PIC_OK;
 }
 
+// The host array of n values at p begins and ends in memory that is not
+// registered with the CUDA runtime.
+bool pageable(const double *p, size_t n)
+{
+    for (const double *q : {p, p + n - 1}) {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, q) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeUnregistered) return false;
+    }
+    return true;
+}
+
 // The configured filter passes over J, the result left in J.
 template <typename T>
 void filter_current(pic_handle *h)
@@ -1368,14 +1383,17 @@ int pic_fetch_fields(pic_handle *h, double *Ex, double *Ey, double *Ez, double *
         }
     if ((size_t)m * n <= (size_t)stage_field_chunk(h)) {
         // small grids: one conversion of all arrays into one staging buffer,
-        // copied from on the same stream, host arrays that follow one another
-        // in one copy (64^2 cells: 88 us as a conversion, a copy and four
-        // stream events per array, 45 us now)
+        // copied from on the same stream, pageable host arrays that follow
+        // one another in one copy (64^2 cells: 88 us as a conversion, a copy
+        // and four stream events per array, 45 us now).  A copy that leaves
+        // one registered range for another, or for pageable memory, is
+        // refused, so arrays in registered memory keep a copy each.
         double *t = (double *)h->stage[0];
         if (m) launch_arrays_f32_to_f64((const float *const *)src, m, t, (long long)n, h->s);
         for (int k = 0; k < m;) {
             int e = k + 1;
-            while (e < m && dst[e] == dst[e - 1] + n) e++;
+            if (e < m && dst[e] == dst[e - 1] + n && pageable(dst[k], n))
+                while (e < m && dst[e] == dst[e - 1] + n && pageable(dst[e], n)) e++;
             CK(cudaMemcpyAsync(dst[k], t + (size_t)k * n, (size_t)(e - k) * n * sizeof(double), cudaMemcpyDeviceToHost, h->s));
             k = e;
         }

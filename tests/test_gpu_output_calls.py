@@ -86,3 +86,36 @@ def test_fetched_fields(nx, ny, layout):
                 assert (buf[:, n:] == 7.0).all()
             if not with_j and out is not None:
                 assert (buf[6:] == 7.0).all()
+
+
+@pytest.mark.parametrize("registered", [(0, 4), (3, 6), (5, 9), (0, 9), (2, 2)])
+def test_fetched_fields_into_partly_registered_memory(registered):
+    """Nine host arrays one after the other, of which some lie in memory that
+    is registered with CUDA (page-aligned: 64 x 64 float64 is 8 pages)."""
+    import mmap
+
+    import torch
+
+    from pictor_b200 import PicConfig, Simulation
+
+    cfg = PicConfig(nx=59, ny=59, dims=2, c=0.45, qi=0.01, precision="fp32", capacity=4096)
+    n = 64 * 64
+    rng = np.random.default_rng(4)
+    f = Fields(*(np.asfortranarray(rng.normal(size=cfg.shape)) for _ in range(9)))
+    buf = np.frombuffer(mmap.mmap(-1, 9 * n * 8), dtype=np.float64).reshape(9, n)
+    buf[:] = 7.0
+    out = Fields(*(buf[k].reshape(cfg.shape, order="F") for k in range(9)))
+    first, last = registered
+    rt = torch.cuda.cudart()
+    with Simulation(cfg) as s:
+        s.load_fields(f)
+        s.load_current(f.Jx, f.Jy, f.Jz)
+        if last > first:
+            assert int(rt.cudaHostRegister(buf[first].ctypes.data, (last - first) * n * 8, 0)) == 0
+        try:
+            s.fetch_fields(out=out)
+        finally:
+            if last > first:
+                rt.cudaHostUnregister(buf[first].ctypes.data)
+    for k in Fields.__dataclass_fields__:
+        assert np.array_equal(getattr(out, k), getattr(f, k).astype(np.float32).astype(np.float64)), k
