@@ -8,7 +8,6 @@
 // the backward-difference node divergence of CalcDivE.
 #include "common.cuh"
 #include "kernels.cuh"
-#include "tile64.cuh"
 
 namespace pic {
 
@@ -255,17 +254,18 @@ __global__ void k_rho_f32(GridP g, PartF32 p, const Counters *__restrict__ cnt, 
 }
 
 // The same after a reorder, one CTA per brick (bricks.cu): the brick's charge
-// is summed in shared memory over the nodes of its box as 64-bit fixed-point
-// words (the scale of tile64.cuh: a unit is at most 2^-50 of the largest
-// charge, below the FP64 rounding of the sums), each added as two 32-bit
-// atomics, and the box is added to the grid once.  A particle outside the box
-// adds to the grid.  537 M particles 6.7 ms, and with the energies below the
-// diagnostics 11.9 ms (23.8 ms with 12 FP64 atomics into L2 per particle).
+// is summed in shared memory over the nodes of its box, and the box is added to
+// the grid once.  A particle outside the box adds to the grid.  The sums are
+// FP64 in any order, as in the grid: 64-bit fixed-point words would be faster
+// (diagnostics of 268 M particles 6.0 ms), but hold fewer bits of light
+// particles, and of any where a brick has over 4096, than FP64 does; with a
+// 32-bit extension of those words 7.3 ms, so 8.4 ms as FP64 atomics of shared
+// memory (11.3 ms into L2; 16.8 M particles in 2D 445 and 481 us).
 constexpr int kRhoNodes = 3072;   // 48 KB, 4 CTAs per SM
 template <int DIMS>
 __global__ void __launch_bounds__(256) k_rho_f32_bricks(GridP g, PartF32 p, Bricks bk, double *rho_neg, double *rho_pos)
 {
-    extern __shared__ unsigned long long s_rho[];   // positive, then negative charge
+    extern __shared__ double s_rho[];   // positive, then negative charge
     const int b = blockIdx.x;
     const uint32_t p0 = bk.tile_start[b], p1 = bk.tile_start[b + 1];
     if (p0 >= p1) return;
@@ -281,10 +281,7 @@ __global__ void __launch_bounds__(256) k_rho_f32_bricks(GridP g, PartF32 p, Bric
     const bool fits = N[0] > 1 && N[1] > 1 && (DIMS == 2 || N[2] > 1) && N[0] <= kBoxAxisMax && N[1] <= kBoxAxisMax &&
                       N[2] <= kBoxAxisMax && N[0] * N[1] * N[2] <= kRhoNodes;
     const int nn = fits ? N[0] * N[1] * N[2] : 0;
-    for (int q = threadIdx.x; q < 2 * nn; q += 256) s_rho[q] = 0ull;
-    const double qmax = (double)__uint_as_float(*bk.wmax_bits) * g.qi;
-    const uint32_t np = p1 - p0;
-    const double S = qmax > 0.0 ? 1125899906842624.0 / qmax * (np > 4096u ? 4096.0 / (double)np : 1.0) : 1.0;
+    for (int q = threadIdx.x; q < 2 * nn; q += 256) s_rho[q] = 0.0;
     __syncthreads();
     for (uint32_t t = p0 + threadIdx.x; t < p1; t += 256) {
         const uint32_t key = p.key[t];
@@ -309,18 +306,16 @@ __global__ void __launch_bounds__(256) k_rho_f32_bricks(GridP g, PartF32 p, Bric
         }
         double w[8];
         corner_weights(DIMS, dx, dy, dz, w);
-        unsigned long long *at = s_rho + (q > 0 ? 0 : nn) + lx + N[0] * (ly + N[1] * lz);
-        const double qS = q * S;
+        double *at = s_rho + (q > 0 ? 0 : nn) + lx + N[0] * (ly + N[1] * lz);
 #pragma unroll
         for (int c = 0; c < (DIMS == 3 ? 8 : 4); c++)
-            add_fixed64(at + (c & 1) + ((c >> 1) & 1) * N[0] + ((c >> 2) & 1) * N[0] * N[1], fixed64(qS * w[c]));
+            atomicAdd(at + (c & 1) + ((c >> 1) & 1) * N[0] + ((c >> 2) & 1) * N[0] * N[1], q * w[c]);
     }
     __syncthreads();
-    const double inv = 1.0 / S;
     const uint32_t mX = 0xffffffffu / (uint32_t)N[0] + 1u, mY = 0xffffffffu / (uint32_t)N[1] + 1u;
     for (int q = threadIdx.x; q < nn; q += 256) {
-        const long long vp = (long long)s_rho[q], vn = (long long)s_rho[nn + q];
-        if (vp == 0 && vn == 0) continue;
+        const double vp = s_rho[q], vn = s_rho[nn + q];
+        if (vp == 0.0 && vn == 0.0) continue;
         const int r = (int)__umulhi((uint32_t)q, mX), xx = q - r * N[0];
         const int zz = (int)__umulhi((uint32_t)r, mY), yy = r - zz * N[1];
         const int c[3] = {hc[0] + lo[0] + xx, hc[1] + lo[1] + yy, DIMS == 3 ? hc[2] + lo[2] + zz : 1};
@@ -337,8 +332,8 @@ __global__ void __launch_bounds__(256) k_rho_f32_bricks(GridP g, PartF32 p, Bric
             }
         }
         const long long o = cidx(g, cc[0], cc[1], cc[2]);
-        if (vp != 0) atomicAdd(rho_pos + o, (double)vp * inv);
-        if (vn != 0) atomicAdd(rho_neg + o, (double)vn * inv);
+        if (vp != 0.0) atomicAdd(rho_pos + o, vp);
+        if (vn != 0.0) atomicAdd(rho_neg + o, vn);
     }
 }
 
@@ -400,7 +395,7 @@ static void deposit_f32(const GridP &g, const PartF32 &p, const Counters *cnt, c
                         double *rho_pos, cudaStream_t s)
 {
     zero_rho(g, rho, rho_pos, s);
-    const size_t sm = 2 * kRhoNodes * sizeof(unsigned long long);
+    const size_t sm = 2 * kRhoNodes * sizeof(double);
     if (bk && g.dims == 3) k_rho_f32_bricks<3><<<bk->ntiles, 256, sm, s>>>(g, p, *bk, rho, rho_pos);
     else if (bk) k_rho_f32_bricks<2><<<bk->ntiles, 256, sm, s>>>(g, p, *bk, rho, rho_pos);
     else k_rho_f32<<<kSMs * 8, 256, 0, s>>>(g, p, cnt, rho, rho_pos);

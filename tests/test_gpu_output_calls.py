@@ -39,6 +39,38 @@ def test_density_by_bricks(shape, dims, ppc, steps):
     assert np.allclose(da["kinetic"], db["kinetic"], rtol=1e-12)
 
 
+@pytest.mark.parametrize("qi", [0.01, -0.01])
+def test_density_by_bricks_keeps_light_particles(qi):
+    """Eight particles 2^-47 as heavy as the others, on nodes of their own, in
+    a brick of 16384, with either sign of the charge unit.  The others lie in
+    pairs of opposite charge at quarters of a cell, so their sums are exact
+    and cancel: the Gauss residual is the density of the heaviest light one,
+    the same reordered and not (one product per node), and FP32's positions
+    give it to 1e-6."""
+    from pictor_b200 import PicConfig, Simulation
+
+    n, light = 32, 2.0 ** -47
+    cfg = PicConfig(nx=n, ny=n, dims=2, c=0.45, qi=qi, precision="fp32", capacity=1 << 15, brick=(32, 32, 1))
+    p = _hot(n, n, 1, 2, 8, 4)
+    m = len(p)
+    rng = np.random.default_rng(4)
+    p.x[:], p.y[:] = 3.0 + rng.integers(0, 4 * n, m) / 4, 3.0 + rng.integers(0, 2 * n, m) / 4
+    for k in ("x", "y"):
+        getattr(p, k)[9::2] = getattr(p, k)[8:-1:2]
+    p.q[8::2], p.q[9::2] = 1.0, -1.0
+    p.x[:8], p.y[:8] = 3.3 + np.arange(8) * 4, 3.7 + 0.75 * n
+    p.q[:8] = light * np.arange(3, 11)
+    p.u[:], p.v[:], p.w[:] = 0.0, 0.0, 0.0
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        for s in (a, b):
+            s.load_particles(p)
+        a.reorder()
+        da, db = a.diagnostics(1.0), b.diagnostics(1.0)
+    assert da["rho_max"] == pytest.approx(db["rho_max"], rel=1e-12) and db["rho_max"] > 0
+    assert da["gauss_linf"] == pytest.approx(db["gauss_linf"], rel=1e-12)
+    assert db["gauss_linf"] == pytest.approx(10 * light * abs(qi) * 0.7 * 0.7, rel=1e-6)
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_kinetic_energy_of_every_flavour(precision):
     from pictor_b200 import PicConfig, Simulation
