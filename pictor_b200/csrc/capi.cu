@@ -576,6 +576,18 @@ int note_reorder(pic_handle *h)
     return PIC_OK;
 }
 
+// Finish a call that loaded particles: as finish; what pic_step learned from
+// the particles that were there before is dropped with them.
+int finish_load(pic_handle *h)
+{
+    if (h->over_host) CK(cudaMemsetAsync(h->bricks.over, 0, kOverWords * sizeof(uint32_t), h->s));
+    const int r = finish(h);
+    h->group_every = h->since_group = h->group_len = h->group_clean = 0;
+    h->group_reported = false;
+    if (h->over_host) *h->over_host = 0;   // no reorder is in flight now
+    return r;
+}
+
 // pic_step with an event pair around every phase of every step (no graphs).
 int step_profiled(pic_handle *h, int32_t nsteps)
 {
@@ -1466,7 +1478,7 @@ int pic_load_particles(pic_handle *h, int64_t n, const double *q, const double *
     c0.np = n;
     CK(cudaMemcpyAsync(h->cnt, &c0, sizeof(Counters), cudaMemcpyHostToDevice, h->s));
     set_sorted(h, false);
-    return finish(h);
+    return finish_load(h);
 }
 
 int pic_fetch_particles(pic_handle *h, int64_t *nout, double *q, double *x, double *y, double *z, double *u, double *v,
@@ -1536,7 +1548,7 @@ int pic_init_weibel(pic_handle *h, double epc, double density, double drift, dou
     set_sorted(h, false);
     int r = launch_weibel(h->g, w, h->tab_x, h->tab_p, h->ntab, p64, p32, h->cnt, h->sc, h->capacity, h->err, h->s);
     if (r) return r;
-    return finish(h);
+    return finish_load(h);
 }
 
 // --- phases --------------------------------------------------------------

@@ -96,3 +96,33 @@ def test_pic_step_reorders_before_the_boxes_are_outgrown():
     for k in ("B2", "E2"):
         assert abs(d32[k] - d64[k]) <= 1e-4 * d64[k]
     assert np.allclose(d32["kinetic"], d64["kinetic"], rtol=1e-4)
+
+
+@pytest.mark.parametrize("how", ["load_particles", "init_weibel"])
+def test_a_reloaded_run_reorders_as_a_new_one(how):
+    """The interval learned from a hot plasma is not applied to the cold one
+    loaded after it: the same number of reorders as in a run of its own."""
+    from pictor_b200 import Simulation
+
+    shape, ppc = (48, 32, 32), 8
+    cfg, sc = _cfg(shape, 3, ppc, 20)
+
+    def load_cold(s):
+        if how == "init_weibel":
+            s.init_weibel(ppc, 0.5, 0.0, 1e-6, 1e-6)
+        else:
+            s.load_particles(_hot(*shape, 3, ppc, 8, 0.01))
+        s.set_step(0)
+        s.reorder()
+        s.phase_times()
+        s.step(45)
+        return s.phase_times()["launches"]["reorder"]
+
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        for s in (a, b):
+            s.profile(True)
+        a.load_particles(_hot(*shape, 3, ppc, 7))
+        a.reorder()
+        a.step(30)      # learns a short interval, and leaves a report unread
+        a.reorder()
+        assert load_cold(a) == load_cold(b)
