@@ -89,6 +89,9 @@ struct pic_handle {
     uint32_t *over_host = nullptr;   // in pin
     cudaEvent_t ev_group = nullptr;
     bool group_reported = false;
+    // moves that Bricks::over does not count happened since the last reorder
+    // (batched and persistent steps)
+    bool moves_uncounted = false;
     // slab form: device counts of the particles sent through the x faces
     uint32_t *slab_sent = nullptr;
     // phase entry points wait for their work (pic_set_sync)
@@ -529,6 +532,11 @@ int step_reorders(pic_handle *h, bool *reorder)
 {
     const int period = h->cfg.reorder_period;
     *reorder = period > 0 && (h->t % period) == 0;
+    if (h->moves_uncounted && h->over_host) {   // the device's count joins the host's
+        const uint32_t moves = (uint32_t)h->since_group;
+        CK(cudaMemcpyAsync(h->bricks.over, &moves, sizeof(moves), cudaMemcpyHostToDevice, h->s));
+        h->moves_uncounted = false;
+    }
     h->since_group++;
     if (*reorder || !h->over_host || !h->sorted || period <= kGroupMin || h->since_group < kGroupMin) return PIC_OK;
     if (h->group_reported) {
@@ -563,6 +571,7 @@ int note_reorder(pic_handle *h)
 {
     h->group_len = std::max(h->group_len, h->since_group);
     h->since_group = 0;
+    h->moves_uncounted = false;
     if (!h->over_host) return PIC_OK;
     // a caller capturing pic_stream: the event could not be waited for
     cudaStreamCaptureStatus cap;
@@ -583,7 +592,7 @@ int finish_load(pic_handle *h)
     if (h->over_host) CK(cudaMemsetAsync(h->bricks.over, 0, kOverWords * sizeof(uint32_t), h->s));
     const int r = finish(h);
     h->group_every = h->since_group = h->group_len = h->group_clean = 0;
-    h->group_reported = false;
+    h->group_reported = h->moves_uncounted = false;
     if (h->over_host) *h->over_host = 0;   // no reorder is in flight now
     return r;
 }
@@ -938,6 +947,7 @@ static BatchRun batch_run_of(pic_handle *h)
     R.p[0] = h->p32[0];
     R.p[1] = h->p32[1];
     R.bk = h->bricks;
+    R.bk.over = nullptr;   // no node pass numbers these moves
     for (int k = 0; k < 3; k++) {
         R.E[k] = (float *)h->E[k];
         R.B[k] = (float *)h->B[k];
@@ -1031,7 +1041,11 @@ static int step_many_batched(pic_handle *const *hs, int32_t n, int32_t nsteps)
             for (size_t a = 0; a < G.runs.size(); a++) {
                 pic_handle *h = G.runs[a];
                 h->t += 1;
+                h->since_group++;
+                h->moves_uncounted = true;
                 if (h->cfg.reorder_period > 0 && (h->t % h->cfg.reorder_period) == 0) {
+                    h->since_group = 0;
+                    h->moves_uncounted = false;
                     g_launches = 0;
                     launch_reorder_f32(h->g, h->p32[h->cur], h->p32[h->cur ^ 1], h->cnt, h->capacity, h->bricks,
                                        h->err, G.s);
@@ -2166,10 +2180,11 @@ static int step_persistent(pic_handle *const *hs, int32_t n, int32_t nsteps, uns
         }
     // the host-side step counters and buffers advance as the sequence does
     std::vector<long long> t((size_t)n);
-    std::vector<int> cur((size_t)n);
+    std::vector<int> cur((size_t)n), since((size_t)n);   // since: moves after the last reorder
     for (int32_t a = 0; a < n; a++) {
         t[(size_t)a] = hs[a]->t;
         cur[(size_t)a] = hs[a]->cur;
+        since[(size_t)a] = hs[a]->since_group;
     }
     auto enqueue = [&]() {
         long long launches = 0;
@@ -2188,7 +2203,9 @@ static int step_persistent(pic_handle *const *hs, int32_t n, int32_t nsteps, uns
             for (int32_t a = 0; a < n; a++) {
                 pic_handle *h = hs[a];
                 t[(size_t)a] += span;
+                since[(size_t)a] += span;
                 if (h->cfg.reorder_period > 0 && t[(size_t)a] % h->cfg.reorder_period == 0) {
+                    since[(size_t)a] = 0;
                     g_launches = 0;
                     const int c = cur[(size_t)a];
                     launch_reorder_f32(h->g, h->p32[c], h->p32[c ^ 1], h->cnt, h->capacity, h->bricks, h->err, s);
@@ -2215,8 +2232,12 @@ static int step_persistent(pic_handle *const *hs, int32_t n, int32_t nsteps, uns
             }
             for (int32_t a = 0; a < n; a++) {
                 t[(size_t)a] += span;
+                since[(size_t)a] += span;
                 const int per = hs[a]->cfg.reorder_period;
-                if (per > 0 && t[(size_t)a] % per == 0) cur[(size_t)a] ^= 1;
+                if (per > 0 && t[(size_t)a] % per == 0) {
+                    since[(size_t)a] = 0;
+                    cur[(size_t)a] ^= 1;
+                }
             }
             done += span;
         }
@@ -2225,6 +2246,8 @@ static int step_persistent(pic_handle *const *hs, int32_t n, int32_t nsteps, uns
     for (int32_t a = 0; a < n; a++) {
         hs[a]->t = t[(size_t)a];
         hs[a]->cur = cur[(size_t)a];
+        hs[a]->since_group = since[(size_t)a];
+        hs[a]->moves_uncounted = since[(size_t)a] > 0;
     }
     h0->launches += launches;
     unsigned status = 0;

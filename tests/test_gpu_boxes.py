@@ -126,3 +126,33 @@ def test_a_reloaded_run_reorders_as_a_new_one(how):
         a.step(30)      # learns a short interval, and leaves a report unread
         a.reorder()
         assert load_cold(a) == load_cold(b)
+
+
+@pytest.mark.parametrize("form", [{"per_phase": True}, {"persistent": True}])
+def test_batched_steps_leave_the_learned_interval_alone(form):
+    """A warm run stepped by pic_step, then for two periods and a half by the
+    batched or persistent form, then by pic_step again, reorders in the last
+    part as often as a run that pic_step stepped throughout (one more or less:
+    the phase in which it starts)."""
+    from pictor_b200 import Simulation, step_many
+
+    shape, ppc = (48, 32, 32), 8
+    cfg, _ = _cfg(shape, 3, ppc, 20)
+    counts = []
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        for s, batched in ((a, False), (b, True)):
+            s.load_particles(_hot(*shape, 3, ppc, 7, 0.15))
+            s.reorder()
+            s.step(25)
+            if batched:
+                step_many([s], 50, **form)
+            else:
+                s.step(50)
+            s.profile(True)
+            s.phase_times()
+            s.step(60)
+            counts.append(s.phase_times()["launches"]["reorder"])
+            s.profile(False)
+    per = 6   # launches of a reorder
+    assert abs(counts[0] - counts[1]) <= per, counts
+    assert min(counts) >= 3 * per
