@@ -103,11 +103,14 @@ struct pic_handle {
     bool tiled64 = false;
     Tiles64 t64 = {};
     std::vector<void *> allocs;
+    // pointers of this handle to arrays it can do without (add_optional)
+    std::vector<void **> optional;
 };
 
 static thread_local long long g_launches = 0;
 static void batch_forget(pic_handle *h);
 static void persist_forget(pic_handle *h);
+static bool release_optional(pic_handle *h);
 
 namespace pic {
 void count_launches(int n) { g_launches += n; }
@@ -135,21 +138,45 @@ int dalloc(pic_handle *h, T **p, size_t n)
     void *q = nullptr;
     if (n == 0) n = 1;
     cudaError_t e = cudaMalloc(&q, n * sizeof(T));
-    if (e != cudaSuccess) return cuda_status(e);
+    if (e == cudaErrorMemoryAllocation && release_optional(h)) {
+        cudaGetLastError();
+        e = cudaMalloc(&q, n * sizeof(T));
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // not left for the next call
+        return cuda_status(e);
+    }
     h->allocs.push_back(q);
     *p = (T *)q;
     return PIC_OK;
 }
 
-// An array the handle does without when the device has no room for it (null).
+// An array the handle can do without (null then): taken only when three times
+// its size stays free on the device after it, for the handle's later
+// allocations and for whatever else the program keeps there, and given back
+// when an allocation of the handle fails.  Below kOptionalSmall bytes it is
+// taken without asking how much is free (0.1 ms, much of a small run's
+// creation).
+constexpr size_t kOptionalSmall = 8 << 20;
 template <typename T>
-int dalloc_optional(pic_handle *h, T **p, size_t n)
+void add_optional(pic_handle *h, T **p, size_t n)
 {
-    const int r = dalloc(h, p, n);
-    if (r != PIC_ERR_OOM) return r;
     *p = nullptr;
-    cudaGetLastError();
-    return PIC_OK;
+    const size_t bytes = n * sizeof(T);
+    if (bytes > kOptionalSmall) {
+        size_t free_bytes = 0, total = 0;
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes / 4 < bytes) {
+            cudaGetLastError();
+            return;
+        }
+    }
+    void *q = nullptr;
+    if (cudaMalloc(&q, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    *p = (T *)q;
+    h->optional.push_back(reinterpret_cast<void **>(p));
 }
 
 // Lehe coefficients, em_update_lehe.F90:8-25 (grid_dx = dy = dz = 1).
@@ -366,7 +393,7 @@ int enqueue_phase(pic_handle *h, int cur, bool reorder, int phase)
                 else launch_cyl_bhalf<float>(g, E, B, h->s);
                 break;
             case PIC_PHASE_MOVE:  // push, deposit and the wrap / outer-radius drop
-                if (h->sorted && h->bricks.nodeA)
+                if (h->sorted)
                     launch_cyl_move_deposit_f32_tiled(g, h->p32[cur], h->bricks, E, B, J, h->err, h->s);
                 else
                     launch_cyl_move_deposit_f32(g, h->p32[cur], h->cnt, E, B, J, h->err, h->s);
@@ -634,12 +661,8 @@ int step_profiled(pic_handle *h, int32_t nsteps)
     return rc;
 }
 
-// The FP32 mover variant is baked into the step graphs: drop them when the
-// tile ranges become valid or stale.
-void set_sorted(pic_handle *h, bool sorted)
+void drop_graphs(pic_handle *h)
 {
-    if (h->sorted == sorted) return;
-    h->sorted = sorted;
     for (auto &row : h->graph)
         for (auto &ge : row)
             if (ge) {
@@ -647,6 +670,35 @@ void set_sorted(pic_handle *h, bool sorted)
                 ge = nullptr;
             }
 }
+
+// The FP32 mover variant is baked into the step graphs: drop them when the
+// tile ranges become valid or stale.
+void set_sorted(pic_handle *h, bool sorted)
+{
+    if (h->sorted == sorted) return;
+    h->sorted = sorted;
+    drop_graphs(h);
+}
+
+}  // namespace
+
+// Give the arrays the handle can do without back to the device; false: there
+// are none.
+static bool release_optional(pic_handle *h)
+{
+    if (h->optional.empty()) return false;
+    // the captured steps refer to them
+    cudaStreamSynchronize(h->s);
+    drop_graphs(h);
+    for (void **p : h->optional) {
+        cudaFree(*p);
+        *p = nullptr;
+    }
+    h->optional.clear();
+    return true;
+}
+
+namespace {
 
 // One step of pic_step as a graph launch on h->s (graphs captured on first use).
 int enqueue_graph_step(pic_handle *h)
@@ -1100,6 +1152,7 @@ void pic_destroy(pic_handle *h)
     if (h->ev_group) cudaEventDestroy(h->ev_group);
     pin_return(h->pin);
     for (void *p : h->allocs) cudaFree(p);
+    for (void **p : h->optional) cudaFree(*p);
     if (h->cs) cudaStreamDestroy(h->cs);
     if (h->s) cudaStreamDestroy(h->s);
     delete h;
@@ -1242,10 +1295,6 @@ int pic_create(const pic_config *cfg, pic_handle **out)
             (r = dalloc(h, &bk.scan_tmp, scan_tmp_len(nt + 1))) ||
             (r = dalloc(h, &bk.wmax_bits, 1))) {
         }
-        // the node averages of the tiled movers, computed once per move
-        // instead of by every brick for its box
-        if (!r && !(r = dalloc_optional(h, (char **)&bk.nodeB, (size_t)g.ncell * sizeof(float2))) && bk.nodeB)
-            r = dalloc_optional(h, (char **)&bk.nodeA, (size_t)g.ncell * sizeof(float4));
         // the boxes' report to step_reorders
         if (!r && g.geom == PIC_GEOM_CARTESIAN && !g.x_external) {
             h->over_host = reinterpret_cast<uint32_t *>(h->pin + kPinOver);
@@ -1287,10 +1336,6 @@ int pic_create(const pic_config *cfg, pic_handle **out)
             !(r = dalloc(h, &T.qmax, 1)))
             h->tiled64 = true;
         T.marks = reinterpret_cast<uint8_t *>(exchange_marks(h->sc));
-        // without the node array the Cartesian tiles average their own nodes;
-        // the cylindrical ones need it
-        if (!r && g.dims == 3) r = dalloc_optional(h, &T.node, 6 * (size_t)g.ncell);
-        if (g.geom == PIC_GEOM_CYLINDRICAL && !T.node) h->tiled64 = false;
     }
     if (!r && c.exact_current) {
         SegRecords &R = h->rec;
@@ -1331,6 +1376,16 @@ int pic_create(const pic_config *cfg, pic_handle **out)
     if (r) {
         pic_destroy(h);
         return r;
+    }
+    // the node averages of the tiled movers, computed once per move instead of
+    // by every brick or tile for its box; last, after what the handle needs
+    if (h->fp32) {
+        Bricks &bk = h->bricks;
+        add_optional(h, &bk.nodeA, (size_t)g.ncell);
+        if (bk.nodeA) add_optional(h, &bk.nodeB, (size_t)g.ncell);
+        if (!bk.nodeB) release_optional(h);
+    } else if (h->tiled64 && g.dims == 3) {
+        add_optional(h, &h->t64.node, 6 * (size_t)g.ncell);
     }
     *out = h;
     return PIC_OK;
@@ -1607,7 +1662,7 @@ int pic_move_deposit(pic_handle *h)
     if (h->g.geom == PIC_GEOM_CYLINDRICAL && h->fp32) {
         float *E[3], *B[3], *J[3];
         field_ptrs(h, E, B, J);
-        if (h->sorted && h->bricks.nodeA)
+        if (h->sorted)
             launch_cyl_move_deposit_f32_tiled(h->g, h->p32[h->cur], h->bricks, E, B, J, h->err, h->s);
         else
             launch_cyl_move_deposit_f32(h->g, h->p32[h->cur], h->cnt, E, B, J, h->err, h->s);
@@ -2344,7 +2399,10 @@ int pic_solve_gauss(pic_handle *h, double tol, int32_t max_iter, int32_t *iters,
     else launch_rho_f64(g, h->p64[h->cur], h->cnt, h->rho, h->rho_pos, h->s);
     int it = 0;
     double rr = 0.0, mean = 0.0;
-    const int rc = solve_gauss(g, h->E, h->fp32, h->rho, tol, max_iter, h->s, &it, &rr, &mean);
+    int rc = solve_gauss(g, h->E, h->fp32, h->rho, tol, max_iter, h->s, &it, &rr, &mean);
+    if (rc == PIC_ERR_OOM && release_optional(h)) {   // its work arrays, allocated before anything else
+        rc = solve_gauss(g, h->E, h->fp32, h->rho, tol, max_iter, h->s, &it, &rr, &mean);
+    }
     if (iters) *iters = it;
     if (rel_residual) *rel_residual = rr;
     if (rho_mean) *rho_mean = mean;

@@ -634,7 +634,9 @@ __global__ void __launch_bounds__(kThreads) k_cyl_move(GridP g, CylP cp, PartF64
 // split) finds its nodes; a particle within one cell of its start deposits
 // into the fixed-point box (two segments of at most one cell per axis add at
 // most 2 q qi to a word), the rest (near-axis sub-steps, long azimuthal
-// steps, cells outside the box) through global memory.
+// steps, cells outside the box) through global memory.  NODES: the grid's node
+// values are in T.node.
+template <bool NODES>
 __global__ void __launch_bounds__(kT64Threads, 2) k_cyl_move_tiled(GridP g, CylP cp, PartF64 p, Tiles64 T,
                                                                    const double *__restrict__ Ex,
                                                                    const double *__restrict__ Ey,
@@ -654,6 +656,8 @@ __global__ void __launch_bounds__(kT64Threads, 2) k_cyl_move_tiled(GridP g, CylP
                 double wt[8];
                 weights<double, 3>(x - i, y - j, z - k, wt);
                 gather_box64<3>(ctx.bx, ctx.sN, nb, wt, pE, pB);
+            } else if (!NODES) {
+                interp3(g, Ex, Ey, Ez, Bx, By, Bz, x, y, z, pE, pB);
             } else {   // from the node array, as a box of the whole grid
                 Box64 whole;
                 whole.NX = g.mx;
@@ -698,12 +702,14 @@ void launch_cyl_move_deposit(const GridP &g, const PartF64 &p, const Counters *c
     if (T) {
         static bool attr_set = false;
         if (!attr_set) {
-            cudaFuncSetAttribute(k_cyl_move_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, kTile64SmemBytes);
+            cudaFuncSetAttribute(k_cyl_move_tiled<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTile64SmemBytes);
+            cudaFuncSetAttribute(k_cyl_move_tiled<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTile64SmemBytes);
             attr_set = true;
         }
-        launch_node_f64(g, *T, E, B, s);
-        k_cyl_move_tiled<<<T->ntiles, kT64Threads, T->smem_bytes, s>>>(g, cp, p, *T, E[0], E[1], E[2], B[0], B[1],
-                                                                        B[2], J[0], J[1], J[2], err);
+        if (T->node) launch_node_f64(g, *T, E, B, s);
+        auto move = T->node ? k_cyl_move_tiled<true> : k_cyl_move_tiled<false>;
+        move<<<T->ntiles, kT64Threads, T->smem_bytes, s>>>(g, cp, p, *T, E[0], E[1], E[2], B[0], B[1], B[2], J[0], J[1],
+                                                           J[2], err);
         count_launches(1);
     }
     // every particle, or the ones appended since the reorder
@@ -862,7 +868,7 @@ struct JAcc {
 // start cell is in it; otherwise, and always for the near-axis sub-stepper,
 // global memory with the same arithmetic, so both forms move particles bit
 // for bit alike.  The new cell, unwrapped from the brick centre, widens bd.
-template <bool TILED>
+template <bool TILED, bool PRE = false>
 __device__ __forceinline__ void cyl_push_f32(const GridP &g, const CylP &cp, const PartF32 &p, uint32_t n,
                                              const PState &st, const float *__restrict__ Ex,
                                              const float *__restrict__ Ey, const float *__restrict__ Ez,
@@ -924,7 +930,7 @@ __device__ __forceinline__ void cyl_push_f32(const GridP &g, const CylP &cp, con
             weights_f32<3>(dx, dy, dz, wt);
             pE[0] = pE[1] = pE[2] = pB[0] = pB[1] = pB[2] = 0.f;
             gather_box<3>(tb, l0 + tb.NX * l1 + tb.NXY * l2, wt, pE, pB);
-        } else if (TILED) {
+        } else if (PRE) {
             interp_nodes(g, tb, i, j, k, dx, dy, dz, pE, pB);
         } else {
             interp3f(g, Ex, Ey, Ez, Bx, By, Bz, i, j, k, dx, dy, dz, pE, pB);
@@ -971,7 +977,7 @@ __device__ __forceinline__ void cyl_push_f32(const GridP &g, const CylP &cp, con
             weights_f32<3>(ox, oy, oz, wt);
             pE[0] = pE[1] = pE[2] = pB[0] = pB[1] = pB[2] = 0.f;
             gather_box<3>(tb, (l0 + sx) + tb.NX * (l1 + sy) + tb.NXY * (l2 + sz), wt, pE, pB);
-        } else if (TILED) {
+        } else if (PRE) {
             interp_nodes(g, tb, ni, nj, nk, ox, oy, oz, pE, pB);
         } else {
             interp3f(g, Ex, Ey, Ez, Bx, By, Bz, ni, nj, nk, ox, oy, oz, pE, pB);
@@ -1167,7 +1173,9 @@ __global__ void __launch_bounds__(kThreads) k_cyl_substep_f32(GridP g, CylP cp, 
 // Tiled form: one CTA per brick (after a reorder).  The box is the stored
 // bounds of the brick's particles widened by one cell (the second gather is
 // at the cell a particle moves to); the radius is not periodic.  Each thread
-// loads its next particle while it moves this one.
+// loads its next particle while it moves this one.  PRE: the grid's node
+// averages are in bk.nodeA / nodeB.
+template <bool PRE>
 __global__ void __launch_bounds__(kTileThreads, 2)
     k_cyl_move_f32_tiled(GridP g, CylP cp, PartF32 p, Bricks bk, const float *__restrict__ Ex,
                          const float *__restrict__ Ey, const float *__restrict__ Ez, const float *__restrict__ Bx,
@@ -1185,7 +1193,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
     // a Strang move is below one cell per axis, a sub-stepped one below two
     tb.gA = bk.nodeA;
     tb.gB = bk.nodeB;
-    tile_setup<3, false, true, true>(g, bk, b, p1 - p0, 1, 2.f, sm, ts, tb, home_lo, home_hi, Ex, Ey, Ez, Bx, By, Bz);
+    tile_setup<3, false, true, PRE>(g, bk, b, p1 - p0, 1, 2.f, sm, ts, tb, home_lo, home_hi, Ex, Ey, Ez, Bx, By, Bz);
     Bounds bd;
     bd.init();
     JAcc acc;
@@ -1196,8 +1204,8 @@ __global__ void __launch_bounds__(kTileThreads, 2)
         for (uint32_t n = n0; n < p1; n += kTileThreads) {
             PState nxt = cur;
             if (p1 - n > kTileThreads) nxt = load_state<3>(p, n + kTileThreads);
-            cyl_push_f32<true>(g, cp, p, n, cur, Ex, Ey, Ez, Bx, By, Bz, Jx, Jy, Jz, err, tb, bd, acc, bk.bid,
-                               bk.count);
+            cyl_push_f32<true, PRE>(g, cp, p, n, cur, Ex, Ey, Ez, Bx, By, Bz, Jx, Jy, Jz, err, tb, bd, acc, bk.bid,
+                                    bk.count);
             cur = nxt;
         }
     }
@@ -1221,16 +1229,18 @@ void launch_cyl_move_deposit_f32_tiled(const GridP &g, const PartF32 &p, const B
 {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_cyl_move_f32_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, kBrickSmemCyl);
+        cudaFuncSetAttribute(k_cyl_move_f32_tiled<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBrickSmemCyl);
+        cudaFuncSetAttribute(k_cyl_move_f32_tiled<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBrickSmemCyl);
         attr_set = true;
     }
     const CylP cp = cyl_params(g);
     // the queue of near-axis slots: the brick-id scratch of the reorder, its
     // length in the scan scratch (both free between reorders)
-    launch_node_avg(g, bk, E, B, s);
+    if (bk.nodeA) launch_node_avg(g, bk, E, B, s);
     cudaMemsetAsync(bk.count, 0, sizeof(uint32_t), s);
-    k_cyl_move_f32_tiled<<<bk.ntiles, kTileThreads, bk.smem_floats * 4, s>>>(g, cp, p, bk, E[0], E[1], E[2], B[0],
-                                                                            B[1], B[2], J[0], J[1], J[2], err);
+    auto move = bk.nodeA ? k_cyl_move_f32_tiled<true> : k_cyl_move_f32_tiled<false>;
+    move<<<bk.ntiles, kTileThreads, bk.smem_floats * 4, s>>>(g, cp, p, bk, E[0], E[1], E[2], B[0], B[1], B[2], J[0], J[1],
+                                                             J[2], err);
     k_cyl_substep_f32<<<kSMs * 4, kThreads, 0, s>>>(g, cp, p, bk.bid, bk.count, E[0], E[1], E[2], B[0], B[1], B[2],
                                                    J[0], J[1], J[2], err);
     k_cyl_axis_current<float><<<dim3((g.my + 127) / 128, g.mz), 128, 0, s>>>(g, J[0], J[1], J[2]);

@@ -223,9 +223,13 @@ int solve_gauss(const GridP &g, void *const E[3], bool fp32, const double *rho, 
     double *buf = nullptr;
     CGScalars *sc = nullptr;
     cudaError_t e = cudaMalloc(&buf, (4 * (size_t)q.n + kPBlocks) * sizeof(double));
-    if (e != cudaSuccess) return PIC_ERR_OOM;
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // not left for the next call
+        return PIC_ERR_OOM;
+    }
     e = cudaMalloc(&sc, sizeof(CGScalars));
     if (e != cudaSuccess) {
+        cudaGetLastError();
         cudaFree(buf);
         return PIC_ERR_OOM;
     }

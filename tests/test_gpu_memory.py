@@ -1,0 +1,133 @@
+"""Runs that nearly fill the device: arrays that only make a run faster are not
+taken, or given back, when what the run needs would not fit beside them.  The
+device is filled with a torch tensor that nothing touches."""
+import contextlib
+
+import numpy as np
+import pytest
+
+from .test_gpu_boxes import _cfg, _hot
+
+pytestmark = pytest.mark.gpu
+
+SLACK = 32 << 20   # allocation granularity, graphs
+
+
+@contextlib.contextmanager
+def _only(room):
+    """`room` bytes of device memory free."""
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - int(room), dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+
+
+def _used(run):
+    """What run() returned and the device memory it held at its end."""
+    import torch
+
+    run()   # kernels loaded
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    held = []
+    out = run(lambda: held.append(before - torch.cuda.mem_get_info()[0]))
+    return out, held[0]
+
+
+def _particles(kind, shape, n):
+    p = _hot(*shape, 3, 1, 3, 0.3)
+    for k in p.NAMES:
+        setattr(p, k, getattr(p, k)[:n].copy())
+    p.flv[:] = 1 + np.arange(n) % 2
+    p.q[:] = np.where(p.flv == 1, 1.0, -1.0)
+    if kind == "cylindrical":
+        p.x[:] = 3.6 + (p.x - 3.0) * (shape[0] - 1) / shape[0]
+        p.q[:] *= p.x - 3.0
+    return p
+
+
+@pytest.mark.parametrize("geom,precision,optional,filt", [
+    ("cartesian", "fp64", 48, 0), ("cylindrical", "fp64", 48, 0), ("cartesian", "fp32", 24, 0),
+    ("cylindrical", "fp32", 24, 0)])
+def test_a_run_that_fits_without_the_optional_arrays(geom, precision, optional, filt):
+    """Room for what a run needs with its outputs, and for part of its optional
+    arrays (`optional` bytes a cell), the density arrays left short of 0.6 of
+    their size once the optional ones are taken: every call succeeds and gives
+    what the run gives with room to spare (particles bit for bit after the
+    first move, fields to the rounding of the current's sums)."""
+    from pictor_b200 import PicConfig, Simulation
+
+    shape = (128, 8, 2048) if geom == "cylindrical" else (128, 128, 128)
+    cells = int(np.prod([n + 5 for n in shape]))
+    p = _particles(geom, shape, 200000)
+    kw = dict(geom="cylindrical", rmin=-0.5, inc_axis=1) if geom == "cylindrical" else dict(curr_filter=filt)
+    cfg = PicConfig(nx=shape[0], ny=shape[1], nz=shape[2], dims=3, c=0.45, qi=0.01, precision=precision,
+                    capacity=300000, reorder_period=0, brick=(8, 8, 4), **kw)
+
+    def run(at_end=lambda: None):
+        with Simulation(cfg) as s:
+            s.load_particles(p)
+            s.reorder()
+            s.step(1)
+            first = s.fetch_particles()
+            s.step(2)
+            d = s.diagnostics(0.01)
+            f = s.fetch_fields(False)
+            at_end()
+            return first, d, f
+
+    (pa, da, fa), used = _used(run)
+    need = used - optional * cells
+    with _only(need + optional * cells - 0.6 * 16 * cells):
+        pb, db, fb = run()
+    with _only(need + SLACK):
+        run()
+    order = [np.lexsort((q.z, q.y, q.x)) for q in (pa, pb)]   # the FP32 reorder's slots are in any order
+    for k in pa.NAMES:
+        assert np.array_equal(getattr(pa, k)[order[0]], getattr(pb, k)[order[1]]), k
+    tol = 1e-12 if precision == "fp64" else 1e-5
+    for k in ("Ex", "Ey", "Ez", "Bx", "By", "Bz"):
+        a, b = getattr(fa, k), getattr(fb, k)
+        assert np.abs(a - b).max() <= tol * max(np.abs(fa.Ex).max(), np.abs(a).max()), k
+    assert np.allclose(da["kinetic"], db["kinetic"], rtol=1e-6)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_optional_arrays_are_given_back(precision):
+    """A run created with room to spare has its optional arrays; when the room
+    goes, a later call that allocates (the density of the diagnostics, the
+    Gauss solve) takes their place, and the run steps on."""
+    from pictor_b200 import Simulation
+
+    shape = (128, 128, 128)
+    cfg, sc = _cfg(shape, 3, 1, 0, precision)
+    p = _particles("cartesian", shape, 200000)
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        for s in (a, b):
+            s.load_particles(p)
+            s.reorder()
+            s.step(1)
+        da = a.diagnostics(sc["masse"])
+        ga = a.solve_gauss(1e-6)
+        with _only(8 << 20):
+            db = b.diagnostics(sc["masse"])
+        with _only(8 << 20):
+            try:
+                b.solve_gauss(1e-6)
+            except RuntimeError as e:   # 4 doubles a cell: more than what is left to give
+                assert "OOM" in str(e)
+        gb = b.solve_gauss(1e-6)
+        for s in (a, b):
+            s.step(3)
+        pa, pb = a.fetch_particles(), b.fetch_particles()
+    assert abs(da["rho_max"] - db["rho_max"]) <= 1e-12 * da["rho_max"]
+    assert ga["iters"] == gb["iters"]
+    order = [np.lexsort((q.z, q.y, q.x)) for q in (pa, pb)]
+    tol = 1e-9 if precision == "fp64" else 1e-3
+    assert np.abs(pa.x[order[0]] - pb.x[order[1]]).max() <= tol
