@@ -34,7 +34,7 @@ struct pic_handle {
     cudaStream_t s = nullptr;
     bool fp32 = false;
     void *E[3] = {}, *B[3] = {}, *J[3] = {};
-    void *Jtmp[3] = {};   // the current filter's second buffer
+    void *Jtmp[3] = {};   // the current filter's second buffer; [1], [2] optional
     double *open_col = nullptr;   // den, vel per (j, k) column of an 'open' particle face (2 my mz)
     // convolutional PML: per-axis tables (6 doubles and a flag per index),
     // twelve psi grids in the handle's precision (E psi1 x,y,z, psi2 x,y,z,
@@ -728,13 +728,22 @@ size_t field_bytes(const pic_handle *h) { return (size_t)h->g.ncell * (h->fp32 ?
 
 int ensure_jtmp(pic_handle *h)
 {
-    for (int c = 0; c < 3; c++) {
-        if (h->Jtmp[c]) continue;
-        const int r = dalloc(h, (char **)&h->Jtmp[c], field_bytes(h));
-        if (r) return r;
-        CK(cudaMemsetAsync(h->Jtmp[c], 0, field_bytes(h), h->s));
-    }
+    if (h->Jtmp[0]) return PIC_OK;
+    const int r = dalloc(h, (char **)&h->Jtmp[0], field_bytes(h));
+    if (r) return r;
+    CK(cudaMemsetAsync(h->Jtmp[0], 0, field_bytes(h), h->s));
     return PIC_OK;
+}
+
+// The filter's buffers of the other two components, with which a pass is one
+// launch for all three.
+void add_jtmp(pic_handle *h)
+{
+    for (int c = 1; c < 3; c++) {
+        if (h->Jtmp[c]) continue;
+        add_optional(h, (char **)&h->Jtmp[c], field_bytes(h));
+        if (h->Jtmp[c]) cudaMemsetAsync(h->Jtmp[c], 0, field_bytes(h), h->s);
+    }
 }
 
 // The density arrays of the diagnostics, in one block.
@@ -1377,13 +1386,19 @@ int pic_create(const pic_config *cfg, pic_handle **out)
         pic_destroy(h);
         return r;
     }
-    // the node averages of the tiled movers, computed once per move instead of
-    // by every brick or tile for its box; last, after what the handle needs
+    // last, after what the handle needs: the filter's further buffers, and the
+    // node averages of the tiled movers, computed once per move instead of by
+    // every brick or tile for its box
+    if (h->Jtmp[0]) add_jtmp(h);
     if (h->fp32) {
         Bricks &bk = h->bricks;
         add_optional(h, &bk.nodeA, (size_t)g.ncell);
         if (bk.nodeA) add_optional(h, &bk.nodeB, (size_t)g.ncell);
-        if (!bk.nodeB) release_optional(h);
+        if (!bk.nodeB && bk.nodeA) {   // of no use alone
+            cudaFree(bk.nodeA);
+            bk.nodeA = nullptr;
+            h->optional.pop_back();
+        }
     } else if (h->tiled64 && g.dims == 3) {
         add_optional(h, &h->t64.node, 6 * (size_t)g.ncell);
     }

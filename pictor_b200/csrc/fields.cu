@@ -262,13 +262,29 @@ void launch_fold(const GridP &g, T *const J[3], cudaStream_t s)
 }
 
 // `passes` filter passes over J, alternating between J and tmp (ghost cells
-// of tmp are not written); returns the buffer that holds the result.
+// of tmp are not written); returns the buffer that holds the result.  With one
+// buffer (tmp[1] or tmp[2] null) component by component, the result in J.
 template <typename T>
 T *const *launch_filter(const GridP &g, int passes, T *const J[3], T *const tmp[3], cudaStream_t s)
 {
     const dim3 block(32, 8, 1);
     dim3 grid = interior_grid(g);
-    grid.z = 3 * (g.dims == 3 ? (unsigned)((g.nz + kFilterKz - 1) / kFilterKz) : 1u);
+    grid.z = g.dims == 3 ? (unsigned)((g.nz + kFilterKz - 1) / kFilterKz) : 1u;
+    if (!tmp[1] || !tmp[2]) {
+        for (int c = 0; c < 3; c++) {
+            T *from = J[c], *to = tmp[0];
+            for (int p = 0; p < passes; p++) {
+                const Comp3<T> a = {{from, from, from}}, b = {{to, to, to}};
+                if (g.dims == 3) k_filter<T, 3><<<grid, block, 0, s>>>(g, a, b);
+                else k_filter<T, 2><<<grid, block, 0, s>>>(g, a, b);
+                count_launches(1);
+                std::swap(from, to);
+            }
+            if (from != J[c]) cudaMemcpyAsync(J[c], from, (size_t)g.ncell * sizeof(T), cudaMemcpyDeviceToDevice, s);
+        }
+        return J;
+    }
+    grid.z *= 3;
     T *const *from = J, *const *to = tmp;
     for (int p = 0; p < passes; p++) {
         const Comp3<T> a = {{from[0], from[1], from[2]}}, b = {{to[0], to[1], to[2]}};

@@ -54,7 +54,7 @@ def _particles(kind, shape, n):
 
 @pytest.mark.parametrize("geom,precision,optional,filt", [
     ("cartesian", "fp64", 48, 0), ("cylindrical", "fp64", 48, 0), ("cartesian", "fp32", 24, 0),
-    ("cylindrical", "fp32", 24, 0)])
+    ("cylindrical", "fp32", 24, 0), ("cartesian", "fp32", 24 + 8, 1), ("cartesian", "fp64", 48 + 16, 2)])
 def test_a_run_that_fits_without_the_optional_arrays(geom, precision, optional, filt):
     """Room for what a run needs with its outputs, and for part of its optional
     arrays (`optional` bytes a cell), the density arrays left short of 0.6 of
