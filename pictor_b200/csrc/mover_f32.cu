@@ -91,6 +91,9 @@ __global__ void __launch_bounds__(kThreads) k_node_avg(GridP g, const float *__r
     }
 }
 
+// The move's number since the reorder, where no node pass counts it.
+__global__ void k_count_move(uint32_t *over) { *over += 1; }
+
 void launch_node_avg(const GridP &g, const Bricks &bk, float *const E[3], float *const B[3], cudaStream_t s)
 {
     const bool cyl = g.geom == PIC_GEOM_CYLINDRICAL;
@@ -205,7 +208,12 @@ void launch_move_deposit_f32_tiled(const GridP &g, const PartF32 &p, const Brick
         return;
     }
     const bool pre = bk.nodeA != nullptr;
-    if (pre) launch_node_avg(g, bk, E, B, s);
+    if (pre) {
+        launch_node_avg(g, bk, E, B, s);
+    } else if (bk.over) {
+        k_count_move<<<1, 1, 0, s>>>(bk.over);
+        count_launches(1);
+    }
 #define PIC_MOVE_TILED(D, X, P)                                                                                      \
     k_move_f32_tiled<D, X, P><<<bk.ntiles, kTileThreads, bytes, s>>>(g, p, bk, E[0], E[1], E[2], B[0], B[1], B[2], J[0], \
                                                                     J[1], J[2], err)

@@ -131,3 +131,29 @@ def test_optional_arrays_are_given_back(precision):
     order = [np.lexsort((q.z, q.y, q.x)) for q in (pa, pb)]
     tol = 1e-9 if precision == "fp64" else 1e-3
     assert np.abs(pa.x[order[0]] - pb.x[order[1]]).max() <= tol
+
+
+def test_outgrown_boxes_are_reported_without_the_node_arrays():
+    """A hot run with no room for the node arrays reorders as often as one that
+    has them."""
+    from pictor_b200 import Simulation
+
+    shape, ppc = (160, 96, 96), 2
+    cfg, _ = _cfg(shape, 3, ppc, 20)
+
+    def run(at_end=lambda: None):
+        with Simulation(cfg) as s:
+            s.init_weibel(ppc, 0.5, 0.0, 0.2, 0.2)
+            s.reorder()
+            s.profile(True)
+            s.phase_times()
+            s.step(40)
+            at_end()
+            t = s.phase_times()["launches"]
+            return t["reorder"], t["move"]
+
+    (reorders, moves), used = _used(run)
+    with _only(used - 24 * 165 * 101 * 101 + SLACK):
+        got, moved = run()
+    assert got == reorders
+    assert moved == moves      # the counting launch stands where the node pass stood
