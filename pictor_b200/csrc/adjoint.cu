@@ -693,7 +693,8 @@ struct pic_adjoint {
     long long cap = 0, np = 0;
     size_t tsz = 8;                 // sizeof(T)
     std::vector<void *> allocs;
-    // particles: initial state, current state, cotangents (x, y, z, u, v, w)
+    // particles: initial state, current state, cotangents (x, y, z, u, v, w;
+    // allocated with the tape), each six arrays in one block
     void *p0[6] = {}, *p[6] = {}, *pb[6] = {};
     void *qw = nullptr;             // weights (T)
     double *q64 = nullptr, *sgn = nullptr;
@@ -704,7 +705,8 @@ struct pic_adjoint {
     // in random order: 64 steps forward 2.0 -> 1.5 ms, gradient 9.4 -> 7.0 ms).
     // What a call returns is in the loaded order.
     uint32_t *perm = nullptr;
-    double *out64 = nullptr;        // staging of what a call returns, 1 array of cap
+    double *out64 = nullptr;        // staging of what a call returns, 1 array of cap: on p, whose
+                                    // contents only a forward run needs while it runs
     // fields: E, B, scratch B_a, cotangents Ebar (2), Bbar; initial E, B
     void *E[3] = {}, *B[3] = {}, *Ba[3] = {}, *Ebar[2][3] = {}, *Bbar[3] = {};
     void *J = nullptr;                // current, 4 words per cell
@@ -721,11 +723,13 @@ struct pic_adjoint {
     long long br_words = 0, br_np = 0, br_steps = 0;
     // checkpoints (every K steps: E, B) and the tape of one segment: the state
     // at the start of every step but the first, whose state is the checkpoint
-    // (E, B and the B between the half steps, in packed blocks of 9 field
-    // arrays; block s holds B between the half steps of step s)
+    // (particles: 6 arrays per step; E and B: 6 field arrays per step, of which
+    // the last, of the end of the segment, holds B only), and, if the device
+    // has the room, the B between the half steps of every step (3 field
+    // arrays), which the reverse step computes again otherwise
     int K = 0, T = 0, tapeK = 0;
     std::vector<void *> ck_p, ck_f;   // per checkpoint: 6 particle arrays / 6 field arrays
-    void *tape_p = nullptr, *tape_f = nullptr;
+    void *tape_p = nullptr, *tape_f = nullptr, *tape_ba = nullptr;
     double *acc = nullptr;            // objective, then 3 parameter gradients
     pic_handle *loader = nullptr;     // FP64 handle whose Weibel loader fills the initial state
 };
@@ -739,11 +743,45 @@ int cstat(cudaError_t e) { return e == cudaSuccess ? PIC_OK : (e == cudaErrorMem
         if (e_ != cudaSuccess) return cstat(e_); \
     } while (0)
 
+// Free an array of aalloc (and forget it).
+void afree(pic_adjoint *a, void **p)
+{
+    if (!*p) return;
+    cudaFree(*p);
+    a->allocs.erase(std::find(a->allocs.begin(), a->allocs.end(), *p));
+    *p = nullptr;
+}
+
+// The cached reverse sweep refers to the tape.
+void drop_sweep(pic_adjoint *a)
+{
+    if (a->gb) cudaGraphExecDestroy(a->gb);
+    a->gb = nullptr;
+}
+
 int aalloc(pic_adjoint *a, void **p, size_t bytes)
 {
-    ACK(cudaMalloc(p, bytes ? bytes : 1));
+    if (bytes == 0) bytes = 1;
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && a->tape_ba) {   // the array the handle can do without
+        cudaGetLastError();
+        drop_sweep(a);
+        afree(a, &a->tape_ba);
+        e = cudaMalloc(p, bytes);
+    }
+    ACK(e);
     a->allocs.push_back(*p);
     return PIC_OK;
+}
+
+// Six particle arrays of one block.
+int aalloc_particles(pic_adjoint *a, void *p[6])
+{
+    char *blk = nullptr;
+    const size_t pn = (size_t)a->cap * a->tsz;
+    const int r = aalloc(a, (void **)&blk, 6 * pn);
+    for (int k = 0; k < 6 && !r; k++) p[k] = blk + k * pn;
+    return r;
 }
 
 unsigned grid_of(long long n)
@@ -817,14 +855,18 @@ void step_fwd(pic_adjoint *a, PS<T> Pi, F3<T> Ei, F3<T> Bi, F3<T> Ba, PS<T> Po, 
     count_launches(4);
 }
 
-// Reverse of a step: P, E the state at its start, Ba the B between its half
-// steps, Bt the B after it.
+// Reverse of a step: P, E, B the state at its start, Ba the B between its half
+// steps (computed here if there is no tape of it), Bt the B after it.
 template <typename T>
-void step_rev(pic_adjoint *a, PS<T> P, F3<T> E, F3<T> Ba, F3<T> Bt, int &cur)
+void step_rev(pic_adjoint *a, PS<T> P, F3<T> E, F3<T> B, F3<T> Ba, F3<T> Bt, int &cur)
 {
     const AG &g = a->g;
     const unsigned gc = grid_of((long long)cells(a)), gp = grid_of(a->np);
     F3<T> Bb = f3<T>(a->Bbar), Ebt = f3<T>(a->Ebar[cur]), Ebp = f3<T>(a->Ebar[cur ^ 1]);
+    if (!a->tape_ba) {
+        k_bhalf<T><<<gc, 256, 0, a->s>>>(g, E, B, Ba);
+        count_launches(1);
+    }
     k_objective_curlB_T<T><<<gc, 256, 0, a->s>>>(g, Bt, Ebt, Bb, (T)g.fc, (T *)a->Nb);   // E_t = E + c curlB(B_t) - J
     k_curlE_T_from<T><<<gc, 256, 0, a->s>>>(g, Bb, Ebt, Ebp, (T)-g.h);                   // second half step
     k_move_T<T><<<gp, 256, 0, a->s>>>(g, P, (const T *)a->qw, a->flv, a->np, E, Ba, Ebt, ps<T>(a->pb), (T *)a->Nb);
@@ -903,11 +945,7 @@ int run_forward(pic_adjoint *a, int nsteps, int K, double *objective)
     }
     if (a->br_mode == kBranchReplay && (a->br_np != a->np || a->br_steps < nsteps)) return PIC_ERR_INVALID;
     if (a->br_mode == kBranchRecord && a->br_words < (long long)nsteps * a->np) {
-        if (a->br_tape) {
-            cudaFree(a->br_tape);
-            a->allocs.erase(std::find(a->allocs.begin(), a->allocs.end(), (void *)a->br_tape));
-            a->br_tape = nullptr;
-        }
+        afree(a, (void **)&a->br_tape);
         a->br_words = 0;
         int q = aalloc(a, (void **)&a->br_tape, (size_t)nsteps * (size_t)a->np * sizeof(unsigned long long));
         if (q) return q;
@@ -936,21 +974,21 @@ template <typename T>
 int ensure_tape(pic_adjoint *a)
 {
     const int K = a->K;
-    if (K <= a->tapeK) return PIC_OK;
-    for (void *t : {a->tape_p, a->tape_f}) {
-        if (!t) continue;
-        cudaFree(t);
-        a->allocs.erase(std::find(a->allocs.begin(), a->allocs.end(), t));
-    }
-    a->tape_p = a->tape_f = nullptr;
-    if (a->gb) {   // the cached sweep refers to the old tape
-        cudaGraphExecDestroy(a->gb);
-        a->gb = nullptr;
-    }
     int r;
-    if ((r = aalloc(a, &a->tape_p, (size_t)K * 6 * (size_t)a->cap * sizeof(T))) ||
-        (r = aalloc(a, &a->tape_f, (size_t)(K + 1) * 9 * cells(a) * sizeof(T))))
+    if (!a->pb[0] && (r = aalloc_particles(a, a->pb))) return r;
+    if (K <= a->tapeK) return PIC_OK;
+    drop_sweep(a);
+    for (void **t : {&a->tape_p, &a->tape_f, &a->tape_ba}) afree(a, t);
+    a->tapeK = 0;
+    if ((r = aalloc(a, &a->tape_p, (size_t)(K - 1) * 6 * (size_t)a->cap * sizeof(T))) ||
+        (r = aalloc(a, &a->tape_f, (size_t)K * 6 * cells(a) * sizeof(T))))
         return r;
+    const size_t ba = (size_t)K * 3 * cells(a) * sizeof(T);
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && ba <= free_bytes / 4) {
+        if (aalloc(a, &a->tape_ba, ba)) a->tape_ba = nullptr;
+    }
+    cudaGetLastError();
     a->tapeK = K;
     return PIC_OK;
 }
@@ -973,9 +1011,11 @@ int enqueue_backward(pic_adjoint *a)
         // sweep reads it
         const int n = t1 - t0;
         auto P = [&](int q) { return q == 0 ? ps_at<T>(a->ck_p[seg], (size_t)a->cap)
-                                            : ps_at<T>((char *)a->tape_p + (size_t)q * 6 * a->cap * sizeof(T), (size_t)a->cap); };
-        auto F = [&](int q, int k) { return q == 0 && k < 2 ? f3_at<T>(a->ck_f[seg], cells(a), k)
-                                                            : f3_at<T>(a->tape_f, cells(a), 3 * q + k); };
+                                            : ps_at<T>((char *)a->tape_p + (size_t)(q - 1) * 6 * a->cap * sizeof(T), (size_t)a->cap); };
+        // k = 0, 1, 2: E, B at the start of step q, B between its half steps
+        auto F = [&](int q, int k) { return k == 2 ? (a->tape_ba ? f3_at<T>(a->tape_ba, cells(a), q) : f3<T>(a->Ba))
+                                            : q == 0 ? f3_at<T>(a->ck_f[seg], cells(a), k)
+                                                     : f3_at<T>(a->tape_f, cells(a), 2 * (q - 1) + k); };
         ACK(cudaMemsetAsync(a->J, 0, 4 * fn, a->s));
         for (int q = 0; q + 1 < n; q++)
             step_fwd<T>(a, P(q), F(q, 0), F(q, 1), F(q, 2), P(q + 1), F(q + 1, 0), F(q + 1, 1), nullptr, -1);
@@ -984,7 +1024,7 @@ int enqueue_backward(pic_adjoint *a)
         k_bhalf<T><<<gc, 256, 0, a->s>>>(a->g, F(n - 1, 0), F(n - 1, 1), F(n - 1, 2));
         k_bhalf<T><<<gc, 256, 0, a->s>>>(a->g, F(n - 1, 0), F(n - 1, 2), F(n, 1));
         count_launches(2);
-        for (int q = n - 1; q >= 0; q--) step_rev<T>(a, P(q), F(q, 0), F(q, 2), F(q + 1, 1), cur);
+        for (int q = n - 1; q >= 0; q--) step_rev<T>(a, P(q), F(q, 0), F(q, 1), F(q, 2), F(q + 1, 1), cur);
     }
     ACK(cudaGetLastError());
     return PIC_OK;
@@ -1052,14 +1092,14 @@ int pic_adj_create(const pic_config *cfg, pic_adjoint **out)
     int r = PIC_OK;
     if (cudaStreamCreateWithFlags(&a->s, cudaStreamNonBlocking) != cudaSuccess) r = PIC_ERR_CUDA;
     const size_t pn = (size_t)a->cap * a->tsz, fn = cells(a) * a->tsz;
-    for (int k = 0; k < 6 && !r; k++)
-        if ((r = aalloc(a, &a->p0[k], pn)) || (r = aalloc(a, &a->p[k], pn)) || (r = aalloc(a, &a->pb[k], pn))) break;
+    if (!r) r = aalloc_particles(a, a->p0);
+    if (!r) r = aalloc_particles(a, a->p);
+    a->out64 = (double *)a->p[0];
     if (!r) r = aalloc(a, &a->qw, pn);
     if (!r) r = aalloc(a, (void **)&a->q64, (size_t)a->cap * sizeof(double));
     if (!r) r = aalloc(a, (void **)&a->sgn, (size_t)a->cap * sizeof(double));
     if (!r) r = aalloc(a, (void **)&a->flv, (size_t)a->cap * sizeof(int));
     if (!r) r = aalloc(a, (void **)&a->perm, (size_t)a->cap * sizeof(uint32_t));
-    if (!r) r = aalloc(a, (void **)&a->out64, (size_t)a->cap * sizeof(double));
     void **fl[] = {a->E, a->B, a->Ba, a->Ebar[0], a->Ebar[1], a->Bbar, a->E0, a->B0};
     for (void **f : fl)
         for (int k = 0; k < 3 && !r; k++) {
@@ -1089,15 +1129,19 @@ void pic_adj_destroy(pic_adjoint *a)
     delete a;
 }
 
-// perm of the n particles src: a stable radix sort of their cells.
+// perm of the n particles src: a stable radix sort of their cells.  Its arrays
+// go on p (6 words of 4 or 8 bytes per particle, free outside a forward run)
+// unless the histograms of a few particles are longer than those.
 static int sort_loaded(pic_adjoint *a, const PartF64 &src, long long n)
 {
     SortScratch sc = {};
     sc.ntiles = sort_tiles(n);
     sc.scan_tmp_len = scan_tmp_len(256 * sc.ntiles);
     const size_t words = 4 * (size_t)n + 256 * sc.ntiles + sc.scan_tmp_len;
-    uint32_t *blk = nullptr;
-    ACK(cudaMalloc((void **)&blk, words * sizeof(uint32_t) + sizeof(long long)));
+    const size_t bytes = words * sizeof(uint32_t) + sizeof(long long);
+    const bool on_p = bytes <= 6 * (size_t)a->cap * a->tsz;
+    uint32_t *blk = (uint32_t *)a->p[0];
+    if (!on_p) ACK(cudaMalloc((void **)&blk, bytes));
     long long *used = (long long *)blk;
     uint32_t *w = blk + 2;
     sc.key[0] = w; sc.key[1] = w + n; sc.idx[0] = w + 2 * n; sc.idx[1] = w + 3 * n;
@@ -1110,7 +1154,7 @@ static int sort_loaded(pic_adjoint *a, const PartF64 &src, long long n)
         r = cstat(cudaMemcpyAsync(a->perm, sc.idx[q], (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, a->s));
     }
     const cudaError_t e = cudaStreamSynchronize(a->s);
-    cudaFree(blk);
+    if (!on_p) cudaFree(blk);
     return r ? r : cstat(e);
 }
 

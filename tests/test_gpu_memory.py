@@ -157,3 +157,38 @@ def test_outgrown_boxes_are_reported_without_the_node_arrays():
         got, moved = run()
     assert got == reorders
     assert moved == moves      # the counting launch stands where the node pass stood
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_an_adjoint_that_fits_without_the_half_step_tape(precision):
+    """Room for the checkpoints and the tape of E and B, not for the tape of
+    the B between the half steps: the reverse steps compute it again, and the
+    gradient is that of a run with room for it (bit for bit: the same values
+    from the same expressions; the particles' sums are of one particle per
+    cell at most, in any order)."""
+    from pictor_b200 import PicConfig
+    from pictor_b200.adjoint import Adjoint
+
+    n, K, size = 1024, 8, 8 if precision == "fp64" else 4
+    cfg = PicConfig(nx=n, ny=n, dims=2, c=0.45, qi=0.01, precision=precision, capacity=20000)
+    p = _hot(n, n, 1, 2, 1, 3, 0.2)
+    for k in p.NAMES:
+        setattr(p, k, getattr(p, k)[:20000].copy())
+    p.flv[:] = 1 + np.arange(20000) % 2
+    p.q[:] = np.where(p.flv == 1, 1.0, -1.0)
+
+    def run(at_end=lambda: None):
+        with Adjoint(cfg) as a:
+            a.load_particles(p)
+            obj = a.forward(2 * K, K)
+            g = a.gradient(drift=0.0, temp=(0.0, 0.0))
+            at_end()
+            return obj, g
+
+    (oa, ga), used = _used(run)
+    with _only(used - 3 * K * n * n * size + SLACK):
+        ob, gb = run()
+    tol = 1e-12 if precision == "fp64" else 1e-4
+    assert abs(oa - ob) <= tol * oa
+    for k in ("u", "v", "w", "x", "y"):
+        assert np.abs(ga[k] - gb[k]).max() <= tol * np.abs(ga[k]).max(), k
