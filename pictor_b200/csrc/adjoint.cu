@@ -119,13 +119,14 @@ __global__ void k_efield(AG g, F3<T> E, F3<T> B, T *J, F3<T> Eout, double *acc)
         const int i = c % g.nx, j = c / g.nx;
         const int cy = at(g, i, j - 1), cx = at(g, i - 1, j);
         const T bx = B.x[c], by = B.y[c], bz = B.z[c];
-        const T ex = (E.x[c] + fc * (bz - B.z[cy])) - J[4 * c];
-        const T ey = (E.y[c] - fc * (bz - B.z[cx])) - J[4 * c + 1];
-        const T ez = ((E.z[c] + fc * (by - B.y[cx])) - fc * (bx - B.x[cy])) - J[4 * c + 2];
+        T *Jc = J + 4 * (size_t)c;
+        const T ex = (E.x[c] + fc * (bz - B.z[cy])) - Jc[0];
+        const T ey = (E.y[c] - fc * (bz - B.z[cx])) - Jc[1];
+        const T ez = ((E.z[c] + fc * (by - B.y[cx])) - fc * (bx - B.x[cy])) - Jc[2];
         Eout.x[c] = ex;
         Eout.y[c] = ey;
         Eout.z[c] = ez;
-        J[4 * c] = J[4 * c + 1] = J[4 * c + 2] = (T)0;
+        Jc[0] = Jc[1] = Jc[2] = (T)0;
         const double dx = bx, dy = by, dz = bz;
         s += 0.5 * (dx * dx + dy * dy + dz * dz);
     }
@@ -372,7 +373,7 @@ __device__ __forceinline__ void segment_values(const T F[3], const T W[2], T v[8
 template <typename T>
 __device__ __forceinline__ void scatter_values(const AG &g, T *J, int cx, int cy, const T v[8])
 {
-    const int c = at(g, cx, cy), cpx = at(g, cx + 1, cy), cpy = at(g, cx, cy + 1), cpxy = at(g, cx + 1, cy + 1);
+    const size_t c = at(g, cx, cy), cpx = at(g, cx + 1, cy), cpy = at(g, cx, cy + 1), cpxy = at(g, cx + 1, cy + 1);
     add_words(J + 4 * c, v[0], v[2], v[4], (T)0);
     add_words(J + 4 * cpx, (T)0, v[3], v[5], (T)0);
     add_words(J + 4 * cpy, v[1], (T)0, v[6], (T)0);

@@ -237,3 +237,38 @@ def test_results_come_in_the_loaded_order(n, precision, tol):
     for k in ("u", "v", "w", "x", "y"):
         ref = grads[0][k]
         assert np.linalg.norm(grads[1][k][order] - ref) <= tol * max(np.linalg.norm(ref), 1e-300), k
+
+
+def test_words_of_cells_past_2_31():
+    """A grid of more than 2^29 cells, whose current has more than 2^31 words:
+    two particles in its last cells and its first give the objective and the
+    gradient of the same particles on a small grid.  Both sit on the same
+    offsets from the end of the grid; the positions' FP32 rounding at 23171
+    (2^-10 of a cell and step) bounds the difference."""
+    import torch
+
+    from pictor_b200 import Particles, PicConfig
+    from pictor_b200.adjoint import Adjoint
+
+    big = 23171
+    assert big * big > 1 << 29
+    need = 140 << 30
+    if torch.cuda.mem_get_info()[0] < need:
+        pytest.skip("needs 140 GB of device memory")
+    res = []
+    for n in (32, big):
+        cfg = PicConfig(nx=n, ny=n, dims=2, c=0.45, qi=0.5, precision="fp32", capacity=64)
+        p = Particles.empty(4)
+        p.q[:], p.flv[:] = (1, -1, 1, -1), (1, 2, 1, 2)
+        p.x[:] = 3.0 + np.array([n - 1.5, n - 1.25, 0.25, n - 0.5])
+        p.y[:] = 3.0 + np.array([n - 1.25, n - 0.5, 0.5, n - 1.75])
+        p.z[:] = 1.5
+        p.u[:], p.v[:], p.w[:] = (0.5, -0.3, 0.2, 0.6), (0.4, 0.2, -0.5, 0.1), (0.1, 0.3, 0.2, -0.4)
+        with Adjoint(cfg) as a:
+            a.load_particles(p)
+            obj = a.forward(2, 2)
+            res.append((obj, a.gradient(drift=0.0, temp=(0.0, 0.0))))
+    (oa, ga), (ob, gb) = res
+    assert oa > 0 and abs(oa - ob) <= 0.02 * oa
+    for k in ("u", "v", "w"):
+        assert np.abs(ga[k] - gb[k]).max() <= 0.02 * np.abs(ga[k]).max(), k
