@@ -21,14 +21,29 @@ int field_energy_blocks(const GridP &g)
     return (int)(b < 1 ? 1 : b);
 }
 
-// Interior rows (j, k) of the grid; a warp takes rows gw, gw + nw, ... and its
-// lanes the cells of a row, so no flat index is divided per cell.
-__device__ __forceinline__ int row_count(const GridP &g) { return g.ny * (g.dims == 3 ? g.nz : 1); }
-__device__ __forceinline__ void row_jk(const GridP &g, int r, int &j, int &k)
+// The interior cells in pieces of rows, warp gw of nw taking pieces gw, gw + nw,
+// ..., so no flat index is divided per cell: a piece is up to kRowPiece cells of
+// one row, or, of rows shorter than half a warp, as many rows as fit into the
+// lanes.  f(offset of the cell, i).  2 x 2^20 cells as two rows of a warp each
+// took 20 ms, rows of 5 cells a sixth of the lanes.
+constexpr int kRowPiece = 512;
+template <typename F>
+__device__ __forceinline__ void for_interior_cells(const GridP &g, F f)
 {
-    const int kk = g.dims == 3 ? r / g.ny : 0;
-    j = 3 + (r - kk * g.ny);
-    k = g.dims == 3 ? 3 + kk : 1;
+    int lw = 5;   // 2^lw lanes per row
+    while (lw > 0 && (1 << (lw - 1)) >= g.nx) lw--;
+    const int lane = threadIdx.x & 31, sub = lane & ((1 << lw) - 1), nw = gridDim.x * (kDiagThreads / 32);
+    const int rows = g.ny * (g.dims == 3 ? g.nz : 1), per = 32 >> lw, groups = (rows - 1) / per + 1,
+              cuts = (g.nx - 1) / kRowPiece + 1;
+    for (long long it = blockIdx.x * (kDiagThreads / 32) + (threadIdx.x >> 5); it < (long long)groups * cuts; it += nw) {
+        const int grp = cuts == 1 ? (int)it : (int)(it / cuts), cut = (int)(it - (long long)grp * cuts);
+        const int r = grp * per + (lane >> lw);
+        if (r >= rows) continue;
+        const int kk = g.dims == 3 ? r / g.ny : 0;
+        const long long c0 = cidx(g, 0, 3 + (r - kk * g.ny), g.dims == 3 ? 3 + kk : 1);
+        const int i0 = 3 + cut * kRowPiece, i1 = min(i0 + kRowPiece, 3 + g.nx);
+        for (int i = i0 + sub; i < i1; i += 1 << lw) f(c0 + i, i);
+    }
 }
 
 __device__ __forceinline__ double block_sum(double v, double *red)
@@ -52,26 +67,19 @@ __global__ void __launch_bounds__(kDiagThreads) k_field_energy_partial(GridP g, 
     __shared__ double red[kDiagThreads / 32];
     double eb = 0, ee = 0;
     const double dtheta = 2.0 * 3.14159265358979323846264 / g.ny;
-    const int lane = threadIdx.x & 31, nw = gridDim.x * (kDiagThreads / 32), rows = row_count(g);
-    for (int row = blockIdx.x * (kDiagThreads / 32) + (threadIdx.x >> 5); row < rows; row += nw) {
-        int j, k;
-        row_jk(g, row, j, k);
-        const long long c0 = cidx(g, 0, j, k);
-        for (int i = 3 + lane; i < 3 + g.nx; i += 32) {
-            const long long c = c0 + i;
-            const double bx = Bx[c], by = By[c], bz = Bz[c], ex = Ex[c], ey = Ey[c], ez = Ez[c];
-            if (g.geom == PIC_GEOM_CYLINDRICAL) {
-                // CalcFldEnergy_cyl (cyl_savedata_routines.F90:8-31): r weights, axis cell excluded
-                if (i < 4) continue;
-                const double r = ((double)i - 3.0) + -0.5, rp = r + 0.5;
-                eb += ((r * (bx * bx) + rp * (by * by)) + rp * (bz * bz)) * dtheta;
-                ee += ((rp * (ex * ex) + r * (ey * ey)) + r * (ez * ez)) * dtheta;
-            } else {
-                eb += (bx * bx + by * by) + bz * bz;
-                ee += (ex * ex + ey * ey) + ez * ez;
-            }
+    for_interior_cells(g, [&](long long c, int i) {
+        const double bx = Bx[c], by = By[c], bz = Bz[c], ex = Ex[c], ey = Ey[c], ez = Ez[c];
+        if (g.geom == PIC_GEOM_CYLINDRICAL) {
+            // CalcFldEnergy_cyl (cyl_savedata_routines.F90:8-31): r weights, axis cell excluded
+            if (i < 4) return;
+            const double r = ((double)i - 3.0) + -0.5, rp = r + 0.5;
+            eb += ((r * (bx * bx) + rp * (by * by)) + rp * (bz * bz)) * dtheta;
+            ee += ((rp * (ex * ex) + r * (ey * ey)) + r * (ez * ez)) * dtheta;
+        } else {
+            eb += (bx * bx + by * by) + bz * bz;
+            ee += (ex * ex + ey * ey) + ez * ez;
         }
-    }
+    });
     const double sb = block_sum(eb, red);
     const double se = block_sum(ee, red);
     if (threadIdx.x == 0) {
@@ -350,20 +358,13 @@ __global__ void __launch_bounds__(kDiagThreads) k_gauss_max(GridP g, const T *__
                                                             const double *__restrict__ rho_pos, double *out2)
 {
     double res = 0, rm = 0;
-    const int lane = threadIdx.x & 31, nw = gridDim.x * (kDiagThreads / 32), rows = row_count(g);
-    for (int row = blockIdx.x * (kDiagThreads / 32) + (threadIdx.x >> 5); row < rows; row += nw) {
-        int j, k;
-        row_jk(g, row, j, k);
-        const long long c0 = cidx(g, 0, j, k);
-        for (int i = 3 + lane; i < 3 + g.nx; i += 32) {
-            const long long c = c0 + i;
-            double div = ((double)Ex[c] - (double)Ex[c - 1]) + ((double)Ey[c] - (double)Ey[c - g.sy]);
-            if (g.dims == 3) div = div + ((double)Ez[c] - (double)Ez[c - g.sz]);
-            const double rp = rho_pos[c];
-            res = fmax(res, fabs(div - (rho_neg[c] + rp)));
-            rm = fmax(rm, fabs(rp));
-        }
-    }
+    for_interior_cells(g, [&](long long c, int) {
+        double div = ((double)Ex[c] - (double)Ex[c - 1]) + ((double)Ey[c] - (double)Ey[c - g.sy]);
+        if (g.dims == 3) div = div + ((double)Ez[c] - (double)Ez[c - g.sz]);
+        const double rp = rho_pos[c];
+        res = fmax(res, fabs(div - (rho_neg[c] + rp)));
+        rm = fmax(rm, fabs(rp));
+    });
     for (int o = 16; o > 0; o >>= 1) {
         res = fmax(res, __shfl_down_sync(0xffffffffu, res, o));
         rm = fmax(rm, __shfl_down_sync(0xffffffffu, rm, o));

@@ -48,6 +48,44 @@ def test_noalloc_energy_matches_diagnostics(dims, nx, ny, nz):
         np.testing.assert_allclose(got, [ref["B2"], ref["E2"]], rtol=1e-12)
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(1, 1, 1), (513, 1, 1), (2, 7, 3), (17, 5, 1), (5, 333, 3), (1 << 21, 2, 1),
+                                      (31, 3, 40), (5, 1 << 18, 1)])
+def test_noalloc_energy_of_long_and_short_rows(nx, ny, nz):
+    """Grids of few long rows and of many short ones, against torch (FP64 sums
+    in another order), in a time no longer than 8 times that of a square grid
+    of as many cells (each cell read once, by as many lanes)."""
+    import torch
+
+    from pictor_b200 import _capi
+
+    L = _capi.lib()
+    dims = 3 if nz > 1 else 2
+
+    def run(nx, ny, nz, dims):
+        shape = ((nz + 5) if dims == 3 else 1, ny + 5, nx + 5)
+        gen = torch.Generator(device="cuda").manual_seed(nx)
+        f = [torch.randn(shape, dtype=torch.float64, device="cuda", generator=gen) for _ in range(6)]
+        out = torch.empty(2, dtype=torch.float64, device="cuda")
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        best = 1e9
+        for _ in range(5):
+            ev[0].record()
+            assert L.pic_field_energy_noalloc(*[C.c_void_p(a.data_ptr()) for a in f], nx, ny, nz, dims,
+                                              C.c_void_p(out.data_ptr()),
+                                              C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+            ev[1].record()
+            torch.cuda.synchronize()
+            best = min(best, ev[0].elapsed_time(ev[1]))
+        k = slice(2, -3) if dims == 3 else slice(None)
+        want = [sum((a[k, 2:-3, 2:-3] ** 2).sum().item() for a in f[q:q + 3]) for q in (3, 0)]
+        np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-12)
+        return best
+
+    t = run(nx, ny, nz, dims)
+    side = max(1, int((nx * ny * nz) ** 0.5))
+    assert t <= 8 * run(side, side, 1, 2) + 0.02
+
+
 def test_noalloc_rejects_bad_sizes():
     from pictor_b200 import _capi
 
