@@ -567,14 +567,7 @@ int step_reorders(pic_handle *h, bool *reorder)
     h->since_group++;
     if (*reorder || !h->over_host || !h->sorted || period <= kGroupMin || h->since_group < kGroupMin) return PIC_OK;
     if (h->group_reported) {
-        // (a caller's capture of pic_stream makes the event invalid: no report then)
-        if (cudaEventSynchronize(h->ev_group) == cudaErrorInvalidValue) {
-            cudaGetLastError();
-            h->group_reported = false;
-            *reorder = h->group_every > 0 && h->since_group >= h->group_every;
-            return PIC_OK;
-        }
-        CK(cudaGetLastError());
+        CK(cudaEventSynchronize(h->ev_group));
         // no later reorder is enqueued yet, so nothing writes the word now
         const int first = (int)*(volatile uint32_t *)h->over_host;
         *(volatile uint32_t *)h->over_host = 0;

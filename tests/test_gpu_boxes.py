@@ -156,3 +156,31 @@ def test_batched_steps_leave_the_learned_interval_alone(form):
     per = 6   # launches of a reorder
     assert abs(counts[0] - counts[1]) <= per, counts
     assert min(counts) >= 3 * per
+
+
+def test_reorders_captured_from_the_handle_stream():
+    """Two reorders captured by the caller from the handle's stream and
+    replayed: the steps after them do not wait for what was only captured."""
+    import torch
+
+    from pictor_b200 import Simulation
+
+    shape = (24, 24, 24)
+    cfg, _ = _cfg(shape, 3, 2, 20)
+    with Simulation(cfg) as s:
+        s.load_particles(_hot(*shape, 3, 2, 9))
+        s.reorder()
+        s.step(1)
+        n = s.particle_count()
+        s.set_sync(False)
+        stream = torch.cuda.ExternalStream(s.stream)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            s.reorder()
+            s.reorder()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        s.set_sync(True)
+        s.step(25)
+        assert s.device_errors() == 0
+        assert s.particle_count() == n
