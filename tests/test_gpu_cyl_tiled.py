@@ -130,3 +130,44 @@ def test_cyl_tiled_steps_track_per_particle_steps(modes):
     np.testing.assert_allclose(da["kinetic"].sum(), db["kinetic"].sum(), rtol=1e-6)
     fa, fb = da["B2"] + da["E2"], db["B2"] + db["E2"]
     assert abs(fa - fb) <= 1e-5 * fb, (fa, fb)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny,nz,n", [(37, 8, 33, 40000), (23, 18, 71, 120000)])
+def test_outgrown_cylinder_boxes_move_like_the_per_particle_form(nx, ny, nz, n, precision):
+    """Stepped without a reorder until the tiles' boxes are cut to shared
+    memory and most particles gather outside them (theta and z seams, the
+    columns next to the outer radius), then one tiled move against the
+    per-particle form from the same slots and fields: particles bit for bit,
+    the current to the rounding of its sums (up to 64 contributions a cell of
+    2^-53 or 2^-24 each: 1e-13, 1e-5 of the largest)."""
+    from pictor_b200 import PicConfig, Simulation
+
+    g = O.make_grid(3, nx, ny, nz, c=0.45, qi=QI, fdtd="yee", qm=(1.0, -1.0))
+    cfg = PicConfig(nx=nx, ny=ny, nz=nz, dims=3, c=0.45, qi=QI, qm=(1.0, -1.0), fdtd="yee", geom="cylindrical",
+                    precision=precision, capacity=4 * n, reorder_period=0, rmin=-0.5, inc_axis=1)
+    p = _particles(g, n, seed=8)
+    p.q[:] *= 1e-3                      # the fields stay what is loaded, the particles fly
+    f = random_fields(g, seed=17, scale=0.02)
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        a.load_particles(p)
+        a.reorder()
+        for _ in range(24):
+            a.load_fields(to_gpu_fields(f))
+            a.step(1)
+        b.load_particles(a.fetch_particles())
+        for s in (a, b):
+            s.load_fields(to_gpu_fields(f))
+            s.move_deposit()
+            s.fold_current()
+        pa, pb = a.fetch_particles(), b.fetch_particles()
+        fa, fb = a.fetch_fields(), b.fetch_fields()
+        assert a.device_errors() == 0
+    assert (pa.flv != 0).sum() > n // 3   # the rest left through the outer radius
+    for k in pa.NAMES:
+        np.testing.assert_array_equal(getattr(pa, k), getattr(pb, k), err_msg=k)
+    tol = 1e-13 if precision == "fp64" else 1e-5
+    for k in ("Jx", "Jy", "Jz"):
+        va, vb = interior(getattr(fa, k), g), interior(getattr(fb, k), g)
+        assert np.abs(vb).max() > 0
+        assert np.abs(va - vb).max() <= tol * np.abs(vb).max(), k
