@@ -11,6 +11,8 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include <cuda.h>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -844,19 +846,45 @@ int fetch_array_f32(pic_handle *h, const float *src, double *dst, long long n, i
     return PIC_OK;
 }
 
-// The host array of n values at p begins and ends in memory that is not
-// registered with the CUDA runtime.
-bool pageable(const double *p, size_t n)
+// End of the range registered with CUDA that holds p; null if p is pageable
+// memory; p itself if the driver cannot tell.
+const double *registered_end(const double *p)
 {
-    for (const double *q : {p, p + n - 1}) {
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, q) != cudaSuccess) {
+    using Query = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-            return false;
+            f = nullptr;
         }
-        if (at.type != cudaMemoryTypeUnregistered) return false;
+        return (Query)f;
+    }();
+    if (!query) return p;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    const CUresult r = query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p);
+    if (r == CUDA_ERROR_INVALID_VALUE) return nullptr;
+    if (r != CUDA_SUCCESS || query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) != CUDA_SUCCESS) return p;
+    return (const double *)(start + size);
+}
+
+// How many of the m host arrays of n values, from the first on, follow one
+// another within one registered range, or in pageable memory throughout.
+int joined_arrays(double *const *a, int m, size_t n)
+{
+    int e = 1;
+    while (e < m && a[e] == a[e - 1] + n) e++;
+    if (e == 1) return 1;
+    const double *end = registered_end(a[0]);
+    if (end) {
+        while (e > 1 && a[e - 1] + n > end) e--;
+        return e;
     }
-    return true;
+    int j = 1;   // (an array registered in part could not be copied alone either)
+    while (j < e && !registered_end(a[j])) j++;
+    return j;
 }
 
 // The configured filter passes over J, the result left in J.
@@ -1477,17 +1505,15 @@ int pic_fetch_fields(pic_handle *h, double *Ex, double *Ey, double *Ez, double *
         }
     if ((size_t)m * n <= (size_t)stage_field_chunk(h)) {
         // small grids: one conversion of all arrays into one staging buffer,
-        // copied from on the same stream, pageable host arrays that follow
-        // one another in one copy (64^2 cells: 88 us as a conversion, a copy
-        // and four stream events per array, 45 us now).  A copy that leaves
-        // one registered range for another, or for pageable memory, is
-        // refused, so arrays in registered memory keep a copy each.
+        // copied from on the same stream, host arrays that follow one another
+        // in one copy (64^2 cells: 88 us as a conversion, a copy and four
+        // stream events per array, 45 us now).  A copy that leaves one
+        // registered range for another, or for pageable memory, is refused,
+        // so arrays are joined within one range or in pageable memory.
         double *t = (double *)h->stage[0];
         if (m) launch_arrays_f32_to_f64((const float *const *)src, m, t, (long long)n, h->s);
         for (int k = 0; k < m;) {
-            int e = k + 1;
-            if (e < m && dst[e] == dst[e - 1] + n && pageable(dst[k], n))
-                while (e < m && dst[e] == dst[e - 1] + n && pageable(dst[e], n)) e++;
+            const int e = k + joined_arrays(dst + k, m - k, n);
             CK(cudaMemcpyAsync(dst[k], t + (size_t)k * n, (size_t)(e - k) * n * sizeof(double), cudaMemcpyDeviceToHost, h->s));
             k = e;
         }

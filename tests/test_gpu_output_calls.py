@@ -120,10 +120,10 @@ def test_fetched_fields(nx, ny, layout):
                 assert (buf[6:] == 7.0).all()
 
 
-@pytest.mark.parametrize("registered", [(0, 4), (3, 6), (5, 9), (0, 9), (2, 2)])
+@pytest.mark.parametrize("registered", [[(0, 4)], [(3, 6)], [(5, 9)], [(0, 9)], [], [(0, 3), (3, 7)], [(1, 2), (2, 9)]])
 def test_fetched_fields_into_partly_registered_memory(registered):
-    """Nine host arrays one after the other, of which some lie in memory that
-    is registered with CUDA (page-aligned: 64 x 64 float64 is 8 pages)."""
+    """Nine host arrays one after the other, of which some lie in one or two
+    ranges registered with CUDA (page-aligned: 64 x 64 float64 is 8 pages)."""
     import mmap
 
     import torch
@@ -137,17 +137,16 @@ def test_fetched_fields_into_partly_registered_memory(registered):
     buf = np.frombuffer(mmap.mmap(-1, 9 * n * 8), dtype=np.float64).reshape(9, n)
     buf[:] = 7.0
     out = Fields(*(buf[k].reshape(cfg.shape, order="F") for k in range(9)))
-    first, last = registered
     rt = torch.cuda.cudart()
     with Simulation(cfg) as s:
         s.load_fields(f)
         s.load_current(f.Jx, f.Jy, f.Jz)
-        if last > first:
+        for first, last in registered:
             assert int(rt.cudaHostRegister(buf[first].ctypes.data, (last - first) * n * 8, 0)) == 0
         try:
             s.fetch_fields(out=out)
         finally:
-            if last > first:
+            for first, _ in registered:
                 rt.cudaHostUnregister(buf[first].ctypes.data)
     for k in Fields.__dataclass_fields__:
         assert np.array_equal(getattr(out, k), getattr(f, k).astype(np.float32).astype(np.float64)), k
