@@ -21,28 +21,34 @@ int field_energy_blocks(const GridP &g)
     return (int)(b < 1 ? 1 : b);
 }
 
-// The interior cells in pieces of rows, warp gw of nw taking pieces gw, gw + nw,
-// ..., so no flat index is divided per cell: a piece is up to kRowPiece cells of
-// one row, or, of rows shorter than half a warp, as many rows as fit into the
-// lanes.  f(offset of the cell, i).  2 x 2^20 cells as two rows of a warp each
-// took 20 ms, rows of 5 cells a sixth of the lanes.
-constexpr int kRowPiece = 512;
+// The interior cells for the warps of the grid, f(offset of the cell, i), with
+// no flat index divided per cell: a warp takes pieces of up to kRowPiece cells
+// of a row, or, of rows of at most half its lanes, as many rows as fit into
+// them.  (A warp per row took 23.5 ms for 2 rows of 2^21 cells, 0.05 ms as a
+// square grid, and left lanes idle in short rows.)
+constexpr int kRowPiece = 256;
 template <typename F>
 __device__ __forceinline__ void for_interior_cells(const GridP &g, F f)
 {
-    int lw = 5;   // 2^lw lanes per row
-    while (lw > 0 && (1 << (lw - 1)) >= g.nx) lw--;
-    const int lane = threadIdx.x & 31, sub = lane & ((1 << lw) - 1), nw = gridDim.x * (kDiagThreads / 32);
-    const int rows = g.ny * (g.dims == 3 ? g.nz : 1), per = 32 >> lw, groups = (rows - 1) / per + 1,
-              cuts = (g.nx - 1) / kRowPiece + 1;
-    for (long long it = blockIdx.x * (kDiagThreads / 32) + (threadIdx.x >> 5); it < (long long)groups * cuts; it += nw) {
-        const int grp = cuts == 1 ? (int)it : (int)(it / cuts), cut = (int)(it - (long long)grp * cuts);
-        const int r = grp * per + (lane >> lw);
-        if (r >= rows) continue;
+    const int lane = threadIdx.x & 31, nw = gridDim.x * (kDiagThreads / 32);
+    const int gw = blockIdx.x * (kDiagThreads / 32) + (threadIdx.x >> 5), rows = g.ny * (g.dims == 3 ? g.nz : 1);
+    auto row_offset = [&](int r) {
         const int kk = g.dims == 3 ? r / g.ny : 0;
-        const long long c0 = cidx(g, 0, 3 + (r - kk * g.ny), g.dims == 3 ? 3 + kk : 1);
-        const int i0 = 3 + cut * kRowPiece, i1 = min(i0 + kRowPiece, 3 + g.nx);
-        for (int i = i0 + sub; i < i1; i += 1 << lw) f(c0 + i, i);
+        return cidx(g, 0, 3 + (r - kk * g.ny), g.dims == 3 ? 3 + kk : 1);
+    };
+    if (g.nx > 16) {
+        const int cuts = (g.nx - 1) / kRowPiece + 1;
+        for (int it = gw; it < rows * cuts; it += nw) {
+            const int r = cuts == 1 ? it : it / cuts, i0 = 3 + (it - r * cuts) * kRowPiece;
+            const int i1 = min(i0 + kRowPiece, 3 + g.nx);
+            const long long c0 = row_offset(r);
+            for (int i = i0 + lane; i < i1; i += 32) f(c0 + i, i);
+        }
+    } else {
+        const int lw = 32 - __clz(g.nx - 1);   // 2^lw lanes hold a row
+        const int i = 3 + (lane & ((1 << lw) - 1));
+        for (int r = (gw << (5 - lw)) + (lane >> lw); r < rows; r += nw << (5 - lw))
+            if (i < 3 + g.nx) f(row_offset(r) + i, i);
     }
 }
 
@@ -396,6 +402,10 @@ static void deposit_f32(const GridP &g, const PartF32 &p, const Counters *cnt, c
                         double *rho_pos, cudaStream_t s)
 {
     zero_rho(g, rho, rho_pos, s);
+    // fewer than two bricks per SM leave it too little in flight: with 24^3
+    // cells and 27 bricks the diagnostics take 82 us, 61 without bricks, with
+    // 218 to 256 bricks (0.9, 1 M particles) the same, with 870 170 and 234
+    if (bk && bk->ntiles < 2 * kSMs) bk = nullptr;
     const size_t sm = 2 * kRhoNodes * sizeof(double);
     if (bk && g.dims == 3) k_rho_f32_bricks<3><<<bk->ntiles, 256, sm, s>>>(g, p, *bk, rho, rho_pos);
     else if (bk) k_rho_f32_bricks<2><<<bk->ntiles, 256, sm, s>>>(g, p, *bk, rho, rho_pos);
