@@ -39,18 +39,44 @@ def test_density_by_bricks(shape, dims, ppc, steps):
     assert np.allclose(da["kinetic"], db["kinetic"], rtol=1e-12)
 
 
+@pytest.mark.parametrize("shape,dims,ppc,steps,brick", [((24, 20, 17), 3, 6, 0, (3, 3, 3)),
+                                                        ((41, 24, 23), 3, 6, 14, (4, 4, 4)),
+                                                        ((96, 75, 1), 2, 6, 25, (4, 4, 1)),
+                                                        ((96, 75, 1), 2, 40, 1, (4, 4, 1)),
+                                                        ((333, 5, 5), 3, 2, 3, (1, 5, 5))])
+def test_density_of_many_bricks(shape, dims, ppc, steps, brick):
+    """As test_density_by_bricks with at least the two bricks per SM from which
+    the density is summed brick by brick."""
+    from pictor_b200 import Simulation
+
+    cfg, sc = _cfg(shape, dims, ppc, 0, brick=brick)
+    assert np.prod([-(-n // b) for n, b in zip(shape, brick)]) >= 2 * 148
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        p = _hot(*shape, dims, ppc, 21)
+        p.q *= np.random.default_rng(2).uniform(0.2, 3.0, size=len(p))
+        a.load_particles(p)
+        a.reorder()
+        a.step(steps)
+        b.load_particles(a.fetch_particles())
+        b.load_fields(a.fetch_fields())
+        da, db = a.diagnostics(sc["masse"]), b.diagnostics(sc["masse"])
+    assert db["rho_max"] > 0
+    for k in ("rho_max", "gauss_linf"):
+        assert abs(da[k] - db[k]) <= 1e-12 * db["rho_max"], k
+
+
 @pytest.mark.parametrize("qi", [0.01, -0.01])
 def test_density_by_bricks_keeps_light_particles(qi):
     """Eight particles 2^-47 as heavy as the others, on nodes of their own, in
-    a brick of 16384, with either sign of the charge unit.  The others lie in
-    pairs of opposite charge at quarters of a cell, so their sums are exact
-    and cancel: the Gauss residual is the density of the heaviest light one,
-    the same reordered and not (one product per node), and FP32's positions
-    give it to 1e-6."""
+    a brick of 16384 (the other 319 bricks are empty), with either sign of the
+    charge unit.  The others lie in pairs of opposite charge at quarters of a
+    cell, so their sums are exact and cancel: the Gauss residual is the density
+    of the heaviest light one, the same reordered and not (one product per
+    node), and FP32's positions give it to 1e-6."""
     from pictor_b200 import PicConfig, Simulation
 
     n, light = 32, 2.0 ** -47
-    cfg = PicConfig(nx=n, ny=n, dims=2, c=0.45, qi=qi, precision="fp32", capacity=1 << 15, brick=(32, 32, 1))
+    cfg = PicConfig(nx=32 * n, ny=10 * n, dims=2, c=0.45, qi=qi, precision="fp32", capacity=1 << 15, brick=(n, n, 1))
     p = _hot(n, n, 1, 2, 8, 4)
     m = len(p)
     rng = np.random.default_rng(4)
