@@ -380,7 +380,8 @@ __device__ __forceinline__ void scatter_values(const AG &g, T *J, int cx, int cy
     add_words(J + 4 * cpxy, (T)0, (T)0, v[7], (T)0);
 }
 
-// Reverse of scatter_seg with Jbar: the cotangents of F and W.
+// Reverse of segment_values and scatter_values with Jbar: the cotangents of F
+// and W.
 template <typename T>
 __device__ __forceinline__ void scatter_seg_T(const AG &g, const F3<T> &Jbar, T sgn, int cx, int cy, const T F[3],
                                               const T W[2], T Fb[3], T Wb[2])

@@ -78,10 +78,10 @@ __device__ __forceinline__ T lgz(const GridP &g, const T *F, long long c0)
 // images, so it needs no launch of its own.  The columns of r that an update
 // leaves alone (ghosts, the axis) copy their images too, as the halo does.
 // The axis conditions read the updated cells next to the axis of two
-// opposite theta and follow in a small launch (k_cyl_axis).  With separate
-// launches for axis, halo, fold and the zeroing of J a step had 49 of them
-// (nr 64, 8 theta, nz 512, FP64: 314 us of a 868 us step; now 6 and
-// 92 us).
+// opposite theta and follow in a small launch (k_cyl_b_axis, k_cyl_e_axis).
+// With separate launches for axis, halo, fold and the zeroing of J a step had
+// 49 of them (nr 64, 8 theta, nz 512, FP64: 314 us of a 868 us step; now 6 and
+// 82 us).
 template <typename T>
 __device__ __forceinline__ void store_yz(const GridP &g, T *F, int i, int j, int k, T v, bool own = true)
 {

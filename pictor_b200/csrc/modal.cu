@@ -163,7 +163,7 @@ __device__ __forceinline__ void emit(const GridP &g, const GridP &gm, const doub
 // synthesis and all images; the columns an update leaves alone are emitted as
 // they are.  With launches for the update, the axis, the halo, the synthesis,
 // the fold and the projection each, a step had 43 of them (nr 128, nz 1024,
-// FP32: 379 us of a 877 us step; now 3 and 114 us).
+// FP32: 379 us of a 877 us step; now 3 and 90 us).
 
 // B half step (cyl_em_update.F90:66-83; Lehe :62-118): i 4..mx-1; then
 // UpdateBzAxis (:231-246: the circulation of Ey(4, :, k) is ny times its m = 0

@@ -304,8 +304,8 @@ __device__ __forceinline__ bool box_fits(const Bricks &bk, const int m[6], int j
 
 // The boxes of brick b for this step (one CTA, ends with a barrier): the
 // stored bounds widened by `margin` cells on each side (movers that gather a
-// second time at the cell they move to), or the brick +- 1 cell when that is
-// too large; strides and byte offsets; the fixed-point scale for the n
+// second time at the cell they move to), cut, when that is too large, to the
+// widest margin around the brick (at most kBoxMarginMax) that fits; strides and byte offsets; the fixed-point scale for the n
 // particles of the brick, whose moves are below dmax cells per axis (current
 // words of 32 bits, or 64 with WIDE); the
 // memory offsets of the box cells along each axis (the periodic interior
