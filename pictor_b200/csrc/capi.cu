@@ -105,8 +105,10 @@ struct pic_handle {
     bool tiled64 = false;
     Tiles64 t64 = {};
     std::vector<void *> allocs;
-    // pointers of this handle to arrays it can do without (add_optional)
+    // pointers of this handle to arrays it can do without (add_optional), and
+    // whether a caller captured launches that use them (kept from then on)
     std::vector<void **> optional;
+    bool optional_captured = false;
 };
 
 static thread_local long long g_launches = 0;
@@ -678,10 +680,10 @@ void set_sorted(pic_handle *h, bool sorted)
 }  // namespace
 
 // Give the arrays the handle can do without back to the device; false: there
-// are none.
+// are none to give.
 static bool release_optional(pic_handle *h)
 {
-    if (h->optional.empty()) return false;
+    if (h->optional.empty() || h->optional_captured) return false;
     // the captured steps refer to them
     cudaStreamSynchronize(h->s);
     drop_graphs(h);
@@ -694,6 +696,15 @@ static bool release_optional(pic_handle *h)
 }
 
 namespace {
+
+// Before a phase call that uses the optional arrays: a caller's graph of
+// queued phase calls (pic_set_sync(h, 0)) may be replayed at any later time.
+void note_capture(pic_handle *h)
+{
+    if (h->sync || h->optional.empty() || h->optional_captured) return;
+    cudaStreamCaptureStatus cap;
+    if (cudaStreamIsCapturing(h->s, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) h->optional_captured = true;
+}
 
 // One step of pic_step as a graph launch on h->s (graphs captured on first use).
 int enqueue_graph_step(pic_handle *h)
@@ -1692,6 +1703,7 @@ int pic_reset_current(pic_handle *h)
 int pic_move_deposit(pic_handle *h)
 {
     if (!h) return PIC_ERR_INVALID;
+    note_capture(h);
     for (int k = 0; k < 3; k++) CK(cudaMemsetAsync(h->J[k], 0, field_bytes(h), h->s));
     if (h->g.geom == PIC_GEOM_CYLINDRICAL && h->fp32) {
         float *E[3], *B[3], *J[3];
@@ -1785,6 +1797,7 @@ int pic_filter_current(pic_handle *h)
     if (!h || h->g.geom == PIC_GEOM_CYLINDRICAL) return PIC_ERR_INVALID;
     const int r = ensure_jtmp(h);
     if (r) return r;
+    note_capture(h);
     if (h->fp32) filter_current<float>(h);
     else filter_current<double>(h);
     return finish_phase(h);

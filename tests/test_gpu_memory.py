@@ -133,6 +133,60 @@ def test_optional_arrays_are_given_back(precision):
     assert np.abs(pa.x[order[0]] - pb.x[order[1]]).max() <= tol
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_optional_arrays_in_a_caller_s_graph_are_kept(precision):
+    """The phases of a step captured by the caller and replayed after a call
+    that found no room: the call fails instead of taking the arrays that the
+    graph uses, and the replay is the step (particles bit for bit: the first
+    move gathers from loaded fields)."""
+    import torch
+
+    from pictor_b200 import Simulation
+    from pictor_b200._capi import PicError
+
+    shape = (128, 128, 128)
+    cfg, sc = _cfg(shape, 3, 1, 0, precision)
+    p = _particles("cartesian", shape, 200000)
+    rng = np.random.default_rng(5)
+
+    def phases(s):
+        s.update_b_half()
+        s.move_deposit()
+        s.exchange_particles()
+        s.update_b_half()
+        s.update_e()
+        s.fold_current()
+        s.add_current()
+        s.reset_current()
+
+    with Simulation(cfg) as a, Simulation(cfg) as b:
+        f = a.fetch_fields(False)
+        for k in ("Ex", "Ey", "Ez", "Bx", "By", "Bz"):
+            getattr(f, k)[...] = rng.normal(scale=0.01, size=cfg.shape)
+        for s in (a, b):
+            s.load_fields(f)
+            s.load_particles(p)
+            s.reorder()
+        a.set_sync(False)
+        stream = torch.cuda.ExternalStream(a.stream)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            phases(a)
+        a.set_sync(True)
+        with _only(8 << 20), pytest.raises(PicError, match="OOM"):
+            a.diagnostics(sc["masse"])
+        with torch.cuda.stream(stream):
+            graph.replay()
+        torch.cuda.synchronize()
+        phases(b)
+        pa, pb = a.fetch_particles(), b.fetch_particles()
+        assert a.device_errors() == 0
+        assert a.diagnostics(sc["masse"])["rho_max"] > 0
+    order = [np.lexsort((q.z, q.y, q.x)) for q in (pa, pb)]
+    for k in pa.NAMES:
+        assert np.array_equal(getattr(pa, k)[order[0]], getattr(pb, k)[order[1]]), k
+
+
 def test_outgrown_boxes_are_reported_without_the_node_arrays():
     """A hot run with no room for the node arrays reorders as often as one that
     has them."""
