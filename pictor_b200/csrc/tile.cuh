@@ -305,13 +305,13 @@ __device__ __forceinline__ bool box_fits(const Bricks &bk, const int m[6], int j
 // The boxes of brick b for this step (one CTA, ends with a barrier): the
 // stored bounds widened by `margin` cells on each side (movers that gather a
 // second time at the cell they move to), cut, when that is too large, to the
-// widest margin around the brick (at most kBoxMarginMax) that fits; strides and byte offsets; the fixed-point scale for the n
-// particles of the brick, whose moves are below dmax cells per axis (current
-// words of 32 bits, or 64 with WIDE); the
-// memory offsets of the box cells along each axis (the periodic interior
-// image, or along a non-periodic x axis (XPER false: the radius of the
-// cylindrical form) the index itself); the current box zeroed and the
-// node-averaged fields staged.
+// widest margin around the brick (at most kBoxMarginMax) that fits; strides
+// and byte offsets; the fixed-point scale for the n particles of the brick,
+// whose moves are below dmax cells per axis (current words of 32 bits, or 64
+// with WIDE); the memory offsets of the box cells along each axis (the
+// periodic interior image, or along a non-periodic x axis (XPER false: the
+// radius of the cylindrical form) the index itself); the current box zeroed
+// and the node-averaged fields staged.
 template <int DIMS, bool XPER, bool WIDE = false, bool PRE = false>
 __device__ __forceinline__ void tile_setup(const GridP &g, const Bricks &bk, int b, uint32_t n, int margin, float dmax,
                                            float *sm, TileShared &ts, TileBox &tb, const int home_lo[3],
