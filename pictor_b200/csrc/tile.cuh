@@ -3,9 +3,9 @@
 //
 // A CTA moves the particles of one brick (bricks.cu groups them).  It stages
 // the node-averaged E and B of a box of cells around the brick in shared
-// memory (each node once per brick instead of 8 times per particle; the
-// Cartesian mover reads them from node arrays that one pass over the grid
-// fills before the move, the cylindrical one averages them itself with
+// memory (each node once per brick instead of 8 times per particle; copied
+// from node arrays that one pass over the grid fills before the move, or, in
+// slabs, batches and runs without those arrays, averaged by the CTA with
 // node_avg) and sums the brick's current in a shared box of fixed-point
 // words (32-bit; 64-bit for the cylindrical form, whose weights span the
 // radius), added to the global J once at the end.  The box is the

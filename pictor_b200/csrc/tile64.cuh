@@ -13,7 +13,7 @@
 //     of the per-particle gathers, so interpolated fields, and with them
 //     positions and momenta, equal the per-particle movers' bit for bit) of
 //     the box of cells the tile's particles occupy, widened by MARGIN cells,
-//     in shared memory;
+//     in shared memory (copied from the grid's node array where there is one);
 //   * it sums the tile's current in a 64-bit fixed-point box in shared memory
 //     and adds the box to J once with FP64 atomics, instead of 16 / 24
 //     global FP64 atomics per particle;
@@ -21,9 +21,9 @@
 //     records the cells its particles move to, which bound the box of the
 //     next step (the particles drift out of their tile between reorders).
 // The current differs from a per-particle mover's only in the order of its
-// sums and the fixed-point rounding of each contribution.  A tile whose box
-// does not fit in shared memory takes its own cells plus one on each side;
-// a particle whose cells lie outside the box gathers and deposits through
+// sums and the fixed-point rounding of each contribution.  A box that does
+// not fit in shared memory is cut to as much of it as fits around the tile (at
+// least the tile's cells and one on each side); a particle whose cells lie outside the box gathers and deposits through
 // global memory with the same arithmetic.
 #pragma once
 
