@@ -23,8 +23,9 @@
 // The current differs from a per-particle mover's only in the order of its
 // sums and the fixed-point rounding of each contribution.  A box that does
 // not fit in shared memory is cut to as much of it as fits around the tile (at
-// least the tile's cells and one on each side); a particle whose cells lie outside the box gathers and deposits through
-// global memory with the same arithmetic.
+// least the tile's cells and one on each side); a particle whose cells lie
+// outside the box gathers and deposits through global memory with the same
+// arithmetic.
 #pragma once
 
 #include "common.cuh"
